@@ -17,6 +17,7 @@
 #include <cmath>
 #include <cstring>
 #include <new>
+#include <type_traits>
 #include <vector>
 
 #include "internal.h"
@@ -69,125 +70,269 @@ void deriche_zero_order(double sigmad, Deriche& out) {
     std::memcpy(out.c, c, sizeof(c));
 }
 
-__global__ void k_widen(const float* __restrict__ in, double* __restrict__ out, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (double)in[i];
-}
-
-__global__ void k_narrow(const double* __restrict__ in, float* __restrict__ out, int64_t n) {
-    for (int64_t i = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
-        out[i] = (float)in[i];
-}
-
 // a·x + b·y + c·z + d·w, each product rounded and the sum taken left to right
 __device__ __forceinline__ double dot4(double a, double x, double b, double y, double c, double z, double d,
                                        double w) {
     return __dadd_rn(__dadd_rn(__dadd_rn(__dmul_rn(a, x), __dmul_rn(b, y)), __dmul_rn(c, z)), __dmul_rn(d, w));
 }
 
-// One line per thread through the fourth-order causal + anti-causal recursion
-// (recursive_gaussian.rs:472-529): the causal pass writes outs into `out`; the
-// anti-causal pass runs backwards with a four-value window and adds each scratch
-// value into out as soon as it is formed (outs[k] + scratch[k], the reference's
-// final roll-in). The border value extends to infinity on both ends. Lines of
-// axis `axis` are indexed by the other two coordinates; a line's element k sits at
-// base + k·stride.
-__global__ void k_gauss_lines(const double* __restrict__ in, double* __restrict__ out, int64_t nx, int64_t ny,
-                              int64_t nz, int axis, Deriche C) {
-    const double n0 = C.c[0], n1 = C.c[1], n2 = C.c[2], n3 = C.c[3];
-    const double d1 = C.c[4], d2 = C.c[5], d3 = C.c[6], d4 = C.c[7];
-    const double m1 = C.c[8], m2 = C.c[9], m3 = C.c[10], m4 = C.c[11];
-    const double bn1 = C.c[12], bn2 = C.c[13], bn3 = C.c[14], bn4 = C.c[15];
-    const double bm1 = C.c[16], bm2 = C.c[17], bm3 = C.c[18], bm4 = C.c[19];
-    int64_t ln, stride, na;  // line length, element stride, lines along the first other axis
-    if (axis == 0) {
-        ln = nx;
-        stride = 1;
-        na = ny;
-    } else if (axis == 1) {
-        ln = ny;
-        stride = nx;
-        na = nx;
-    } else {
-        ln = nz;
-        stride = nx * ny;
-        na = nx;
+// The line recursion (recursive_gaussian.rs:472-529): a causal and an anti-causal
+// fourth-order pass, the border value extended to infinity on both ends, out = causal +
+// anti-causal. Both passes have one shape. Walking away from its own border, a pass at
+// step j takes a sample x_j, forms
+//     v_j = (x_j·c0 + x_{j−1}·c1 + x_{j−2}·c2 + x_{j−3}·c3)
+//         − (v_{j−1}·d1 + v_{j−2}·d2 + v_{j−3}·d3 + v_{j−4}·d4)
+// (samples before the border are the border value e; a v before the border enters as
+// e·b_l instead of v·d_l), and contributes v_j to element j from that end. The causal
+// pass takes x_j = element j, the anti-causal one the element before (one nearer its
+// border). Every product and sum is separately rounded in the reference's order.
+struct Recursion {
+    double c0, c1, c2, c3, d1, d2, d3, d4, b1, b2, b3, b4;
+    double e, w1, w2, w3, q1, q2, q3, q4;
+
+    __device__ __forceinline__ void start(const Deriche& C, int dir, double border) {
+        const double* n = C.c + (dir ? 8 : 0);
+        const double* b = C.c + (dir ? 16 : 12);
+        c0 = n[0]; c1 = n[1]; c2 = n[2]; c3 = n[3];
+        d1 = C.c[4]; d2 = C.c[5]; d3 = C.c[6]; d4 = C.c[7];
+        b1 = b[0]; b2 = b[1]; b3 = b[2]; b4 = b[3];
+        e = w1 = w2 = w3 = border;
+        q1 = q2 = q3 = q4 = 0.0;
     }
-    const int64_t nlines = (nx * ny * nz) / ln;
-    for (int64_t L = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; L < nlines;
-         L += (int64_t)gridDim.x * blockDim.x) {
-        // line L → (a, b): the two coordinates other than `axis`, first one fastest
-        const int64_t a = L % na, b = L / na;
-        int64_t base;
-        if (axis == 0)
-            base = a * nx + b * nx * ny;  // (y, z)
-        else if (axis == 1)
-            base = a + b * nx * ny;  // (x, z)
-        else
-            base = a + b * nx;  // (x, y)
-        const double* __restrict__ data = in + base;
-        double* __restrict__ o = out + base;
-        // ---- causal pass
-        const double v1 = data[0];
-        const double x1 = data[stride], x2 = data[2 * stride], x3 = data[3 * stride];
-        double o0 = dot4(v1, n0, v1, n1, v1, n2, v1, n3);
-        double o1 = dot4(x1, n0, v1, n1, v1, n2, v1, n3);
-        double o2 = dot4(x2, n0, x1, n1, v1, n2, v1, n3);
-        double o3 = dot4(x3, n0, x2, n1, x1, n2, v1, n3);
-        o0 = __dsub_rn(o0, dot4(v1, bn1, v1, bn2, v1, bn3, v1, bn4));
-        o1 = __dsub_rn(o1, dot4(o0, d1, v1, bn2, v1, bn3, v1, bn4));
-        o2 = __dsub_rn(o2, dot4(o1, d1, o0, d2, v1, bn3, v1, bn4));
-        o3 = __dsub_rn(o3, dot4(o2, d1, o1, d2, o0, d3, v1, bn4));
-        o[0] = o0;
-        o[stride] = o1;
-        o[2 * stride] = o2;
-        o[3 * stride] = o3;
-        // window: data[i-1..i-3] and outs[i-1..i-4]
-        double p1 = x3, p2 = x2, p3 = x1;
-        double q1 = o3, q2 = o2, q3 = o1, q4 = o0;
-        for (int64_t i = 4; i < ln; ++i) {
-            const double x = data[i * stride];
-            double v = dot4(x, n0, p1, n1, p2, n2, p3, n3);
-            v = __dsub_rn(v, dot4(q1, d1, q2, d2, q3, d3, q4, d4));
-            o[i * stride] = v;
-            p3 = p2;
-            p2 = p1;
-            p1 = x;
-            q4 = q3;
-            q3 = q2;
-            q2 = q1;
-            q1 = v;
+    // the sum over the samples, which does not depend on the recursion
+    __device__ __forceinline__ double samples(double x) {
+        const double a = dot4(x, c0, w1, c1, w2, c2, w3, c3);
+        w3 = w2;
+        w2 = w1;
+        w1 = x;
+        return a;
+    }
+    // BORDER: the step index where it is below 4, else 4
+    template <int BORDER = 4>
+    __device__ __forceinline__ double next(double a) {
+        const double r = dot4(BORDER >= 1 ? q1 : e, BORDER >= 1 ? d1 : b1, BORDER >= 2 ? q2 : e, BORDER >= 2 ? d2 : b2,
+                              BORDER >= 3 ? q3 : e, BORDER >= 3 ? d3 : b3, BORDER >= 4 ? q4 : e, BORDER >= 4 ? d4 : b4);
+        const double v = __dsub_rn(a, r);
+        q4 = q3;
+        q3 = q2;
+        q2 = q1;
+        q1 = v;
+        return v;
+    }
+    template <int BORDER>
+    __device__ __forceinline__ double step(double x) {
+        return next<BORDER>(samples(x));
+    }
+};
+
+// A warp takes 16 lines: lanes 0–15 run the causal pass of one line each, lanes 16–31 the
+// anti-causal pass of the same lines, both walking at once from opposite ends. Until the
+// middle each leaves its v in shared memory; past it each finds the other pass's v there
+// and the element is finished. So a line is read twice (the second time from L2) and
+// written once, no partial result leaves the chip, and the two serial chains, which are
+// what one line costs (five dependent FP64 operations a step), run side by side.
+// One-warp CTAs of n·128 B shared memory: seven on an SM at n = 256, where the chain (40
+// cycles a step) and the FP64 pipe (15 operations a step, 2 cycles each, 7/4 warps a
+// scheduler) are about even. So what stands beside the chain must be little and must not
+// join it: steps go in blocks of eight, each block's chain runs beside the next block's
+// sample sums, and the shared-memory rows are numbered by step, so that a block's
+// accesses are constant offsets from one address. The volume stays FP64 between axes and
+// is f32 on both ends: the first pass widens as it reads, the last narrows as it writes.
+// 251×256×243: 108, 120 and 113 µs for the three axes; one line per thread with the
+// partial results in global memory took 285 µs an axis, and widening and narrowing
+// passes of their own another 58 µs.
+constexpr int GL = 16;       // lines a warp
+constexpr int GB = 8;        // steps a block
+constexpr int GROW = 32;     // doubles a shared-memory row: the lanes' v of one step
+constexpr int GROW_X = 33;   // in the x-axis pass, which also reads it by columns
+
+// The doubles of shared memory for a line of n: rows for the steps up to its middle.
+__host__ __device__ inline size_t gauss_rows(int64_t n) { return (size_t)(n / 2 + 1); }
+
+// Steps j0 … j0 + 7 of both passes (the line's last block may have fewer): a holds the
+// block's sample sums and is given the next block's, from its samples xn. A lane's v of
+// step j < n/2 is left at its column of row j; past the middle the other pass's v of the
+// same element is at the partner lane's column of row n − 1 − j, and done(u, place, out)
+// finishes that element.
+template <int ROW, class Done>
+__device__ __forceinline__ void eight_steps(Recursion& R, int j0, int n, double (&a)[GB], const double (&xn)[GB],
+                                            double* part, Done done) {
+    const int lane = threadIdx.x, half = n / 2;
+    if (j0 > 0 && j0 + GB <= half) {
+        double* row = part + j0 * ROW + lane;
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            row[u * ROW] = R.next(a[u]);
+            a[u] = R.samples(xn[u]);
         }
-        // ---- anti-causal pass
-        const double v2 = data[(ln - 1) * stride];
-        const double y1 = data[(ln - 1) * stride], y2 = data[(ln - 2) * stride], y3 = data[(ln - 3) * stride];
-        double s1 = dot4(v2, m1, v2, m2, v2, m3, v2, m4);  // scratch[ln-1]
-        double s2 = dot4(y1, m1, v2, m2, v2, m3, v2, m4);  // scratch[ln-2]
-        double s3 = dot4(y2, m1, y1, m2, v2, m3, v2, m4);  // scratch[ln-3]
-        double s4 = dot4(y3, m1, y2, m2, y1, m3, v2, m4);  // scratch[ln-4]
-        s1 = __dsub_rn(s1, dot4(v2, bm1, v2, bm2, v2, bm3, v2, bm4));
-        s2 = __dsub_rn(s2, dot4(s1, d1, v2, bm2, v2, bm3, v2, bm4));
-        s3 = __dsub_rn(s3, dot4(s2, d1, s1, d2, v2, bm3, v2, bm4));
-        s4 = __dsub_rn(s4, dot4(s3, d1, s2, d2, s1, d3, v2, bm4));
-        o[(ln - 1) * stride] = __dadd_rn(o[(ln - 1) * stride], s1);
-        o[(ln - 2) * stride] = __dadd_rn(o[(ln - 2) * stride], s2);
-        o[(ln - 3) * stride] = __dadd_rn(o[(ln - 3) * stride], s3);
-        o[(ln - 4) * stride] = __dadd_rn(o[(ln - 4) * stride], s4);
-        // window: data[i..i+3] and scratch[i..i+3], writing scratch[i-1]
-        double e0 = data[(ln - 4) * stride], e1 = y3, e2 = y2, e3 = y1;
-        double t0 = s4, t1 = s3, t2 = s2, t3 = s1;
-        for (int64_t i = ln - 4; i > 0; --i) {
-            double v = dot4(e0, m1, e1, m2, e2, m3, e3, m4);
-            v = __dsub_rn(v, dot4(t0, d1, t1, d2, t2, d3, t3, d4));
-            o[(i - 1) * stride] = __dadd_rn(o[(i - 1) * stride], v);
-            e3 = e2;
-            e2 = e1;
-            e1 = e0;
-            e0 = data[(i - 1) * stride];
-            t3 = t2;
-            t2 = t1;
-            t1 = t0;
-            t0 = v;
+    } else if (j0 > half && j0 + GB <= n) {
+        double* row = part + (n - 1 - j0) * ROW + (lane ^ GL);
+        double o[GB];
+#pragma unroll
+        for (int u = 0; u < GB; ++u) o[u] = row[-u * ROW];
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            o[u] = __dadd_rn(R.next(a[u]), o[u]);
+            a[u] = R.samples(xn[u]);
+        }
+#pragma unroll
+        for (int u = 0; u < GB; ++u) done(u, row - u * ROW, o[u]);
+    } else {
+        // the line's first block, the one its middle falls in, its last
+#pragma unroll
+        for (int u = 0; u < GB; ++u) {
+            const int j = j0 + u;
+            if (j < n) {
+                double v;
+                if (j0 > 0 || u >= 4)
+                    v = R.next(a[u]);
+                else
+                    v = u == 0 ? R.next<0>(a[u]) : (u == 1 ? R.next<1>(a[u]) : (u == 2 ? R.next<2>(a[u]) : R.next<3>(a[u])));
+                if (j < half) {
+                    part[j * ROW + lane] = v;
+                } else {
+                    __syncwarp();  // what the passes left each other is in place
+                    // on the middle element of an odd line both passes stand at once
+                    double* at = part + (n - 1 - j) * ROW + (lane ^ GL);
+                    const double o = __shfl_xor_sync(0xffffffffu, v, GL);
+                    done(u, at, __dadd_rn(v, 2 * j + 1 == n ? o : *at));
+                }
+            }
+            a[u] = R.samples(xn[u]);
+        }
+    }
+}
+
+// Axes 1 and 2: lane l of a half walks line 16·CTA + l; neighbouring lines are neighbours in
+// memory (128-byte rows of FP64). A lane keeps the samples of two to three blocks
+// requested. Lanes past the last line repeat it (and write the same values).
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(32) k_gauss_strided(const TI* __restrict__ in, TO* __restrict__ out, int64_t nlines,
+                                                      int n, int64_t stride, int64_t na, int64_t sb, const Deriche C) {
+    extern __shared__ double part[];
+    const int dir = threadIdx.x / GL;
+    const int64_t L = min((int64_t)blockIdx.x * GL + (threadIdx.x & (GL - 1)), nlines - 1);
+    const int64_t first = (L % na) + (L / na) * sb + (dir ? (int64_t)(n - 1) * stride : 0);
+    const TI* __restrict__ from = in + first;
+    TO* __restrict__ to = out + first;
+    const int64_t ds = dir ? -stride : stride;
+    // the samples of a block: step j takes element j (causal) or j − 1 (anti-causal) from
+    // this lane's end
+    auto fetch = [&](int j0, TI (&x)[GB]) {
+        if (j0 > 0 && j0 + GB <= n) {
+            const TI* p = from + (j0 - dir) * ds;
+#pragma unroll
+            for (int u = 0; u < GB; ++u) x[u] = p[u * ds];
+        } else {
+#pragma unroll
+            for (int u = 0; u < GB; ++u) x[u] = from[min(max(j0 + u - dir, 0), n - 1) * ds];
+        }
+    };
+    TI ring[2][GB];
+    double a[GB], xn[GB];
+    fetch(0, ring[0]);
+    Recursion R;
+    R.start(C, dir, (double)from[0]);
+#pragma unroll
+    for (int u = 0; u < GB; ++u) a[u] = R.samples((double)ring[0][u]);
+    fetch(GB, ring[0]);
+    fetch(2 * GB, ring[1]);
+    for (int j0 = 0; j0 < n; j0 += 2 * GB) {
+#pragma unroll
+        for (int b = 0; b < 2; ++b) {
+            const int j = j0 + b * GB;
+            if (j < n) {
+#pragma unroll
+                for (int u = 0; u < GB; ++u) xn[u] = (double)ring[b][u];
+                fetch(j + 3 * GB, ring[b]);
+                TO* p = to + j * ds;
+                eight_steps<GROW>(R, j, n, a, xn, part, [&](int u, double*, double v) { p[u * ds] = (TO)v; });
+            }
+        }
+    }
+}
+
+// Axis 0: a line is contiguous, so the warp moves 32 steps of its 16 lines (from both
+// ends) through a shared-memory tile, row by row, requested a tile ahead. Finished
+// elements replace what the passes left, and leave line by line at the end.
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(32) k_gauss_rows(const TI* __restrict__ in, TO* __restrict__ out, int64_t nlines,
+                                                   int n, const Deriche C) {
+    extern __shared__ double part[];  // the rows, then the tile [32][33]
+    constexpr int CH = 32;
+    TI* tile = reinterpret_cast<TI*>(part + gauss_rows(n) * GROW_X);
+    const int lane = threadIdx.x, dir = lane / GL;
+    const int64_t line0 = (int64_t)blockIdx.x * GL;
+    const int lines = (int)min((int64_t)GL, nlines - line0);
+    const TI* __restrict__ from = in + line0 * n;
+    TI f[GL], b[GL];
+    auto request = [&](int j0) {
+        const int tf = min(j0 + lane, n - 1), tb = n - 1 - min(max(j0 + lane - 1, 0), n - 1);
+#pragma unroll
+        for (int r = 0; r < GL; ++r) {
+            const int row = min(r, lines - 1) * n;
+            f[r] = from[row + tf];
+            b[r] = from[row + tb];
+        }
+    };
+    auto place = [&]() {
+        __syncwarp();  // the last tile has been read
+#pragma unroll
+        for (int r = 0; r < GL; ++r) {
+            tile[r * 33 + lane] = f[r];
+            tile[(GL + r) * 33 + lane] = b[r];
+        }
+        __syncwarp();
+    };
+    request(0);
+    place();
+    request(CH);
+    Recursion R;
+    R.start(C, dir, (double)tile[lane * 33]);
+    double a[GB], xn[GB];
+#pragma unroll
+    for (int u = 0; u < GB; ++u) a[u] = R.samples((double)tile[lane * 33 + u]);
+    for (int j0 = 0; j0 < n; j0 += GB) {
+        const int next = (j0 + GB) & (CH - 1);  // the next block's place in the tile
+        if (next == 0) {
+            place();
+            request(j0 + GB + CH);
+        }
+#pragma unroll
+        for (int u = 0; u < GB; ++u) xn[u] = (double)tile[lane * 33 + next + u];
+        eight_steps<GROW_X>(R, j0, n, a, xn, part, [&](int, double* place, double v) { *place = v; });
+    }
+    __syncwarp();
+    for (int r = 0; r < lines; ++r) {
+        TO* row = out + (line0 + r) * n;
+#pragma unroll 8
+        for (int k = lane; k < n; k += 32)
+            row[k] = (TO)(2 * k < n ? part[k * GROW_X + r] : part[(n - 1 - k) * GROW_X + GL + r]);
+    }
+}
+
+// Lines too long for a warp's partial results in shared memory: one line per thread, the
+// causal pass left in `mid` (FP64) and read back by the anti-causal one.
+template <typename TI, typename TO>
+__global__ void k_gauss_long(const TI* __restrict__ in, double* __restrict__ mid, TO* __restrict__ out, int64_t nlines,
+                             int64_t n, int64_t stride, int64_t na, int64_t sa, int64_t sb, const Deriche C) {
+    for (int64_t L = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; L < nlines; L += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t base = (L % na) * sa + (L / na) * sb;
+        for (int dir = 0; dir < 2; ++dir) {
+            Recursion R;
+            const int64_t first = base + (dir ? (n - 1) * stride : 0), ds = dir ? -stride : stride;
+            R.start(C, dir, (double)in[first]);
+            for (int64_t j = 0; j < n; ++j) {
+                const double x = (double)in[first + (j > dir ? j - dir : 0) * ds];
+                const double v = j >= 4 ? R.step<4>(x)
+                                        : (j == 0 ? R.step<0>(x)
+                                                  : (j == 1 ? R.step<1>(x) : (j == 2 ? R.step<2>(x) : R.step<3>(x))));
+                const int64_t at = first + j * ds;
+                if (!dir)
+                    mid[at] = v;
+                else
+                    out[at] = (TO)__dadd_rn(mid[at], v);
+            }
         }
     }
 }
@@ -289,6 +434,48 @@ int grid_of(int64_t n, int sms) {
     return g < 1 ? 1 : (int)g;
 }
 
+size_t gauss_smem(int axis, int64_t n, size_t esize) {
+    return gauss_rows(n) * (axis == 0 ? GROW_X : GROW) * 8 + (axis == 0 ? 32 * 33 * esize : 0);
+}
+
+// Lines of more than about 1,800 elements do not fit what a CTA may opt in to.
+bool long_line(mi_context* ctx, int axis, int64_t n, size_t esize) {
+    int optin = 0;
+    if (cudaDeviceGetAttribute(&optin, cudaDevAttrMaxSharedMemoryPerBlockOptin, ctx->device) != cudaSuccess) {
+        cudaGetLastError();
+        return true;
+    }
+    return gauss_smem(axis, n, esize) > (size_t)optin || n > (1 << 20);
+}
+
+// One axis of one volume. `mid`: FP64 scratch for long lines.
+template <typename TI, typename TO>
+mi_status gauss_axis(mi_context* ctx, const TI* in, double* mid, TO* out, const int64_t* sz, int axis, const Deriche& C) {
+    cudaStream_t st = ctx->stream;
+    const int64_t n = sz[axis], nlines = sz[0] * sz[1] * sz[2] / n;
+    const int64_t stride = axis == 0 ? 1 : (axis == 1 ? sz[0] : sz[0] * sz[1]);
+    // line L starts at (L % na)·sa + (L / na)·sb
+    const int64_t na = axis == 1 ? sz[0] : nlines, sa = axis == 0 ? n : 1, sb = axis == 1 ? sz[0] * sz[1] : 0;
+    const int64_t ctas = (nlines + GL - 1) / GL;
+    if (long_line(ctx, axis, n, sizeof(TI)) || ctas > 0x7fffffff) {
+        k_gauss_long<TI, TO><<<grid_of(nlines, ctx->num_sms), 256, 0, st>>>(in, mid, out, nlines, n, stride, na, sa, sb, C);
+    } else if (axis == 0) {
+        if constexpr (std::is_same<TI, float>::value) {  // axis 0 is the first: it reads the image
+            const size_t sm = gauss_smem(0, n, sizeof(TI));
+            const mi_status s = mi::raise_smem_limit(ctx, (const void*)k_gauss_rows<TI, TO>, sm);
+            if (s != MI_OK) return s;
+            k_gauss_rows<TI, TO><<<(unsigned)ctas, 32, sm, st>>>(in, out, nlines, (int)n, C);
+        }
+    } else {
+        const size_t sm = gauss_smem(axis, n, sizeof(TI));
+        const mi_status s = mi::raise_smem_limit(ctx, (const void*)k_gauss_strided<TI, TO>, sm);
+        if (s != MI_OK) return s;
+        k_gauss_strided<TI, TO><<<(unsigned)ctas, 32, sm, st>>>(in, out, nlines, (int)n, stride, na, sb, C);
+    }
+    MI_CHECK_CUDA(ctx, cudaGetLastError());
+    return MI_OK;
+}
+
 mi_status new_image(mi_context* ctx, const mi_geometry& geo, mi_image** out) {
     const int64_t n = geo.size[0] * geo.size[1] * geo.size[2];
     float* d = nullptr;
@@ -335,32 +522,39 @@ mi_status mi_image_smooth(mi_context* ctx, const mi_image* in, const double* sig
     if (s != MI_OK) return s;
     const int64_t n = in->n;
     cudaStream_t st = ctx->stream;
-    double *a = nullptr, *b = nullptr;
-    cudaError_t e = cudaMalloc(&a, (size_t)n * 8);
-    if (e == cudaSuccess) e = cudaMalloc(&b, (size_t)n * 8);
-    if (e == cudaSuccess) {
-        k_widen<<<grid_of(n, ctx->num_sms), 256, 0, st>>>(in->data, a, n);
-        e = cudaGetLastError();
-    }
-    for (int d = 0; d < 3 && e == cudaSuccess; ++d) {
-        if (!(sigma3[d] > 0.0)) continue;
+    // f32 in, FP64 between axes (two volumes in turn), f32 out
+    int axes[3], na = 0;
+    bool need_mid = false;
+    for (int d = 0; d < 3; ++d)
+        if (sigma3[d] > 0.0) {
+            axes[na++] = d;
+            need_mid = need_mid || long_line(ctx, d, g.size[d], sizeof(double));
+        }
+    double* v[3] = {nullptr, nullptr, nullptr};  // the two volumes, the long lines' scratch
+    cudaError_t e = cudaSuccess;
+    if (na > 1) e = cudaMalloc(&v[0], (size_t)n * 8);
+    if (e == cudaSuccess && na > 2) e = cudaMalloc(&v[1], (size_t)n * 8);
+    if (e == cudaSuccess && need_mid) e = cudaMalloc(&v[2], (size_t)n * 8);
+    if (e == cudaSuccess && na == 0) e = cudaMemcpyAsync(res->data, in->data, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
+    for (int i = 0; i < na && e == cudaSuccess && s == MI_OK; ++i) {
+        const int d = axes[i];
         Deriche C;
         deriche_zero_order(sigma3[d] / g.spacing[d], C);
-        const int64_t nlines = n / g.size[d];
-        k_gauss_lines<<<grid_of(nlines, ctx->num_sms), 256, 0, st>>>(a, b, g.size[0], g.size[1], g.size[2], d, C);
-        e = cudaGetLastError();
-        std::swap(a, b);
-    }
-    if (e == cudaSuccess) {
-        k_narrow<<<grid_of(n, ctx->num_sms), 256, 0, st>>>(a, res->data, n);
-        e = cudaGetLastError();
+        const bool first = i == 0, last = i == na - 1;
+        if (first && last)
+            s = gauss_axis(ctx, in->data, v[2], res->data, g.size, d, C);
+        else if (first)
+            s = gauss_axis(ctx, in->data, v[2], v[0], g.size, d, C);
+        else if (last)
+            s = gauss_axis(ctx, v[(i - 1) & 1], v[2], res->data, g.size, d, C);
+        else
+            s = gauss_axis(ctx, v[(i - 1) & 1], v[2], v[i & 1], g.size, d, C);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(a);
-    cudaFree(b);
-    if (e != cudaSuccess) {
+    for (double* p : v) cudaFree(p);
+    if (e != cudaSuccess || s != MI_OK) {
         mi_image_free(res);
-        return mi::cuda_status(ctx, e, "mi_image_smooth");
+        return e != cudaSuccess ? mi::cuda_status(ctx, e, "mi_image_smooth") : s;
     }
     *out = res;
     return MI_OK;
