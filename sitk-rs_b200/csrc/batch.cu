@@ -261,10 +261,11 @@ mi_status shape_batch(mi_batch* b, int chunk, int copies) {
         pd.a.fine_copies = fine;
     }
     if (poff > b->partials_cap) return set_error(ctx, MI_ERR_INVALID_ARGUMENT, "batch chunk shape too fine");
-    cudaFree(b->d_chunks);
+    dev_free(ctx, b->d_chunks);
     b->d_chunks = nullptr;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&b->d_chunks, chunks.size() * sizeof(Chunk)));
-    MI_CHECK_CUDA(ctx, cudaMemcpy(b->d_chunks, chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice));
+    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &b->d_chunks, chunks.size() * sizeof(Chunk)));
+    MI_CHECK_CUDA(ctx, cudaMemcpyAsync(b->d_chunks, chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice,
+                                       ctx->stream));
     b->nchunks = (int)chunks.size();
     b->chunk = chunk;
     b->copies = copies;
@@ -282,10 +283,10 @@ mi_status shape_batch(mi_batch* b, int chunk, int copies) {
     b->grid_hist = std::max(1, std::min(b->nchunks, ctx->num_sms * std::max(occ_h, 1)));
     b->grid_deriv = std::max(1, std::min(b->nchunks, ctx->num_sms * std::max(occ_d, 1)));
     if ((size_t)b->grid_hist * chunk > b->exq_len) {
-        cudaFree(b->d_exq);
+        dev_free(ctx, b->d_exq);
         b->d_exq = nullptr;
         b->exq_len = 0;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&b->d_exq, (size_t)b->grid_hist * chunk * sizeof(uint32_t)));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &b->d_exq, (size_t)b->grid_hist * chunk * sizeof(uint32_t)));
         b->exq_len = (size_t)b->grid_hist * chunk;
     }
     release_graph(b);
@@ -432,15 +433,16 @@ bool same_cfg(const mi_rsgd_config& a, const mi_rsgd_config& c) {
 void free_batch(mi_batch* b) {
     if (!b) return;
     cudaSetDevice(b->ctx->device);
-    cudaStreamSynchronize(b->ctx->stream);
+    mi_context* ctx = b->ctx;
+    cudaStreamSynchronize(ctx->stream);
     release_graph(b);
-    cudaFree(b->d_pairs);
-    cudaFree(b->d_chunks);
-    cudaFree(b->d_partials);
-    cudaFree(b->d_active);
-    cudaFree(b->d_marks);
-    cudaFree(b->d_exq);
-    if (b->h_active) cudaFreeHost(b->h_active);
+    dev_free(ctx, b->d_pairs);
+    dev_free(ctx, b->d_chunks);
+    dev_free(ctx, b->d_partials);
+    dev_free(ctx, b->d_active);
+    dev_free(ctx, b->d_marks);
+    dev_free(ctx, b->d_exq);
+    pinned_free(ctx, b->h_active);
     for (mi_metric* m : b->metrics)
         if (m) mi_metric_destroy(m);
     delete b;
@@ -519,11 +521,11 @@ mi_status mi_batch_create(mi_context* ctx, int npairs, const mi_image* const* fi
         max_chunks += (size_t)std::max<int64_t>(1, (m->n_samples + 2047) / 2048);
     }
     if (s == MI_OK) {
-        cudaError_t e = cudaMalloc(&b->d_pairs, (size_t)npairs * sizeof(PairDev));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_partials, max_chunks * NMOM * sizeof(double));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_active, sizeof(unsigned int));
-        if (e == cudaSuccess) e = cudaMallocHost(&b->h_active, sizeof(unsigned int));
-        if (e == cudaSuccess) e = cudaMalloc(&b->d_marks, 2 * sizeof(unsigned long long));
+        cudaError_t e = dev_alloc(ctx, &b->d_pairs, (size_t)npairs * sizeof(PairDev));
+        if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_partials, max_chunks * NMOM * sizeof(double));
+        if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_active, sizeof(unsigned int));
+        if (e == cudaSuccess) e = pinned_alloc(ctx, reinterpret_cast<void**>(&b->h_active), nullptr);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_marks, 2 * sizeof(unsigned long long));
         if (e != cudaSuccess) s = cuda_status(ctx, e, "mi_batch_create");
         b->partials_cap = max_chunks * NMOM;
     }

@@ -452,12 +452,12 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
     if ((size_t)ncoef > m->bs_cap) {
-        cudaFree(m->bs_coef);
-        cudaFree(m->bs_deriv);
+        dev_free(ctx, m->bs_coef);
+        dev_free(ctx, m->bs_deriv);
         m->bs_coef = m->bs_deriv = nullptr;
         m->bs_cap = 0;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->bs_coef, (size_t)ncoef * sizeof(double)));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->bs_deriv, (size_t)ncoef * sizeof(double)));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_coef, (size_t)ncoef * sizeof(double)));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_deriv, (size_t)ncoef * sizeof(double)));
         m->bs_cap = (size_t)ncoef;
     }
     MI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->bs_coef, coef, (size_t)ncoef * sizeof(double), cudaMemcpyHostToDevice, st));
@@ -487,8 +487,8 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     // depends on the fixed point and the grid only)
     if (derivative && (!m->bs_have_key || std::memcmp(m->bs_key, fixed18, sizeof(m->bs_key)) != 0)) {
         m->bs_have_key = false;
-        cudaFree(m->bs_order);
-        cudaFree(m->bs_off);
+        dev_free(ctx, m->bs_order);
+        dev_free(ctx, m->bs_off);
         m->bs_order = nullptr;
         m->bs_off = nullptr;
         const bool any = S.gsize[0] > 3 && S.gsize[1] > 3 && S.gsize[2] > 3;
@@ -500,12 +500,12 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
             uint32_t *cell = nullptr, *idx = nullptr, *cell_sorted = nullptr, *count = nullptr;
             void* tmp = nullptr;
             size_t sort_bytes = 0, scan_bytes = 0;
-            cudaError_t e = cudaMalloc(&cell, (size_t)n * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&idx, (size_t)n * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&cell_sorted, (size_t)n * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&count, (size_t)(ncells + 1) * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&m->bs_order, (size_t)n * 4);
-            if (e == cudaSuccess) e = cudaMalloc(&m->bs_off, (size_t)(ncells + 1) * 4);
+            cudaError_t e = dev_alloc(ctx, &cell, (size_t)n * 4);
+            if (e == cudaSuccess) e = dev_alloc(ctx, &idx, (size_t)n * 4);
+            if (e == cudaSuccess) e = dev_alloc(ctx, &cell_sorted, (size_t)n * 4);
+            if (e == cudaSuccess) e = dev_alloc(ctx, &count, (size_t)(ncells + 1) * 4);
+            if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_order, (size_t)n * 4);
+            if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_off, (size_t)(ncells + 1) * 4);
             if (e == cudaSuccess) e = cudaMemsetAsync(count, 0, (size_t)(ncells + 1) * 4, st);
             if (e == cudaSuccess) {
                 const int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->num_sms * 8));
@@ -517,24 +517,24 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
                                                     32, st);
             if (e == cudaSuccess)
                 e = cub::DeviceScan::ExclusiveSum(nullptr, scan_bytes, count, m->bs_off, (int)(ncells + 1), st);
-            if (e == cudaSuccess) e = cudaMalloc(&tmp, std::max(sort_bytes, scan_bytes));
+            if (e == cudaSuccess) e = dev_alloc(ctx, &tmp, std::max(sort_bytes, scan_bytes));
             if (e == cudaSuccess)
                 e = cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, cell, cell_sorted, idx, m->bs_order, (int)n, 0, 32,
                                                     st);
             if (e == cudaSuccess)
                 e = cub::DeviceScan::ExclusiveSum(tmp, scan_bytes, count, m->bs_off, (int)(ncells + 1), st);
             if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-            cudaFree(tmp);
-            cudaFree(cell);
-            cudaFree(idx);
-            cudaFree(cell_sorted);
-            cudaFree(count);
+            dev_free(ctx, tmp);
+            dev_free(ctx, cell);
+            dev_free(ctx, idx);
+            dev_free(ctx, cell_sorted);
+            dev_free(ctx, count);
             if (e != cudaSuccess) return cuda_status(ctx, e, "B-spline support cells");
         }
         std::memcpy(m->bs_key, fixed18, sizeof(m->bs_key));
         m->bs_have_key = true;
     }
-    if (!m->bs_pr) MI_CHECK_CUDA(ctx, cudaMalloc(&m->bs_pr, (size_t)B * B * sizeof(float)));
+    if (!m->bs_pr) MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_pr, (size_t)B * B * sizeof(float)));
     size_t hsm = (size_t)(((B * B + B) + 1) & ~1) * sizeof(unsigned long long);
     S.smem_coef = hsm + (size_t)ncoef * sizeof(double) <= 96 * 1024 ? 1 : 0;
     if (S.smem_coef) hsm += (size_t)ncoef * sizeof(double);

@@ -325,32 +325,33 @@ int64_t rows_of(int l, int B) {  // GEMM rows (output voxels × batch) of layer 
 
 void free_net(mi_initnet* n) {
     if (!n) return;
+    mi_context* ctx = n->ctx;
     for (auto& l : n->L) {
-        cudaFree(l.w);
-        cudaFree(l.b);
-        cudaFree(l.gw);
-        cudaFree(l.gb);
-        cudaFree(l.mw);
-        cudaFree(l.vw);
-        cudaFree(l.mb);
-        cudaFree(l.vb);
-        cudaFree(l.wb);
-        cudaFree(l.wtb);
+        mi::dev_free(ctx, l.w);
+        mi::dev_free(ctx, l.b);
+        mi::dev_free(ctx, l.gw);
+        mi::dev_free(ctx, l.gb);
+        mi::dev_free(ctx, l.mw);
+        mi::dev_free(ctx, l.vw);
+        mi::dev_free(ctx, l.mb);
+        mi::dev_free(ctx, l.vb);
+        mi::dev_free(ctx, l.wb);
+        mi::dev_free(ctx, l.wtb);
     }
-    cudaFree(n->x0);
-    for (auto p : n->col) cudaFree(p);
-    for (auto p : n->z) cudaFree(p);
-    for (auto p : n->xb) cudaFree(p);
-    cudaFree(n->dz);
-    cudaFree(n->dx);
-    cudaFree(n->dcol);
-    cudaFree(n->part);
-    cudaFree(n->loss);
-    cudaFree(n->dzb);
-    cudaFree(n->tA);
-    cudaFree(n->tB);
-    cudaFree(n->slices);
-    cudaFree(n->err);
+    mi::dev_free(ctx, n->x0);
+    for (auto p : n->col) mi::dev_free(ctx, p);
+    for (auto p : n->z) mi::dev_free(ctx, p);
+    for (auto p : n->xb) mi::dev_free(ctx, p);
+    mi::dev_free(ctx, n->dz);
+    mi::dev_free(ctx, n->dx);
+    mi::dev_free(ctx, n->dcol);
+    mi::dev_free(ctx, n->part);
+    mi::dev_free(ctx, n->loss);
+    mi::dev_free(ctx, n->dzb);
+    mi::dev_free(ctx, n->tA);
+    mi::dev_free(ctx, n->tB);
+    mi::dev_free(ctx, n->slices);
+    mi::dev_free(ctx, n->err);
     delete n;
 }
 
@@ -483,8 +484,8 @@ mi_status mi_initnet_create(mi_context* ctx, uint64_t seed, int max_batch, mi_in
     const int B = max_batch;
     cudaError_t e = cudaSuccess;
     auto alloc = [&](auto** p, size_t bytes) {
-        if (e == cudaSuccess) e = cudaMalloc((void**)p, bytes);
-        if (e == cudaSuccess) e = cudaMemset(*p, 0, bytes);
+        if (e == cudaSuccess) e = dev_alloc(ctx, p, bytes);
+        if (e == cudaSuccess) e = cudaMemsetAsync(*p, 0, bytes, ctx->stream);
     };
     // weights: He-uniform from a SplitMix64 stream seeded by `seed`
     uint64_t state = seed;
@@ -526,7 +527,7 @@ mi_status mi_initnet_create(mi_context* ctx, uint64_t seed, int max_batch, mi_in
         const double bound = std::sqrt(6.0 / fan_in) * (l == NLAYER - 1 ? 0.1 : 1.0);
         for (int o = 0; o < L.out; ++o)
             for (int k = 0; k < L.in; ++k) hw[(size_t)o * L.kp + k] = (float)((2.0 * next_u() - 1.0) * bound);
-        if (e == cudaSuccess) e = cudaMemcpy(L.w, hw.data(), wn * 4, cudaMemcpyHostToDevice);
+        if (e == cudaSuccess) e = cudaMemcpyAsync(L.w, hw.data(), wn * 4, cudaMemcpyHostToDevice, ctx->stream);
         const int64_t rows = rows_of(l, B);
         max_rows_kp = std::max(max_rows_kp, (size_t)rows * L.kp);
         max_rows_out = std::max(max_rows_out, (size_t)rows * L.out);
@@ -688,13 +689,13 @@ mi_status mi_gemm_bf16_tn(mi_context* ctx, int M, int N, int K, const void* A, i
         return MI_ERR_INVALID_ARGUMENT;
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     unsigned int* err = nullptr;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&err, sizeof(unsigned int)));
+    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &err, sizeof(unsigned int)));
     cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned int), ctx->stream);
     // a product whose M × N tiles alone would leave most SMs idle is split over K into
     // partial products summed in slice order, as the network's layers do
     const int S = ldc == N ? mi::k_splits(M, N, K) : 1;
     float* slices = nullptr;
-    if (e == cudaSuccess && S > 1) e = cudaMalloc(&slices, (size_t)S * M * N * sizeof(float));
+    if (e == cudaSuccess && S > 1) e = mi::dev_alloc(ctx, &slices, (size_t)S * M * N * sizeof(float));
     const auto* a16 = static_cast<const __nv_bfloat16*>(A);
     const auto* b16 = static_cast<const __nv_bfloat16*>(B);
     if (e == cudaSuccess && S > 1) {
@@ -709,8 +710,8 @@ mi_status mi_gemm_bf16_tn(mi_context* ctx, int M, int N, int K, const void* A, i
     unsigned int h = 0;
     if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(slices);
-    cudaFree(err);
+    mi::dev_free(ctx, slices);
+    mi::dev_free(ctx, err);
     if (e != cudaSuccess) return mi::cuda_status(ctx, e, "mi_gemm_bf16_tn");
     if (h) return mi::set_error(ctx, MI_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait gave up");
     return MI_OK;

@@ -3,10 +3,22 @@
 
 #include <cuda_runtime.h>
 #include <cstdint>
+#include <list>
+#include <mutex>
 #include <string>
 #include <vector>
 
 #include "mi_b200.h"
+
+namespace mi {
+// A CUDA array a destroyed metric left for the next one of the same shape.
+struct SpareArray {
+    cudaArray_t array;
+    size_t extent[3], element;
+    bool layered;
+    size_t bytes() const { return extent[0] * extent[1] * extent[2] * element; }
+};
+}  // namespace mi
 
 struct mi_context {
     int device = 0;
@@ -14,6 +26,12 @@ struct mi_context {
     size_t l2_bytes = 0;
     cudaStream_t stream = nullptr;
     std::string last_error;
+    // what outlives an object (context.cu): device memory, pinned blocks, texture arrays
+    cudaMemPool_t pool = nullptr;
+    std::mutex spare_mutex;
+    std::vector<unsigned char*> pinned_slabs, pinned_spare;
+    std::list<mi::SpareArray> spare_arrays;  // oldest first
+    size_t spare_array_bytes = 0;
 };
 
 struct mi_image {
@@ -207,6 +225,26 @@ namespace mi {
 
 mi_status set_error(mi_context* ctx, mi_status s, const std::string& msg);
 mi_status cuda_status(mi_context* ctx, cudaError_t e, const char* where);
+// Device memory from the context's pool, ordered on the context's stream: a block may be
+// freed while work on that stream still uses it, and what reuses it comes after that
+// work. Memory that another stream touches is freed only once that stream is done.
+cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes);
+template <typename T>
+cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
+    void* v = nullptr;
+    const cudaError_t e = dev_alloc_bytes(ctx, &v, bytes);
+    *p = static_cast<T*>(v);
+    return e;
+}
+void dev_free(mi_context* ctx, void* p);
+// A block of PINNED_BLOCK bytes of pinned host memory mapped into the device; `dev` (its
+// device address) may be null.
+constexpr size_t PINNED_BLOCK = 512;
+cudaError_t pinned_alloc(mi_context* ctx, void** host, void** dev);
+void pinned_free(mi_context* ctx, void* host);
+// A 3-D or layered array of 4-byte float or 2-byte unsigned elements.
+cudaError_t array_alloc(mi_context* ctx, cudaArray_t* out, const cudaExtent& ext, size_t element, bool layered);
+void array_free(mi_context* ctx, cudaArray_t array, const cudaExtent& ext, size_t element, bool layered);
 // Raises (never lowers) a kernel's dynamic shared-memory limit on the context's device.
 mi_status raise_smem_limit(mi_context* ctx, const void* fn, size_t bytes);
 

@@ -360,13 +360,13 @@ mi_status minmax(mi_context* ctx, const float* vals, const uint32_t* idx, const 
     const int block = 256;
     const int grid = grid_for(n, block, ctx->num_sms * 4);
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&d, (size_t)grid * 2 * sizeof(float)));
+    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &d, (size_t)grid * 2 * sizeof(float)));
     k_minmax<<<grid, block, 0, ctx->stream>>>(vals, idx, mask, n, d);
     std::vector<float> h((size_t)grid * 2);
     cudaError_t e = cudaGetLastError();
     if (e == cudaSuccess) e = cudaMemcpyAsync(h.data(), d, h.size() * sizeof(float), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-    cudaFree(d);
+    dev_free(ctx, d);
     if (e != cudaSuccess) return cuda_status(ctx, e, "minmax");
     float l = INFINITY, u = -INFINITY;
     for (int b = 0; b < grid; ++b) {
@@ -413,35 +413,38 @@ int hist_grid(mi_context* ctx, int64_t n, int occ, int B) {
 void free_metric(mi_metric* m) {
     if (!m) return;
     if (m->mtex) cudaDestroyTextureObject(m->mtex);
-    if (m->marray) cudaFreeArray(m->marray);
-    cudaFree(m->fixed);
-    cudaFree(m->moving);
-    cudaFree(m->mmask);
-    cudaFree(m->samples);
-    cudaFree(m->fbin);
-    cudaFree(m->codes);
-    cudaFree(m->chunk_run);
-    cudaFree(m->run_brick);
-    cudaFree(m->run_chunk0);
-    cudaFree(m->run_start);
-    cudaFree(m->ws.hist);
-    cudaFree(m->ws.partials);
-    cudaFree(m->ws.vsum);
-    cudaFree(m->ws.exq);
-    cudaFree(m->ws.result);
-    cudaFree(m->ws.done_counter);
-    cudaFree(m->ws.rec_bins);
-    cudaFree(m->ws.rec_f);
-    cudaFree(m->ws.rec_g);
-    if (m->ws.host_result) cudaFreeHost(m->ws.host_result);
+    mi_context* ctx = m->ctx;
+    array_free(ctx, m->marray,
+               make_cudaExtent((size_t)m->mgeo.size[0], (size_t)m->mgeo.size[1], (size_t)m->mgeo.size[2]),
+               m->base.mbf16 ? 2 : 4, m->base.mlayered != 0);
+    dev_free(ctx, m->fixed);
+    dev_free(ctx, m->moving);
+    dev_free(ctx, m->mmask);
+    dev_free(ctx, m->samples);
+    dev_free(ctx, m->fbin);
+    dev_free(ctx, m->codes);
+    dev_free(ctx, m->chunk_run);
+    dev_free(ctx, m->run_brick);
+    dev_free(ctx, m->run_chunk0);
+    dev_free(ctx, m->run_start);
+    dev_free(ctx, m->ws.hist);
+    dev_free(ctx, m->ws.partials);
+    dev_free(ctx, m->ws.vsum);
+    dev_free(ctx, m->ws.exq);
+    dev_free(ctx, m->ws.result);
+    dev_free(ctx, m->ws.done_counter);
+    dev_free(ctx, m->ws.rec_bins);
+    dev_free(ctx, m->ws.rec_f);
+    dev_free(ctx, m->ws.rec_g);
+    pinned_free(ctx, m->ws.host_result);
     for (int i = 0; i < 5; ++i)
         if (m->ws.ev[i]) cudaEventDestroy(m->ws.ev[i]);
     moments_free(m);
-    cudaFree(m->bs_coef);
-    cudaFree(m->bs_deriv);
-    cudaFree(m->bs_order);
-    cudaFree(m->bs_off);
-    cudaFree(m->bs_pr);
+    dev_free(ctx, m->bs_coef);
+    dev_free(ctx, m->bs_deriv);
+    dev_free(ctx, m->bs_order);
+    dev_free(ctx, m->bs_off);
+    dev_free(ctx, m->bs_pr);
     delete m;
 }
 
@@ -480,7 +483,7 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
     const int block = 256;
     if (strategy == MI_SAMPLING_NONE) {
         count = nvox;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&draw, pad4(count) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &draw, pad4(count) * 4));
         k_iota_stride<<<grid_for(count, block, ctx->num_sms * 8), block, 0, st>>>(count, 1, draw);
     } else if (strategy == MI_SAMPLING_REGULAR) {
         if (!(smp->percentage > 0.0) || !std::isfinite(smp->percentage))
@@ -488,7 +491,7 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         int64_t stride = (int64_t)std::ceil(1.0 / smp->percentage);
         if (stride < 1) stride = 1;
         count = (nvox + stride - 1) / stride;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&draw, pad4(count) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &draw, pad4(count) * 4));
         k_iota_stride<<<grid_for(count, block, ctx->num_sms * 8), block, 0, st>>>(count, (uint64_t)stride, draw);
     } else if (strategy == MI_SAMPLING_RANDOM) {
         if (!(smp->percentage > 0.0) || !std::isfinite(smp->percentage))
@@ -496,7 +499,7 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         count = (int64_t)((double)nvox * smp->percentage);
         if (count >= ((int64_t)1 << 31))
             return set_error(ctx, MI_ERR_INVALID_ARGUMENT, "sample count exceeds 2^31");
-        MI_CHECK_CUDA(ctx, cudaMalloc(&draw, pad4(count) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &draw, pad4(count) * 4));
         if (count)
             k_draw_random<<<grid_for(count, block, ctx->num_sms * 8), block, 0, st>>>(smp->seed, (uint64_t)nvox,
                                                                                          count, draw);
@@ -515,7 +518,7 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
                                      std::to_string(nvox) + " voxels");
             h[i] = (uint32_t)v;
         }
-        MI_CHECK_CUDA(ctx, cudaMalloc(&draw, pad4(count) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &draw, pad4(count) * 4));
         if (count) MI_CHECK_CUDA(ctx, cudaMemcpyAsync(draw, h.data(), (size_t)count * 4, cudaMemcpyHostToDevice, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
     } else {
@@ -531,21 +534,21 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         uint8_t* flags = nullptr;
         uint32_t* out = nullptr;
         int* nsel = nullptr;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&flags, (size_t)count));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&out, pad4(count) * 4));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&nsel, sizeof(int)));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &flags, (size_t)count));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &out, pad4(count) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &nsel, sizeof(int)));
         k_mask_flags<<<grid_for(count, block, ctx->num_sms * 8), block, 0, st>>>(draw, count, fixed_mask->data, flags);
         MI_CHECK_CUDA(ctx, cub::DeviceSelect::Flagged(nullptr, tmp_bytes, draw, flags, out, nsel, (int)count, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&tmp, tmp_bytes));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &tmp, tmp_bytes));
         MI_CHECK_CUDA(ctx, cub::DeviceSelect::Flagged(tmp, tmp_bytes, draw, flags, out, nsel, (int)count, st));
         int h = 0;
         MI_CHECK_CUDA(ctx, cudaMemcpyAsync(&h, nsel, sizeof(int), cudaMemcpyDeviceToHost, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(tmp);
+        dev_free(ctx, tmp);
         tmp = nullptr;
-        cudaFree(flags);
-        cudaFree(nsel);
-        cudaFree(draw);
+        dev_free(ctx, flags);
+        dev_free(ctx, nsel);
+        dev_free(ctx, draw);
         kept = out;
         nkept = h;
     }
@@ -561,23 +564,23 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         while (bits < 64 && ((uint64_t)1 << bits) < kmax) ++bits;
         unsigned long long *keys = nullptr, *keys_out = nullptr;
         uint32_t* sorted = nullptr;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&keys, (size_t)nkept * 8));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&keys_out, (size_t)nkept * 8));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&sorted, pad4(nkept) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &keys, (size_t)nkept * 8));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &keys_out, (size_t)nkept * 8));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &sorted, pad4(nkept) * 4));
         k_brick_key_bl<<<grid_for(nkept, block, ctx->num_sms * 8), block, 0, st>>>(kept, nkept, nx, ny, bl, nbx, nby,
                                                                                   keys);
         MI_CHECK_CUDA(ctx, cudaGetLastError());
         tmp_bytes = 0;
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys_out, kept, sorted,
                                                            (int)nkept, 0, bits, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&tmp, tmp_bytes));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &tmp, tmp_bytes));
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys_out, kept, sorted, (int)nkept,
                                                            0, bits, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(tmp);
-        cudaFree(keys);
-        cudaFree(keys_out);
-        cudaFree(kept);
+        dev_free(ctx, tmp);
+        dev_free(ctx, keys);
+        dev_free(ctx, keys_out);
+        dev_free(ctx, kept);
         kept = sorted;
     } else if (nkept > 1 && SAMPLE_BRICK_LOG2 > 0) {
         const int lb = SAMPLE_BRICK_LOG2;
@@ -589,35 +592,35 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         while (bits < 64 && ((uint64_t)1 << bits) < kmax) ++bits;
         unsigned long long *keys = nullptr, *keys_out = nullptr;
         uint32_t* sorted = nullptr;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&keys, (size_t)nkept * 8));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&keys_out, (size_t)nkept * 8));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&sorted, pad4(nkept) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &keys, (size_t)nkept * 8));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &keys_out, (size_t)nkept * 8));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &sorted, pad4(nkept) * 4));
         k_brick_key<<<grid_for(nkept, block, ctx->num_sms * 8), block, 0, st>>>(kept, nkept, nx, ny, lb, nbx, nby, keys);
         MI_CHECK_CUDA(ctx, cudaGetLastError());
         tmp_bytes = 0;
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys, keys_out, kept, sorted,
                                                            (int)nkept, 0, bits, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&tmp, tmp_bytes));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &tmp, tmp_bytes));
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortPairs(tmp, tmp_bytes, keys, keys_out, kept, sorted, (int)nkept,
                                                            0, bits, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(tmp);
-        cudaFree(keys);
-        cudaFree(keys_out);
-        cudaFree(kept);
+        dev_free(ctx, tmp);
+        dev_free(ctx, keys);
+        dev_free(ctx, keys_out);
+        dev_free(ctx, kept);
         kept = sorted;
     } else if (nkept > 1) {
         uint32_t* sorted = nullptr;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&sorted, pad4(nkept) * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &sorted, pad4(nkept) * 4));
         int bits = 1;
         while (bits < 32 && ((uint64_t)1 << bits) < (uint64_t)nvox) ++bits;
         tmp_bytes = 0;
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortKeys(nullptr, tmp_bytes, kept, sorted, (int)nkept, 0, bits, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&tmp, tmp_bytes));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &tmp, tmp_bytes));
         MI_CHECK_CUDA(ctx, cub::DeviceRadixSort::SortKeys(tmp, tmp_bytes, kept, sorted, (int)nkept, 0, bits, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
-        cudaFree(tmp);
-        cudaFree(kept);
+        dev_free(ctx, tmp);
+        dev_free(ctx, kept);
         kept = sorted;
     }
     m->samples = kept;
@@ -639,16 +642,16 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
         // one chunk of padding keeps every launch shape non-empty
         m->nchunks = 1;
         m->nruns = 1;
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->codes, BRICK_CHUNK * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->codes, BRICK_CHUNK * 4));
         MI_CHECK_CUDA(ctx, cudaMemsetAsync(m->codes, 0xFF, BRICK_CHUNK * 4, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->chunk_run, 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->chunk_run, 4));
         MI_CHECK_CUDA(ctx, cudaMemsetAsync(m->chunk_run, 0, 4, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->run_brick, 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->run_brick, 4));
         MI_CHECK_CUDA(ctx, cudaMemsetAsync(m->run_brick, 0, 4, st));
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->run_start, 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->run_start, 4));
         MI_CHECK_CUDA(ctx, cudaMemsetAsync(m->run_start, 0, 4, st));
         const uint32_t r0[2] = {0u, 1u};
-        MI_CHECK_CUDA(ctx, cudaMalloc(&m->run_chunk0, 2 * 4));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->run_chunk0, 2 * 4));
         MI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->run_chunk0, r0, 2 * 4, cudaMemcpyHostToDevice, st));
         MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
         return MI_OK;
@@ -660,15 +663,15 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
     size_t tb = 0;
     auto done = [&](mi_status s) {
         cudaStreamSynchronize(st);
-        cudaFree(whole);
-        cudaFree(bid);
-        cudaFree(uniq);
-        cudaFree(nch);
-        cudaFree(chunk_off);
-        cudaFree(run_start);
-        cudaFree(counts);
-        cudaFree(nruns_d);
-        cudaFree(tmp);
+        dev_free(ctx, whole);
+        dev_free(ctx, bid);
+        dev_free(ctx, uniq);
+        dev_free(ctx, nch);
+        dev_free(ctx, chunk_off);
+        dev_free(ctx, run_start);
+        dev_free(ctx, counts);
+        dev_free(ctx, nruns_d);
+        dev_free(ctx, tmp);
         return s;
     };
 #define TRY_L(expr)                                                      \
@@ -685,10 +688,10 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
         const uint64_t kmax = (uint64_t)(nbx * nby * nbz) << (3 * bl);
         int bits = 1;
         while (bits < 64 && ((uint64_t)1 << bits) < kmax) ++bits;
-        cudaError_t e = cudaMalloc(&keys, (size_t)n * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&keys_out, (size_t)n * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&iota, (size_t)n * 4);
-        if (e == cudaSuccess) e = cudaMalloc(&whole, (size_t)n * 4);
+        cudaError_t e = dev_alloc(ctx, &keys, (size_t)n * 8);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &keys_out, (size_t)n * 8);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &iota, (size_t)n * 4);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &whole, (size_t)n * 4);
         if (e == cudaSuccess) {
             k_iota_stride<<<grid_for(n, block, ctx->num_sms * 8), block, 0, st>>>(n, 1, iota);
             k_brick_key_bl<<<grid_for(n, block, ctx->num_sms * 8), block, 0, st>>>(iota, n, nx, ny, bl, nbx, nby, keys);
@@ -696,43 +699,43 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
         }
         if (e == cudaSuccess)
             e = cub::DeviceRadixSort::SortPairs(nullptr, tb, keys, keys_out, iota, whole, (int)n, 0, bits, st);
-        if (e == cudaSuccess) e = cudaMalloc(&tmp, tb);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &tmp, tb);
         if (e == cudaSuccess)
             e = cub::DeviceRadixSort::SortPairs(tmp, tb, keys, keys_out, iota, whole, (int)n, 0, bits, st);
         if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-        cudaFree(keys);
-        cudaFree(keys_out);
-        cudaFree(iota);
-        cudaFree(tmp);
+        dev_free(ctx, keys);
+        dev_free(ctx, keys_out);
+        dev_free(ctx, iota);
+        dev_free(ctx, tmp);
         tmp = nullptr;
         tb = 0;
         if (e != cudaSuccess) return done(cuda_status(ctx, e, "brick layout of the whole grid"));
         list = whole;
     }
-    TRY_L(cudaMalloc(&bid, (size_t)n * 4));
-    TRY_L(cudaMalloc(&uniq, (size_t)n * 4));
-    TRY_L(cudaMalloc(&counts, (size_t)n * 4));
-    TRY_L(cudaMalloc(&nruns_d, sizeof(int)));
+    TRY_L(dev_alloc(ctx, &bid, (size_t)n * 4));
+    TRY_L(dev_alloc(ctx, &uniq, (size_t)n * 4));
+    TRY_L(dev_alloc(ctx, &counts, (size_t)n * 4));
+    TRY_L(dev_alloc(ctx, &nruns_d, sizeof(int)));
     k_brick_of<<<grid_for(n, block, ctx->num_sms * 8), block, 0, st>>>(list, n, nx, ny, bl, nbx, nby, bid);
     TRY_L(cudaGetLastError());
     TRY_L(cub::DeviceRunLengthEncode::Encode(nullptr, tb, bid, uniq, counts, nruns_d, (int)n, st));
-    TRY_L(cudaMalloc(&tmp, tb));
+    TRY_L(dev_alloc(ctx, &tmp, tb));
     TRY_L(cub::DeviceRunLengthEncode::Encode(tmp, tb, bid, uniq, counts, nruns_d, (int)n, st));
     int nruns = 0;
     TRY_L(cudaMemcpyAsync(&nruns, nruns_d, sizeof(int), cudaMemcpyDeviceToHost, st));
     TRY_L(cudaStreamSynchronize(st));
-    cudaFree(tmp);
+    dev_free(ctx, tmp);
     tmp = nullptr;
-    TRY_L(cudaMalloc(&nch, (size_t)nruns * 4));
-    TRY_L(cudaMalloc(&chunk_off, (size_t)nruns * 4));
-    TRY_L(cudaMalloc(&run_start, (size_t)nruns * 4));
+    TRY_L(dev_alloc(ctx, &nch, (size_t)nruns * 4));
+    TRY_L(dev_alloc(ctx, &chunk_off, (size_t)nruns * 4));
+    TRY_L(dev_alloc(ctx, &run_start, (size_t)nruns * 4));
     k_run_chunks<<<grid_for(nruns, block, ctx->num_sms * 8), block, 0, st>>>(counts, nruns, nch);
     TRY_L(cudaGetLastError());
     tb = 0;
     size_t tb2 = 0;
     TRY_L(cub::DeviceScan::ExclusiveSum(nullptr, tb, nch, chunk_off, nruns, st));
     TRY_L(cub::DeviceScan::ExclusiveSum(nullptr, tb2, reinterpret_cast<const uint32_t*>(counts), run_start, nruns, st));
-    TRY_L(cudaMalloc(&tmp, std::max(tb, tb2)));
+    TRY_L(dev_alloc(ctx, &tmp, std::max(tb, tb2)));
     TRY_L(cub::DeviceScan::ExclusiveSum(tmp, tb, nch, chunk_off, nruns, st));
     TRY_L(cub::DeviceScan::ExclusiveSum(tmp, tb2, reinterpret_cast<const uint32_t*>(counts), run_start, nruns, st));
     uint32_t last[2] = {0, 0};
@@ -744,10 +747,10 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
         return done(set_error(ctx, MI_ERR_INVALID_ARGUMENT, "too many samples for the brick layout"));
     m->nchunks = nchunks;
     m->nruns = nruns;
-    TRY_L(cudaMalloc(&m->codes, (size_t)nchunks * BRICK_CHUNK * 4));
+    TRY_L(dev_alloc(ctx, &m->codes, (size_t)nchunks * BRICK_CHUNK * 4));
     TRY_L(cudaMemsetAsync(m->codes, 0xFF, (size_t)nchunks * BRICK_CHUNK * 4, st));
-    TRY_L(cudaMalloc(&m->chunk_run, (size_t)nchunks * 4));
-    TRY_L(cudaMalloc(&m->run_brick, (size_t)nruns * 4));
+    TRY_L(dev_alloc(ctx, &m->chunk_run, (size_t)nchunks * 4));
+    TRY_L(dev_alloc(ctx, &m->run_brick, (size_t)nruns * 4));
     k_run_fill<<<grid_for(nruns, block, ctx->num_sms * 8), block, 0, st>>>(uniq, nruns, chunk_off, nch, nbx, nby,
                                                                            m->run_brick, m->chunk_run);
     TRY_L(cudaGetLastError());
@@ -756,9 +759,9 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
     TRY_L(cudaGetLastError());
     // the first sample of every run in the walk order, the first chunk of every run and
     // the chunk count after the last
-    TRY_L(cudaMalloc(&m->run_start, (size_t)nruns * 4));
+    TRY_L(dev_alloc(ctx, &m->run_start, (size_t)nruns * 4));
     TRY_L(cudaMemcpyAsync(m->run_start, run_start, (size_t)nruns * 4, cudaMemcpyDeviceToDevice, st));
-    TRY_L(cudaMalloc(&m->run_chunk0, ((size_t)nruns + 1) * 4));
+    TRY_L(dev_alloc(ctx, &m->run_chunk0, ((size_t)nruns + 1) * 4));
     TRY_L(cudaMemcpyAsync(m->run_chunk0, chunk_off, (size_t)nruns * 4, cudaMemcpyDeviceToDevice, st));
     {
         const uint32_t total = (uint32_t)nchunks;
@@ -1148,7 +1151,7 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
     uint16_t* mbits = nullptr;  // BF16 storage: the rounded volume's bits, for the texture
     auto fail = [&](mi_status s) {
         cudaStreamSynchronize(st);
-        cudaFree(mbits);
+        dev_free(ctx, mbits);
         free_metric(m);
         return s;
     };
@@ -1157,19 +1160,19 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         cudaError_t _e = (expr);                                         \
         if (_e != cudaSuccess) return fail(cuda_status(ctx, _e, #expr)); \
     } while (0)
-    TRY_CUDA(cudaMalloc(&m->fixed, (size_t)nvox * 4));
-    TRY_CUDA(cudaMalloc(&m->moving, (size_t)mvox * 4));
+    TRY_CUDA(dev_alloc(ctx, &m->fixed, (size_t)nvox * 4));
+    TRY_CUDA(dev_alloc(ctx, &m->moving, (size_t)mvox * 4));
     TRY_CUDA(cudaMemcpyAsync(m->fixed, fixed->data, (size_t)nvox * 4, cudaMemcpyDeviceToDevice, st));
     TRY_CUDA(cudaMemcpyAsync(m->moving, moving->data, (size_t)mvox * 4, cudaMemcpyDeviceToDevice, st));
     if (storage == MI_STORAGE_BF16) {
         // the metric sees the volume rounded to BF16 everywhere: the range, the exact
         // fallback's copy (the widened values) and the texture (the bits)
-        TRY_CUDA(cudaMalloc(&mbits, (size_t)mvox * 2));
+        TRY_CUDA(dev_alloc(ctx, &mbits, (size_t)mvox * 2));
         k_round_bf16<<<grid_for(mvox, 256, ctx->num_sms * 8), 256, 0, st>>>(m->moving, mvox, mbits);
         TRY_CUDA(cudaGetLastError());
     }
     if (moving_mask) {
-        TRY_CUDA(cudaMalloc(&m->mmask, (size_t)mvox));
+        TRY_CUDA(dev_alloc(ctx, &m->mmask, (size_t)mvox));
         TRY_CUDA(cudaMemcpyAsync(m->mmask, moving_mask, (size_t)mvox, cudaMemcpyHostToDevice, st));
     }
     mi_status s = build_samples(ctx, m, fixed_mask, sampling, nvox, mattes);
@@ -1237,7 +1240,6 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         // slice, whose cell corners come in two gathers, when the volume fits the
         // layered limits; else a block-linear 3-D array read by eight point fetches
         const bool b16 = storage == MI_STORAGE_BF16;
-        const cudaChannelFormatDesc fmt = b16 ? cudaCreateChannelDesc<unsigned short>() : cudaCreateChannelDesc<float>();
         const size_t esize = b16 ? 2 : 4;
         const cudaExtent ext = make_cudaExtent((size_t)moving->geo.size[0], (size_t)moving->geo.size[1],
                                                (size_t)moving->geo.size[2]);
@@ -1247,8 +1249,9 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         TRY_CUDA(cudaDeviceGetAttribute(&ll, cudaDevAttrMaxTexture2DLayeredLayers, ctx->device));
         const bool layered = moving->geo.size[0] <= lw && moving->geo.size[1] <= lh && moving->geo.size[2] <= ll &&
                              MOVING_LAYERED && texture == MI_TEXTURE_AUTO && mattes;
-        TRY_CUDA(cudaMalloc3DArray(&m->marray, &fmt, ext, layered ? cudaArrayLayered : 0));
         P.mlayered = layered ? 1 : 0;
+        P.mbf16 = b16 ? 1 : 0;
+        TRY_CUDA(array_alloc(ctx, &m->marray, ext, esize, layered));
         cudaMemcpy3DParms cp = {};
         cp.srcPtr = make_cudaPitchedPtr(b16 ? (void*)mbits : (void*)m->moving, (size_t)moving->geo.size[0] * esize,
                                         (size_t)moving->geo.size[0], (size_t)moving->geo.size[1]);
@@ -1258,11 +1261,10 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         const cudaError_t ce = cudaMemcpy3DAsync(&cp, st);
         if (mbits) {
             cudaStreamSynchronize(st);
-            cudaFree(mbits);
+            dev_free(ctx, mbits);
             mbits = nullptr;
         }
         TRY_CUDA(ce);
-        P.mbf16 = b16 ? 1 : 0;
         cudaResourceDesc res = {};
         res.resType = cudaResourceTypeArray;
         res.res.array.array = m->marray;
@@ -1303,7 +1305,7 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
     }
 
     // The exact fixed bin of every sample (a pure function of the fixed value).
-    TRY_CUDA(cudaMalloc(&m->fbin, pad4(m->n_samples)));
+    TRY_CUDA(dev_alloc(ctx, &m->fbin, pad4(m->n_samples)));
     k_fixed_bins<<<grid_for(m->n_samples, 256, ctx->num_sms * 8), 256, 0, st>>>(P, m->fixed, m->samples,
                                                                               m->n_samples, m->fbin);
     TRY_CUDA(cudaGetLastError());
@@ -1375,13 +1377,13 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
     {
         // padded to whole groups of four samples; padding records keep moving bin 0
         const size_t ns = pad4(m->n_samples);
-        TRY_CUDA(cudaMalloc(&ws.rec_bins, ns * sizeof(uint16_t)));
+        TRY_CUDA(dev_alloc(ctx, &ws.rec_bins, ns * sizeof(uint16_t)));
         TRY_CUDA(cudaMemsetAsync(ws.rec_bins, 0, ns * sizeof(uint16_t), st));
-        TRY_CUDA(cudaMalloc(&ws.rec_f, ns * sizeof(float)));
-        TRY_CUDA(cudaMalloc(&ws.rec_g, 3 * ns * sizeof(float)));
+        TRY_CUDA(dev_alloc(ctx, &ws.rec_f, ns * sizeof(float)));
+        TRY_CUDA(dev_alloc(ctx, &ws.rec_g, 3 * ns * sizeof(float)));
     }
     // joint B², fixed counts B, then the joint part's B column sums
-    TRY_CUDA(cudaMalloc(&ws.hist, ghist_bytes(B)));
+    TRY_CUDA(dev_alloc(ctx, &ws.hist, ghist_bytes(B)));
     TRY_CUDA(cudaMemsetAsync(ws.hist, 0, ghist_bytes(B), st));
     // partials serve both forms: the split form's k_deriv grid and, should the form
     // be switched, the fused grid
@@ -1390,9 +1392,9 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
             grid_for((int64_t)pad4(m->n_samples) / 4, DERIV_BLOCK, ctx->num_sms * std::max(occ_d, 1))));
         ws.grid_split_hist = ws.grid_hist;
         ws.grid_split_deriv = grid_for((int64_t)pad4(m->n_samples) / 4, DERIV_BLOCK, ctx->num_sms * std::max(occ_d, 1));
-        TRY_CUDA(cudaMalloc(&ws.partials, (size_t)pgrid * NMOM * 8));
+        TRY_CUDA(dev_alloc(ctx, &ws.partials, (size_t)pgrid * NMOM * 8));
     }
-    TRY_CUDA(cudaMalloc(&ws.vsum, (size_t)value_slices(B) * 8));
+    TRY_CUDA(dev_alloc(ctx, &ws.vsum, (size_t)value_slices(B) * 8));
     {
         // a grid-stride walk gives a CTA at most ceil(n / (grid·block))·block samples
         auto cap = [&](int grid) -> uint32_t {
@@ -1403,15 +1405,15 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         ws.exq_cap_hist = cap(ws.grid_hist);
         ws.exq_cap_eval = cap(ws.grid_eval);
         const size_t len = std::max((size_t)ws.grid_hist * ws.exq_cap_hist, (size_t)ws.grid_eval * ws.exq_cap_eval);
-        TRY_CUDA(cudaMalloc(&ws.exq, std::max<size_t>(len, 1) * sizeof(uint32_t)));
+        TRY_CUDA(dev_alloc(ctx, &ws.exq, std::max<size_t>(len, 1) * sizeof(uint32_t)));
     }
-    TRY_CUDA(cudaMalloc(&ws.result, RESULT_DOUBLES * 8));
-    TRY_CUDA(cudaMalloc(&ws.done_counter, 4 * sizeof(unsigned int)));
+    TRY_CUDA(dev_alloc(ctx, &ws.result, RESULT_DOUBLES * 8));
+    TRY_CUDA(dev_alloc(ctx, &ws.done_counter, 4 * sizeof(unsigned int)));
     TRY_CUDA(cudaMemsetAsync(ws.done_counter, 0, 4 * sizeof(unsigned int), st));
     TRY_CUDA(cudaMemsetAsync(ws.result, 0, RESULT_DOUBLES * 8, st));
-    TRY_CUDA(cudaHostAlloc(&ws.host_result, RESULT_DOUBLES * 8, cudaHostAllocMapped));
+    static_assert(RESULT_DOUBLES * 8 <= PINNED_BLOCK, "the result's mirror is one pinned block");
+    TRY_CUDA(pinned_alloc(ctx, reinterpret_cast<void**>(&ws.host_result), reinterpret_cast<void**>(&ws.host_result_dev)));
     std::memset(ws.host_result, 0, RESULT_DOUBLES * 8);  // no stale sequence number
-    TRY_CUDA(cudaHostGetDevicePointer(reinterpret_cast<void**>(&ws.host_result_dev), ws.host_result, 0));
     TRY_CUDA(cudaStreamSynchronize(st));
 #undef TRY_CUDA
     *out = m;
@@ -1567,11 +1569,11 @@ mi_status mi_metric_sample_decisions(mi_metric* m, const double* stages, int nst
     int32_t *d_fb = nullptr, *d_mb = nullptr;
     int64_t* d_fl = nullptr;
     cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaMalloc(&d_st, cap);
-    if (e == cudaSuccess) e = cudaMalloc(&d_ex, cap);
-    if (e == cudaSuccess) e = cudaMalloc(&d_fb, cap * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&d_mb, cap * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&d_fl, cap * 8);
+    cudaError_t e = dev_alloc(ctx, &d_st, cap);
+    if (e == cudaSuccess) e = dev_alloc(ctx, &d_ex, cap);
+    if (e == cudaSuccess) e = dev_alloc(ctx, &d_fb, cap * 4);
+    if (e == cudaSuccess) e = dev_alloc(ctx, &d_mb, cap * 4);
+    if (e == cudaSuccess) e = dev_alloc(ctx, &d_fl, cap * 8);
     if (e == cudaSuccess) {
         const int block = 256;
         k_decisions<<<grid_for(ns, block, ctx->num_sms * 8), block, 0, st>>>(P, m->moving, m->mmask, m->samples, m->fbin,
@@ -1584,11 +1586,11 @@ mi_status mi_metric_sample_decisions(mi_metric* m, const double* stages, int nst
     if (e == cudaSuccess && moving_bin) e = cudaMemcpyAsync(moving_bin, d_mb, (size_t)ns * 4, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess && flat) e = cudaMemcpyAsync(flat, d_fl, (size_t)ns * 8, cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_st);
-    cudaFree(d_ex);
-    cudaFree(d_fb);
-    cudaFree(d_mb);
-    cudaFree(d_fl);
+    dev_free(ctx, d_st);
+    dev_free(ctx, d_ex);
+    dev_free(ctx, d_fb);
+    dev_free(ctx, d_mb);
+    dev_free(ctx, d_fl);
     if (e != cudaSuccess) return cuda_status(ctx, e, "mi_metric_sample_decisions");
     return MI_OK;
 }

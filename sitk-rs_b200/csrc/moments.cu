@@ -282,29 +282,30 @@ mi_status moments_setup(mi_metric* m) {
     const int64_t n = std::max<int64_t>(m->n_samples, 1);
     w.grid = (int)std::max<int64_t>(1, std::min<int64_t>((n + MOM_BLOCK - 1) / MOM_BLOCK, (int64_t)ctx->num_sms * occ));
     cudaStream_t st = ctx->stream;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&w.partials, (size_t)w.grid * NCC2_SLOTS * sizeof(double)));
-    MI_CHECK_CUDA(ctx, cudaMalloc(&w.result, 2 * NCC2_SLOTS * sizeof(double)));
-    MI_CHECK_CUDA(ctx, cudaMalloc(&w.counter, 2 * sizeof(unsigned int)));
+    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &w.partials, (size_t)w.grid * NCC2_SLOTS * sizeof(double)));
+    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &w.result, 2 * NCC2_SLOTS * sizeof(double)));
+    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &w.counter, 2 * sizeof(unsigned int)));
     MI_CHECK_CUDA(ctx, cudaMemsetAsync(w.counter, 0, 2 * sizeof(unsigned int), st));
     MI_CHECK_CUDA(ctx, cudaMemsetAsync(w.result, 0, 2 * NCC2_SLOTS * sizeof(double), st));
     if (m->samples && m->n_samples > 0) {
-        MI_CHECK_CUDA(ctx, cudaMalloc(&w.fval, (size_t)m->n_samples * sizeof(float)));
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &w.fval, (size_t)m->n_samples * sizeof(float)));
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>((m->n_samples + 255) / 256, (int64_t)ctx->num_sms * 8));
         k_gather_fixed<<<g, 256, 0, st>>>(m->fixed, m->samples, m->n_samples, w.fval);
         MI_CHECK_CUDA(ctx, cudaGetLastError());
     }
-    MI_CHECK_CUDA(ctx, cudaHostAlloc(&w.host, NCC2_SLOTS * sizeof(double), cudaHostAllocMapped));
-    MI_CHECK_CUDA(ctx, cudaHostGetDevicePointer(reinterpret_cast<void**>(&w.host_dev), w.host, 0));
+    static_assert(NCC2_SLOTS * sizeof(double) <= PINNED_BLOCK, "the moments' mirror is one pinned block");
+    MI_CHECK_CUDA(ctx, pinned_alloc(ctx, reinterpret_cast<void**>(&w.host), reinterpret_cast<void**>(&w.host_dev)));
     return MI_OK;
 }
 
 void moments_free(mi_metric* m) {
+    mi_context* ctx = m->ctx;
     MomentsWs& w = m->mom;
-    cudaFree(w.partials);
-    cudaFree(w.result);
-    cudaFree(w.counter);
-    cudaFree(w.fval);
-    if (w.host) cudaFreeHost(w.host);
+    dev_free(ctx, w.partials);
+    dev_free(ctx, w.result);
+    dev_free(ctx, w.counter);
+    dev_free(ctx, w.fval);
+    pinned_free(ctx, w.host);
     w = MomentsWs{};
 }
 

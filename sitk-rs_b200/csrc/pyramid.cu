@@ -479,10 +479,10 @@ mi_status gauss_axis(mi_context* ctx, const TI* in, double* mid, TO* out, const 
 mi_status new_image(mi_context* ctx, const mi_geometry& geo, mi_image** out) {
     const int64_t n = geo.size[0] * geo.size[1] * geo.size[2];
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&d, (size_t)n * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)n * sizeof(float)));
     mi_image* img = new (std::nothrow) mi_image();
     if (!img) {
-        cudaFree(d);
+        mi::dev_free(ctx, d);
         return MI_ERR_OUT_OF_MEMORY;
     }
     img->ctx = ctx;
@@ -532,9 +532,9 @@ mi_status mi_image_smooth(mi_context* ctx, const mi_image* in, const double* sig
         }
     double* v[3] = {nullptr, nullptr, nullptr};  // the two volumes, the long lines' scratch
     cudaError_t e = cudaSuccess;
-    if (na > 1) e = cudaMalloc(&v[0], (size_t)n * 8);
-    if (e == cudaSuccess && na > 2) e = cudaMalloc(&v[1], (size_t)n * 8);
-    if (e == cudaSuccess && need_mid) e = cudaMalloc(&v[2], (size_t)n * 8);
+    if (na > 1) e = mi::dev_alloc(ctx, &v[0], (size_t)n * 8);
+    if (e == cudaSuccess && na > 2) e = mi::dev_alloc(ctx, &v[1], (size_t)n * 8);
+    if (e == cudaSuccess && need_mid) e = mi::dev_alloc(ctx, &v[2], (size_t)n * 8);
     if (e == cudaSuccess && na == 0) e = cudaMemcpyAsync(res->data, in->data, (size_t)n * 4, cudaMemcpyDeviceToDevice, st);
     for (int i = 0; i < na && e == cudaSuccess && s == MI_OK; ++i) {
         const int d = axes[i];
@@ -551,7 +551,7 @@ mi_status mi_image_smooth(mi_context* ctx, const mi_image* in, const double* sig
             s = gauss_axis(ctx, v[(i - 1) & 1], v[2], v[i & 1], g.size, d, C);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    for (double* p : v) cudaFree(p);
+    for (double* p : v) mi::dev_free(ctx, p);
     if (e != cudaSuccess || s != MI_OK) {
         mi_image_free(res);
         return e != cudaSuccess ? mi::cuda_status(ctx, e, "mi_image_smooth") : s;

@@ -113,10 +113,10 @@ mi_status new_cube(mi_context* ctx, int n, mi_image** out) {
     g.direction[0] = g.direction[4] = g.direction[8] = 1.0;
     const int64_t nv = (int64_t)n * n * n;
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, cudaMalloc(&d, (size_t)nv * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)nv * sizeof(float)));
     mi_image* img = new (std::nothrow) mi_image();
     if (!img) {
-        cudaFree(d);
+        mi::dev_free(ctx, d);
         return MI_ERR_OUT_OF_MEMORY;
     }
     img->ctx = ctx;
@@ -161,9 +161,9 @@ mi_status mi_synth_pair(mi_context* ctx, int n, int nblobs, const double* blobs5
     Blob* db = nullptr;
     double* base = nullptr;
     cudaStream_t st = ctx->stream;
-    cudaError_t e = cudaMalloc(&db, hb.size() * sizeof(Blob));
+    cudaError_t e = mi::dev_alloc(ctx, &db, hb.size() * sizeof(Blob));
     if (e == cudaSuccess) e = cudaMemcpyAsync(db, hb.data(), hb.size() * sizeof(Blob), cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMalloc(&base, (size_t)nv * sizeof(double));
+    if (e == cudaSuccess) e = mi::dev_alloc(ctx, &base, (size_t)nv * sizeof(double));
     const unsigned long long kf = mix64((unsigned long long)seed + 1ull * GAMMA);
     const unsigned long long km = mix64((unsigned long long)seed + 2ull * GAMMA);
     const int grid = (int)std::min<long long>((nv + 255) / 256, (long long)ctx->num_sms * 16);
@@ -178,8 +178,8 @@ mi_status mi_synth_pair(mi_context* ctx, int n, int nblobs, const double* blobs5
         e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(db);
-    cudaFree(base);
+    mi::dev_free(ctx, db);
+    mi::dev_free(ctx, base);
     if (e != cudaSuccess) {
         mi_image_free(f);
         mi_image_free(m);
