@@ -6,6 +6,7 @@
 // to_host (cuda/image.rs:269-280). Complex and vector pixels are refused by name.
 
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -43,6 +44,21 @@ mi_status raise_smem_limit(mi_context* ctx, const void* fn, size_t bytes) {
     if (e != cudaSuccess) return cuda_status(ctx, e, "cudaFuncSetAttribute");
     cur = bytes;
     return MI_OK;
+}
+
+// The tensor-map encoder of the driver (cuTensorMapEncodeTiled), found once.
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
+    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
+        void* p = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
+        }
+        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
+    }();
+    return fn;
 }
 
 // What an object gives back is kept for the next one. On the B200 a cudaMalloc / cudaFree

@@ -153,7 +153,7 @@ k_gemm_tn(int M, int N, int K, const __nv_bfloat16* __restrict__ A, int lda, con
         }
         // a CTA-wide decision, so every thread leaves the loop (or not) together
         ok = __syncthreads_and(done != 0) != 0;
-        if (!ok && threadIdx.x == 0) atomicOr(err, 1u);
+        if (!ok && threadIdx.x == 0) *reinterpret_cast<volatile unsigned int*>(err) = 1u;
         phase ^= 1u;
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     }

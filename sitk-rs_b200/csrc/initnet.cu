@@ -22,12 +22,10 @@
 #include <vector>
 
 #include "gemm_tc.cuh"
+#include "gemm_tma.cuh"
 #include "internal.h"
 
 namespace mi {
-
-cudaError_t gemm_bf16_tn(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-                         float* C, int ldc, unsigned int* err, cudaStream_t st);
 
 namespace {
 
@@ -44,8 +42,60 @@ cudaError_t launch_gemm(int M, int N, int K, const __nv_bfloat16* A, int lda, co
 
 int n_tile(int N) { return N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128; }
 
-cudaError_t gemm_dispatch(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-                          float* C, int ldc, int splits, unsigned int* err, cudaStream_t st) {
+// A row-major BF16 matrix [rows][K] in tiles of `box` rows × 64 k, 128-byte swizzle; k and
+// rows past the ends read as zero. False where TMA cannot read it (row pitch or base
+// not a multiple of 16 bytes).
+bool operand_map(CUtensorMap* map, const __nv_bfloat16* p, int rows, int K, int ld, int box) {
+    if (ld % 8 != 0 || ((uintptr_t)p & 15) != 0 || !tensor_map_encoder()) return false;
+    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
+    const cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
+    const cuuint32_t bx[2] = {(cuuint32_t)tc::TILE_K, (cuuint32_t)box}, es[2] = {1, 1};
+    return tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dim, stride, bx,
+                                es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
+template <int NT>
+cudaError_t launch_tma(mi_context* ctx, int M, int N, int K, const CUtensorMap& a, const CUtensorMap& b, float* C,
+                       int ldc, int splits, unsigned int* err) {
+    constexpr uint32_t sm = tc::TmaShape<NT>::SMEM;
+    if (raise_smem_limit(ctx, (const void*)tc::k_gemm_tma<NT>, sm) != MI_OK) return cudaErrorInvalidValue;
+    const int64_t items = (int64_t)((M + tc::TILE_M - 1) / tc::TILE_M) * ((N + NT - 1) / NT) * splits;
+    const int grid = (int)std::min<int64_t>(items, ctx->num_sms);
+    tc::k_gemm_tma<NT><<<grid, tc::TMA_THREADS, sm, ctx->stream>>>(a, b, M, N, K, C, ldc, splits, err);
+    return cudaGetLastError();
+}
+
+// The N tile of the TMA kernel. Its tiles are 128 × 256 where that leaves at least as few
+// columns of padding and as full a last round of CTAs as 128 × 128, which needs half
+// as much again of shared-memory bandwidth per product.
+int tma_n_tile(mi_context* ctx, int M, int N, int splits) {
+    if (N <= 128) return n_tile(N);
+    const int64_t mt = (M + tc::TILE_M - 1) / tc::TILE_M;
+    auto rounds = [&](int nt) {
+        const int64_t items = mt * ((N + nt - 1) / nt) * splits;
+        return (items + ctx->num_sms - 1) / ctx->num_sms;
+    };
+    return 2 * rounds(256) * 3 <= rounds(128) * 4 ? 256 : 128;
+}
+
+// C, or with splits > 1 the K slices' partial products one after another (M × ldc each).
+// TMA operands go to k_gemm_tma; others, whose rows only plain loads can read, to
+// k_gemm_tn. Same slices, same order of accumulation, same bits.
+cudaError_t gemm_dispatch(mi_context* ctx, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
+                          int ldb, float* C, int ldc, int splits, unsigned int* err) {
+    const int nt = tma_n_tile(ctx, M, N, splits);
+    CUtensorMap a, b;
+    if (operand_map(&a, A, M, K, lda, tc::TILE_M) && operand_map(&b, B, N, K, ldb, nt)) {
+        switch (nt) {
+            case 16: return launch_tma<16>(ctx, M, N, K, a, b, C, ldc, splits, err);
+            case 32: return launch_tma<32>(ctx, M, N, K, a, b, C, ldc, splits, err);
+            case 64: return launch_tma<64>(ctx, M, N, K, a, b, C, ldc, splits, err);
+            case 128: return launch_tma<128>(ctx, M, N, K, a, b, C, ldc, splits, err);
+            default: return launch_tma<256>(ctx, M, N, K, a, b, C, ldc, splits, err);
+        }
+    }
+    cudaStream_t st = ctx->stream;
     switch (n_tile(N)) {
         case 16: return launch_gemm<16>(M, N, K, A, lda, B, ldb, C, ldc, splits, err, st);
         case 32: return launch_gemm<32>(M, N, K, A, lda, B, ldb, C, ldc, splits, err, st);
@@ -53,16 +103,6 @@ cudaError_t gemm_dispatch(int M, int N, int K, const __nv_bfloat16* A, int lda, 
         default: return launch_gemm<128>(M, N, K, A, lda, B, ldb, C, ldc, splits, err, st);
     }
 }
-
-}  // namespace
-
-// C[M×N] = A[M×K]·B[N×K]ᵀ on the stream; the N tile follows N.
-cudaError_t gemm_bf16_tn(int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-                         float* C, int ldc, unsigned int* err, cudaStream_t st) {
-    return gemm_dispatch(M, N, K, A, lda, B, ldb, C, ldc, 1, err, st);
-}
-
-namespace {
 
 constexpr int NCONV = 4;
 constexpr int CH[NCONV + 1] = {2, 16, 32, 64, 128};
@@ -312,7 +352,8 @@ struct mi_initnet {
     float *dz = nullptr, *dx = nullptr, *dcol = nullptr, *part = nullptr, *loss = nullptr;
     __nv_bfloat16 *dzb = nullptr, *tA = nullptr, *tB = nullptr;
     float* slices = nullptr;  // split-K partial products
-    unsigned int* err = nullptr;
+    unsigned int* err = nullptr;    // pinned host word a GEMM raises when a wait gives up, and
+    unsigned int* err_dev = nullptr;  // its device address
 };
 
 namespace mi {
@@ -351,7 +392,7 @@ void free_net(mi_initnet* n) {
     mi::dev_free(ctx, n->tA);
     mi::dev_free(ctx, n->tB);
     mi::dev_free(ctx, n->slices);
-    mi::dev_free(ctx, n->err);
+    pinned_free(ctx, n->err);
     delete n;
 }
 
@@ -372,8 +413,8 @@ cudaError_t mm(mi_initnet* n, int M, int N, int K, const __nv_bfloat16* A, int l
                float* C) {
     cudaStream_t st = n->ctx->stream;
     const int S = k_splits(M, N, K);
-    if (S == 1) return gemm_dispatch(M, N, K, A, lda, B, ldb, C, N, 1, n->err, st);
-    cudaError_t e = gemm_dispatch(M, N, K, A, lda, B, ldb, n->slices, N, S, n->err, st);
+    if (S == 1) return gemm_dispatch(n->ctx, M, N, K, A, lda, B, ldb, C, N, 1, n->err_dev);
+    cudaError_t e = gemm_dispatch(n->ctx, M, N, K, A, lda, B, ldb, n->slices, N, S, n->err_dev);
     if (e != cudaSuccess) return e;
     k_sum_slices<<<grid1((int64_t)M * N), 256, 0, st>>>(n->slices, S, (int64_t)M * N, C);
     return cudaGetLastError();
@@ -555,7 +596,8 @@ mi_status mi_initnet_create(mi_context* ctx, uint64_t seed, int max_batch, mi_in
     alloc(&n->dzb, max_act * 2);
     alloc(&n->tA, std::max(max_rows_out, max_act) * 2);
     alloc(&n->tB, max_rows_kp * 2);
-    alloc(&n->err, 4);
+    if (e == cudaSuccess) e = pinned_alloc(ctx, (void**)&n->err, (void**)&n->err_dev);
+    if (e == cudaSuccess) *n->err = 0u;
     if (e == cudaSuccess) e = mi::refresh_bf16(n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
@@ -602,12 +644,10 @@ mi_status mi_initnet_set(mi_initnet* n, int which, const float* w, const float* 
 }
 
 static mi_status check_err(mi_initnet* n, cudaError_t e, const char* where) {
-    unsigned int h = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, n->err, 4, cudaMemcpyDeviceToHost, n->ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->ctx->stream);
     if (e != cudaSuccess) return mi::cuda_status(n->ctx, e, where);
-    if (h) {
-        cudaMemsetAsync(n->err, 0, 4, n->ctx->stream);
+    if (*n->err) {
+        *n->err = 0u;
         return mi::set_error(n->ctx, MI_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait gave up");
     }
     return MI_OK;
@@ -688,9 +728,9 @@ mi_status mi_gemm_bf16_tn(mi_context* ctx, int M, int N, int K, const void* A, i
     if (!ctx || M < 1 || N < 1 || K < 1 || !A || !B || !C || lda < K || ldb < K || ldc < N)
         return MI_ERR_INVALID_ARGUMENT;
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
-    unsigned int* err = nullptr;
-    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &err, sizeof(unsigned int)));
-    cudaError_t e = cudaMemsetAsync(err, 0, sizeof(unsigned int), ctx->stream);
+    unsigned int *err = nullptr, *err_dev = nullptr;  // a pinned word and its device address
+    cudaError_t e = mi::pinned_alloc(ctx, (void**)&err, (void**)&err_dev);
+    if (e == cudaSuccess) *err = 0u;
     // a product whose M × N tiles alone would leave most SMs idle is split over K into
     // partial products summed in slice order, as the network's layers do
     const int S = ldc == N ? mi::k_splits(M, N, K) : 1;
@@ -699,19 +739,18 @@ mi_status mi_gemm_bf16_tn(mi_context* ctx, int M, int N, int K, const void* A, i
     const auto* a16 = static_cast<const __nv_bfloat16*>(A);
     const auto* b16 = static_cast<const __nv_bfloat16*>(B);
     if (e == cudaSuccess && S > 1) {
-        e = mi::gemm_dispatch(M, N, K, a16, lda, b16, ldb, slices, N, S, err, ctx->stream);
+        e = mi::gemm_dispatch(ctx, M, N, K, a16, lda, b16, ldb, slices, N, S, err_dev);
         if (e == cudaSuccess) {
             mi::k_sum_slices<<<mi::grid1((int64_t)M * N), 256, 0, ctx->stream>>>(slices, S, (int64_t)M * N, C);
             e = cudaGetLastError();
         }
     } else if (e == cudaSuccess) {
-        e = mi::gemm_bf16_tn(M, N, K, a16, lda, b16, ldb, C, ldc, err, ctx->stream);
+        e = mi::gemm_dispatch(ctx, M, N, K, a16, lda, b16, ldb, C, ldc, 1, err_dev);
     }
-    unsigned int h = 0;
-    if (e == cudaSuccess) e = cudaMemcpyAsync(&h, err, sizeof(h), cudaMemcpyDeviceToHost, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
+    const unsigned int h = err ? *reinterpret_cast<volatile unsigned int*>(err) : 0u;
     mi::dev_free(ctx, slices);
-    mi::dev_free(ctx, err);
+    mi::pinned_free(ctx, err);
     if (e != cudaSuccess) return mi::cuda_status(ctx, e, "mi_gemm_bf16_tn");
     if (h) return mi::set_error(ctx, MI_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait gave up");
     return MI_OK;

@@ -2,6 +2,7 @@
 #pragma once
 
 #include <cuda_runtime.h>
+#include <cudaTypedefs.h>
 #include <cstdint>
 #include <list>
 #include <mutex>
@@ -225,6 +226,9 @@ namespace mi {
 
 mi_status set_error(mi_context* ctx, mi_status s, const std::string& msg);
 mi_status cuda_status(mi_context* ctx, cudaError_t e, const char* where);
+// The driver's cuTensorMapEncodeTiled, or null.
+PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
+
 // Device memory from the context's pool, ordered on the context's stream: a block may be
 // freed while work on that stream still uses it, and what reuses it comes after that
 // work. Memory that another stream touches is freed only once that stream is done.

@@ -772,21 +772,6 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
     return done(MI_OK);
 }
 
-// The tensor-map encoder of the driver (cuTensorMapEncodeTiled), found once.
-PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
-    static const PFN_cuTensorMapEncodeTiled_v12000 fn = [] {
-        void* p = nullptr;
-        cudaDriverEntryPointQueryResult q;
-        if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &p, cudaEnableDefault, &q) != cudaSuccess ||
-            q != cudaDriverEntryPointSuccess) {
-            cudaGetLastError();
-            return (PFN_cuTensorMapEncodeTiled_v12000) nullptr;
-        }
-        return reinterpret_cast<PFN_cuTensorMapEncodeTiled_v12000>(p);
-    }();
-    return fn;
-}
-
 // The staged-tile pass's shape (tile.cuh): whether the linear moving volume meets the
 // tensor-map rules (row pitch a multiple of 16 bytes), its grid (one CTA per SM), and the
 // most samples one of its threads takes: over the CTAs' contiguous chunk ranges, the
