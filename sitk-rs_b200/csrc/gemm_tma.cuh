@@ -20,6 +20,10 @@
 // 4096³: 137 µs a call (1,005 TFLOP/s, 0.63 of 1.59 PFLOP/s; four rounds of CTAs for 3.46
 // rounds of tiles); the one-stage kernel of gemm_tc.cuh took 1,489 µs.
 //
+// An operand may also be stored the other way round, k slowest ("k-rows": element (r, k) at
+// k·ld + r, as a product's transpose needs it): its tiles come as boxes of 64 rows × 64 k
+// and the instruction reads them MN-major, so nothing is transposed beforehand.
+//
 // Every wait is bounded: a role that gives up raises *err (a word the host can read, so the
 // call needs no copy back) and leaves, the others follow
 // (their own waits see the flag), the copies in flight are waited for and the tensor
@@ -92,6 +96,25 @@ __device__ __forceinline__ uint64_t swizzled_desc(uint32_t addr) {
     return (uint64_t)((addr >> 4) & 0x3FFFu) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) | (2ull << 61);
 }
 
+// The same of an MN-major tile (boxes of 64 rows × 64 k: 128-byte lines of 64 rows, one k
+// each): 8192 bytes from one 64 rows to the next, 1024 from eight k to the next.
+__device__ __forceinline__ uint64_t swizzled_desc_mn(uint32_t addr) {
+    return (uint64_t)((addr >> 4) & 0x3FFFu) | ((uint64_t)(8192 >> 4) << 16) | ((uint64_t)(1024 >> 4) << 32) | (1ull << 46) |
+           (2ull << 61);
+}
+
+// What becomes of an element z of the product: stored in C (where not null), and with X as
+// BF16 of z + bias[column], negative values cut off when relu is set. With a bias C gets
+// z + bias. Splits store the plain partial products.
+struct Epilogue {
+    float* C;
+    int ldc;
+    const float* bias;
+    __nv_bfloat16* X;
+    int ldx;
+    int relu;
+};
+
 // Work item `item`: K slices slowest, then columns, rows fastest (CTAs that run together
 // share a B tile and the A tiles stay in L2).
 struct Item {
@@ -108,10 +131,22 @@ __device__ __forceinline__ Item item_at(int item, int mt, int nt, int ktiles, in
     return w;
 }
 
-template <int NT>
+// `rows` rows from `row` at 64 k from `k` into dst.
+template <int ROWS, bool KROWS>
+__device__ __forceinline__ void request_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, int k, int row) {
+    if (!KROWS) {
+        tma_tile(dst, map, bar, k, row);
+    } else {
+#pragma unroll
+        for (int r = 0; r < ROWS; r += 64) tma_tile(dst + r * 128, map, bar, row + r, k);
+    }
+}
+
+template <int NT, bool A_KROWS, bool B_KROWS>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
 k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int M, int N, int K,
-           float* __restrict__ C, int ldc, int splits, unsigned int* __restrict__ err) {
+           const Epilogue E, int splits, unsigned int* __restrict__ err) {
+    static_assert(!B_KROWS || NT % 64 == 0, "k-rows tiles come in boxes of 64");
     using S = TmaShape<NT>;
     extern __shared__ uint8_t raw[];
     __shared__ uint32_t tmem_slot;
@@ -162,8 +197,8 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                     }
                     const uint32_t dst = base + s * S::STAGE;
                     bar_expect(full + s * 8, S::STAGE);
-                    tma_tile(dst, &mapA, full + s * 8, kt * TILE_K, w.m0);
-                    tma_tile(dst + S::A_BYTES, &mapB, full + s * 8, kt * TILE_K, w.n0);
+                    request_tile<TILE_M, A_KROWS>(dst, &mapA, full + s * 8, kt * TILE_K, w.m0);
+                    request_tile<NT, B_KROWS>(dst + S::A_BYTES, &mapB, full + s * 8, kt * TILE_K, w.n0);
                 }
             }
             if (!ok) {
@@ -176,7 +211,10 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         __syncwarp();
     } else if (warp == 1) {
         if (lane == 0) {
-            const uint32_t idesc = instr_desc(TILE_M, NT);
+            // bits 15 and 16: A and B are MN-major
+            const uint32_t idesc = instr_desc(TILE_M, NT) | (A_KROWS ? 1u << 15 : 0u) | (B_KROWS ? 1u << 16 : 0u);
+            // sixteen k further: 32 bytes inside the swizzled rows, or two groups of eight k
+            constexpr uint64_t A_STEP = A_KROWS ? 2048 >> 4 : 32 >> 4, B_STEP = B_KROWS ? 2048 >> 4 : 32 >> 4;
             uint32_t count = 0, tiles = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
@@ -192,18 +230,18 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                         break;
                     }
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                    const uint64_t ad = swizzled_desc(base + s * S::STAGE);
-                    const uint64_t bd = swizzled_desc(base + s * S::STAGE + S::A_BYTES);
+                    const uint32_t at = base + s * S::STAGE, bt = at + S::A_BYTES;
+                    const uint64_t ad = A_KROWS ? swizzled_desc_mn(at) : swizzled_desc(at);
+                    const uint64_t bd = B_KROWS ? swizzled_desc_mn(bt) : swizzled_desc(bt);
 #pragma unroll
                     for (int q = 0; q < TILE_K / 16; ++q) {
-                        // sixteen k further: 32 bytes inside the swizzled rows
                         const uint32_t acc = (kt > w.kt0 || q > 0) ? 1u : 0u;
                         asm volatile(
                             "{\n\t.reg .pred p;\n\t"
                             "setp.ne.b32 p, %4, 0;\n\t"
                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
                             "}" ::"r"(tmem + a * NT),
-                            "l"(ad + q * 2), "l"(bd + q * 2), "r"(idesc), "r"(acc));
+                            "l"(ad + q * A_STEP), "l"(bd + q * B_STEP), "r"(idesc), "r"(acc));
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                      empty + s * 8)
@@ -226,7 +264,8 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     } else {
         const int quad = warp & 3;  // the tensor-memory lanes this warp can read
         float* block = reinterpret_cast<float*>(raw + (epi - smem_u32(raw))) + (warp - 2) * 32 * 36;
-        const bool vec = (ldc & 3) == 0 && ((uintptr_t)C & 15) == 0;
+        const int ldc = E.ldc;
+        const bool vec = (ldc & 3) == 0 && ((uintptr_t)E.C & 15) == 0;
         uint32_t tiles = 0;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const Item w = item_at<NT>(it, mt, nt, ktiles, per);
@@ -236,7 +275,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                 if (!__all_sync(0xffffffffu, bar_wait(tfull + a * 8, (tiles >> 1) & 1, &quit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
-            float* out = C + (size_t)w.z * M * ldc;
+            float* out = E.C + (size_t)w.z * M * ldc;
             constexpr int W = NT < 32 ? NT : 32;  // columns a block
             const int row0 = w.m0 + quad * 32;
 #pragma unroll 1
@@ -273,9 +312,20 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                 for (int i = 0; i < 32; i += ROWS) {
                     const int rr = i + lane / PER_ROW, row = row0 + rr;
                     if (row < M) {
-                        const float4 v = *reinterpret_cast<const float4*>(block + rr * 36 + q);
+                        float4 v = *reinterpret_cast<const float4*>(block + rr * 36 + q);
                         float* dst = out + (size_t)row * ldc + col;
-                        if (vec && col + 4 <= N) {
+                        if (E.bias && col + 4 <= N) {  // the layers' widths are multiples of four
+                            const float4 b = __ldg(reinterpret_cast<const float4*>(E.bias + col));
+                            v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
+                            if (E.X) {
+                                if (E.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
+                                const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
+                                *reinterpret_cast<uint2*>(E.X + (size_t)row * E.ldx + col) =
+                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
+                            }
+                        }
+                        if (!E.C) {
+                        } else if (vec && col + 4 <= N) {
                             *reinterpret_cast<float4*>(dst) = v;
                         } else {
                             if (col < N) dst[0] = v.x;

@@ -42,27 +42,35 @@ cudaError_t launch_gemm(int M, int N, int K, const __nv_bfloat16* A, int lda, co
 
 int n_tile(int N) { return N <= 16 ? 16 : N <= 32 ? 32 : N <= 64 ? 64 : 128; }
 
-// A row-major BF16 matrix [rows][K] in tiles of `box` rows × 64 k, 128-byte swizzle; k and
-// rows past the ends read as zero. False where TMA cannot read it (row pitch or base
-// not a multiple of 16 bytes).
-bool operand_map(CUtensorMap* map, const __nv_bfloat16* p, int rows, int K, int ld, int box) {
-    if (ld % 8 != 0 || ((uintptr_t)p & 15) != 0 || !tensor_map_encoder()) return false;
-    const cuuint64_t dim[2] = {(cuuint64_t)K, (cuuint64_t)rows};
-    const cuuint64_t stride[1] = {(cuuint64_t)ld * 2};
-    const cuuint32_t bx[2] = {(cuuint32_t)tc::TILE_K, (cuuint32_t)box}, es[2] = {1, 1};
-    return tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(p), dim, stride, bx,
+// One operand of a product: element (r, k) at r·ld + k, or with k_rows at k·ld + r.
+struct Operand {
+    const __nv_bfloat16* p;
+    int ld;
+    bool k_rows;
+};
+
+// The operand's tiles, `box` rows × 64 k (64 × 64 with k_rows), 128-byte swizzle; k and rows
+// past the ends read as zero. False where TMA cannot read it (pitch or base not a
+// multiple of 16 bytes).
+bool operand_map(CUtensorMap* map, const Operand& o, int rows, int K, int box) {
+    if (o.ld % 8 != 0 || ((uintptr_t)o.p & 15) != 0 || !tensor_map_encoder()) return false;
+    const cuuint64_t dim[2] = {(cuuint64_t)(o.k_rows ? rows : K), (cuuint64_t)(o.k_rows ? K : rows)};
+    const cuuint64_t stride[1] = {(cuuint64_t)o.ld * 2};
+    const cuuint32_t bx[2] = {64, (cuuint32_t)(o.k_rows ? 64 : box)}, es[2] = {1, 1};
+    static_assert(tc::TILE_K == 64, "tiles of 64 k");
+    return tensor_map_encoder()(map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<__nv_bfloat16*>(o.p), dim, stride, bx,
                                 es, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
-template <int NT>
-cudaError_t launch_tma(mi_context* ctx, int M, int N, int K, const CUtensorMap& a, const CUtensorMap& b, float* C,
-                       int ldc, int splits, unsigned int* err) {
+template <int NT, bool AK, bool BK>
+cudaError_t launch_tma(mi_context* ctx, int M, int N, int K, const CUtensorMap& a, const CUtensorMap& b,
+                       const tc::Epilogue& E, int splits, unsigned int* err) {
     constexpr uint32_t sm = tc::TmaShape<NT>::SMEM;
-    if (raise_smem_limit(ctx, (const void*)tc::k_gemm_tma<NT>, sm) != MI_OK) return cudaErrorInvalidValue;
+    if (raise_smem_limit(ctx, (const void*)tc::k_gemm_tma<NT, AK, BK>, sm) != MI_OK) return cudaErrorInvalidValue;
     const int64_t items = (int64_t)((M + tc::TILE_M - 1) / tc::TILE_M) * ((N + NT - 1) / NT) * splits;
     const int grid = (int)std::min<int64_t>(items, ctx->num_sms);
-    tc::k_gemm_tma<NT><<<grid, tc::TMA_THREADS, sm, ctx->stream>>>(a, b, M, N, K, C, ldc, splits, err);
+    tc::k_gemm_tma<NT, AK, BK><<<grid, tc::TMA_THREADS, sm, ctx->stream>>>(a, b, M, N, K, E, splits, err);
     return cudaGetLastError();
 }
 
@@ -79,22 +87,47 @@ int tma_n_tile(mi_context* ctx, int M, int N, int splits) {
     return 2 * rounds(256) * 3 <= rounds(128) * 4 ? 256 : 128;
 }
 
-// C, or with splits > 1 the K slices' partial products one after another (M × ldc each).
-// TMA operands go to k_gemm_tma; others, whose rows only plain loads can read, to
-// k_gemm_tn. Same slices, same order of accumulation, same bits.
-cudaError_t gemm_dispatch(mi_context* ctx, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
-                          int ldb, float* C, int ldc, int splits, unsigned int* err) {
-    const int nt = tma_n_tile(ctx, M, N, splits);
+// The product by TMA: E's outputs, or with splits > 1 the K slices' partial products one
+// after another in E.C (M × ldc each). cudaErrorNotSupported where TMA cannot read an
+// operand. Both operands may be k_rows, or B alone.
+cudaError_t product(mi_context* ctx, int M, int N, int K, const Operand& A, const Operand& B, const tc::Epilogue& E,
+                    int splits, unsigned int* err) {
+    int nt = tma_n_tile(ctx, M, N, splits);
+    if (B.k_rows) nt = std::max(nt, 64);
     CUtensorMap a, b;
-    if (operand_map(&a, A, M, K, lda, tc::TILE_M) && operand_map(&b, B, N, K, ldb, nt)) {
+    if (!operand_map(&a, A, M, K, tc::TILE_M) || !operand_map(&b, B, N, K, nt)) return cudaErrorNotSupported;
+#define MI_PRODUCT(NT, AK, BK) return launch_tma<NT, AK, BK>(ctx, M, N, K, a, b, E, splits, err)
+    if (A.k_rows) {
         switch (nt) {
-            case 16: return launch_tma<16>(ctx, M, N, K, a, b, C, ldc, splits, err);
-            case 32: return launch_tma<32>(ctx, M, N, K, a, b, C, ldc, splits, err);
-            case 64: return launch_tma<64>(ctx, M, N, K, a, b, C, ldc, splits, err);
-            case 128: return launch_tma<128>(ctx, M, N, K, a, b, C, ldc, splits, err);
-            default: return launch_tma<256>(ctx, M, N, K, a, b, C, ldc, splits, err);
+            case 64: MI_PRODUCT(64, true, true);
+            case 128: MI_PRODUCT(128, true, true);
+            default: MI_PRODUCT(256, true, true);
         }
     }
+    if (B.k_rows) {
+        switch (nt) {
+            case 64: MI_PRODUCT(64, false, true);
+            case 128: MI_PRODUCT(128, false, true);
+            default: MI_PRODUCT(256, false, true);
+        }
+    }
+    switch (nt) {
+        case 16: MI_PRODUCT(16, false, false);
+        case 32: MI_PRODUCT(32, false, false);
+        case 64: MI_PRODUCT(64, false, false);
+        case 128: MI_PRODUCT(128, false, false);
+        default: MI_PRODUCT(256, false, false);
+    }
+#undef MI_PRODUCT
+}
+
+// C = A·Bᵀ for operands of any pitch: those TMA cannot read take k_gemm_tn's plain loads.
+// Same slices, same order of accumulation, same bits.
+cudaError_t gemm_dispatch(mi_context* ctx, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
+                          int ldb, float* C, int ldc, int splits, unsigned int* err) {
+    const cudaError_t e = product(ctx, M, N, K, Operand{A, lda, false}, Operand{B, ldb, false},
+                                  tc::Epilogue{C, ldc, nullptr, nullptr, 0, 0}, splits, err);
+    if (e != cudaErrorNotSupported) return e;
     cudaStream_t st = ctx->stream;
     switch (n_tile(N)) {
         case 16: return launch_gemm<16>(M, N, K, A, lda, B, ldb, C, ldc, splits, err, st);
@@ -124,142 +157,136 @@ __global__ void k_to_bf16(const float* __restrict__ in, __nv_bfloat16* __restric
     GSTRIDE(i, n) out[i] = __float2bfloat16(in[i]);
 }
 
-// out[c][r] = in[r][c] (rows × cols in, cols × rows out), FP32 or BF16 in, BF16 out
-template <typename T>
-__global__ void k_transpose(const T* __restrict__ in, int rows, int cols, int ldi, __nv_bfloat16* __restrict__ out,
-                            int ldo) {
-    __shared__ float tile[32][33];
-    const int r0 = blockIdx.y * 32, c0 = blockIdx.x * 32;
-    for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-        const int r = r0 + dy, c = c0 + threadIdx.x;
-        tile[dy][threadIdx.x] = (r < rows && c < cols) ? (float)in[(int64_t)r * ldi + c] : 0.0f;
-    }
-    __syncthreads();
-    for (int dy = threadIdx.y; dy < 32; dy += blockDim.y) {
-        const int c = c0 + dy, r = r0 + threadIdx.x;
-        if (c < cols && r < rows) out[(int64_t)c * ldo + r] = __float2bfloat16(tile[threadIdx.x][dy]);
-    }
+__device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
+    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&v);
 }
 
-template <typename T>
-cudaError_t transpose(const T* in, int rows, int cols, int ldi, __nv_bfloat16* out, int ldo, cudaStream_t st) {
-    dim3 g((cols + 31) / 32, (rows + 31) / 32), b(32, 8);
-    k_transpose<T><<<g, b, 0, st>>>(in, rows, cols, ldi, out, ldo);
-    return cudaGetLastError();
-}
-
-// im2col of a channels-last volume (B × D³ × Cin, BF16) for a 3³ stride-2 pad-1
-// convolution: row (b, z, y, x) of the D/2 output grid, column ((kz·3+ky)·3+kx)·Cin + c
-__global__ void k_im2col(const __nv_bfloat16* __restrict__ x, int B, int D, int Cin, int kp,
-                         __nv_bfloat16* __restrict__ col) {
-    const int Do = D / 2;
-    const int64_t rows = (int64_t)B * Do * Do * Do;
-    GSTRIDE(i, rows * kp) {
-        const int64_t row = i / kp;
-        const int k = (int)(i - row * kp);
-        __nv_bfloat16 v = __float2bfloat16(0.0f);
-        if (k < 27 * Cin) {
-            const int c = k % Cin, t = k / Cin;
-            const int kx = t % 3, ky = (t / 3) % 3, kz = t / 9;
-            int64_t r = row;
-            const int xo = (int)(r % Do);
-            r /= Do;
-            const int yo = (int)(r % Do);
-            r /= Do;
-            const int zo = (int)(r % Do);
-            const int b = (int)(r / Do);
-            const int xi = 2 * xo + kx - 1, yi = 2 * yo + ky - 1, zi = 2 * zo + kz - 1;
-            if (xi >= 0 && xi < D && yi >= 0 && yi < D && zi >= 0 && zi < D)
-                v = x[((((int64_t)b * D + zi) * D + yi) * D + xi) * Cin + c];
-        }
-        col[i] = v;
-    }
-}
-
-// the transpose of im2col as a gather: dX(b, z, y, x, c) = Σ over the output voxels
-// and kernel taps that read it of dXcol (FP32), in a fixed order
-__global__ void k_col2im(const float* __restrict__ dcol, int B, int D, int Cin, int kp, float* __restrict__ dx) {
-    const int Do = D / 2;
-    const int64_t n = (int64_t)B * D * D * D * Cin;
+// im2col of a channels-last volume (B × D³ × CIN) for a 3³ stride-2 pad-1 convolution: row
+// (b, z, y, x) of the D/2 output grid, column ((kz·3+ky)·3+kx)·CIN + c, zeros to KP columns.
+// A thread fills eight columns (16 bytes): eight channels of one tap, or, in the first
+// layer, both channels of four taps, read from the FP32 input and rounded here. With
+// one column a thread and divisions by run-time sizes the two large layers took 138
+// and 131 µs for 64 pairs (29 MB written each).
+template <int D, int CIN, int KP, typename T>
+__global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, __nv_bfloat16* __restrict__ col) {
+    constexpr int Do = D / 2, PARTS = KP / 8;
+    const int64_t n = (int64_t)B * Do * Do * Do * PARTS;
     GSTRIDE(i, n) {
-        int64_t r = i;
-        const int c = (int)(r % Cin);
-        r /= Cin;
-        const int xi = (int)(r % D);
-        r /= D;
-        const int yi = (int)(r % D);
-        r /= D;
-        const int zi = (int)(r % D);
-        const int b = (int)(r / D);
+        const int part = (int)(i % PARTS);
+        const int64_t row = i / PARTS;
+        const int xo = (int)(row % Do), yo = (int)(row / Do % Do), zo = (int)(row / (Do * Do) % Do);
+        const int64_t b = row / (Do * Do * Do);
+        auto at = [&](int t) -> const T* {  // the input voxel under tap t, or null
+            const int xi = 2 * xo + t % 3 - 1, yi = 2 * yo + t / 3 % 3 - 1, zi = 2 * zo + t / 9 - 1;
+            if (t >= 27 || (unsigned)xi >= (unsigned)D || (unsigned)yi >= (unsigned)D || (unsigned)zi >= (unsigned)D)
+                return nullptr;
+            return x + (((b * D + zi) * D + yi) * D + xi) * CIN;
+        };
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if constexpr (CIN == 2) {
+            uint32_t w[4];
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const T* p = at(part * 4 + q);
+                const float2 f = p ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f);
+                w[q] = pack_bf16(f.x, f.y);
+            }
+            v = make_uint4(w[0], w[1], w[2], w[3]);
+        } else {
+            const T* p = at(part / (CIN / 8));
+            if (p) v = __ldg(reinterpret_cast<const uint4*>(p + part % (CIN / 8) * 8));
+        }
+        reinterpret_cast<uint4*>(col)[i] = v;
+    }
+}
+
+// The end of a layer's forward product that was split over K: the slices summed in order,
+// the bias, ReLU, BF16.
+__global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t mn, const float* __restrict__ bias,
+                             int cols, __nv_bfloat16* __restrict__ x) {
+    GSTRIDE(i, mn) {
         float acc = 0.0f;
-        for (int kz = 0; kz < 3; ++kz) {
-            const int tz = zi + 1 - kz;
-            if (tz < 0 || (tz & 1) || tz / 2 >= Do) continue;
-            for (int ky = 0; ky < 3; ++ky) {
-                const int ty = yi + 1 - ky;
-                if (ty < 0 || (ty & 1) || ty / 2 >= Do) continue;
-                for (int kx = 0; kx < 3; ++kx) {
-                    const int tx = xi + 1 - kx;
-                    if (tx < 0 || (tx & 1) || tx / 2 >= Do) continue;
-                    const int64_t row = (((int64_t)b * Do + tz / 2) * Do + ty / 2) * Do + tx / 2;
-                    acc += dcol[row * kp + ((kz * 3 + ky) * 3 + kx) * Cin + c];
+        for (int s = 0; s < splits; ++s) acc += part[(int64_t)s * mn + i];
+        x[i] = __float2bfloat16(fmaxf(acc + bias[i % cols], 0.0f));
+    }
+}
+
+// The gradient dZ of the layer below from that of a layer's input: dx through the ReLU (its
+// output a is positive where its input was), as BF16 for the next products, and the
+// CTA's column sums (the bias gradient) of the FP32 values into part[CTA]. dx comes
+// from the layer's product dcol: for a fully connected layer it is dcol itself (D = 0); for
+// a convolution over D³ inputs of C channels it is the transpose of im2col as a gather,
+// the output voxels and taps that read the input voxel, in a fixed order. A thread keeps
+// four channels, so that its sums stay in registers. (Gather, ReLU, conversion and sums
+// were five launches; the sums, 4,096 rows a thread in order, took 0.9–1.1 ms each.)
+template <int D, int C, int KP>
+__global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol, const __nv_bfloat16* __restrict__ a,
+                                                  int64_t rows, __nv_bfloat16* __restrict__ dzb, float* __restrict__ part) {
+    constexpr int G = C / 4;  // threads a row
+    static_assert(256 % G == 0, "a thread's channels stay the same");
+    __shared__ float4 sums[256];
+    const int c = (threadIdx.x % G) * 4;
+    float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) / G; r < rows; r += (int64_t)gridDim.x * (256 / G)) {
+        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+        if constexpr (D == 0) {
+            v = __ldg(reinterpret_cast<const float4*>(dcol + r * C + c));
+        } else {
+            constexpr int Do = D / 2;
+            const int xi = (int)(r % D), yi = (int)(r / D % D), zi = (int)(r / (D * D) % D);
+            const int64_t b = r / (D * D * D);
+#pragma unroll
+            for (int kz = 0; kz < 3; ++kz) {
+                const int tz = zi + 1 - kz;
+                if (tz < 0 || (tz & 1) || tz / 2 >= Do) continue;
+#pragma unroll
+                for (int ky = 0; ky < 3; ++ky) {
+                    const int ty = yi + 1 - ky;
+                    if (ty < 0 || (ty & 1) || ty / 2 >= Do) continue;
+#pragma unroll
+                    for (int kx = 0; kx < 3; ++kx) {
+                        const int tx = xi + 1 - kx;
+                        if (tx < 0 || (tx & 1) || tx / 2 >= Do) continue;
+                        const int64_t row = ((b * Do + tz / 2) * Do + ty / 2) * Do + tx / 2;
+                        const float4 t =
+                            __ldg(reinterpret_cast<const float4*>(dcol + row * KP + ((kz * 3 + ky) * 3 + kx) * C + c));
+                        v = make_float4(v.x + t.x, v.y + t.y, v.z + t.z, v.w + t.w);
+                    }
                 }
             }
         }
-        dx[i] = acc;
+        const uint2 act = __ldg(reinterpret_cast<const uint2*>(a + r * C + c));
+        // ReLU outputs: not negative, so positive means not zero
+        v.x = act.x & 0x7fffu ? v.x : 0.f;
+        v.y = act.x & 0x7fff0000u ? v.y : 0.f;
+        v.z = act.y & 0x7fffu ? v.z : 0.f;
+        v.w = act.y & 0x7fff0000u ? v.w : 0.f;
+        *reinterpret_cast<uint2*>(dzb + r * C + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
+        sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
+    }
+    sums[threadIdx.x] = sum;
+    __syncthreads();
+    if (threadIdx.x < G) {
+        for (int t = threadIdx.x + G; t < 256; t += G) {
+            const float4 o = sums[t];
+            sum = make_float4(sum.x + o.x, sum.y + o.y, sum.z + o.z, sum.w + o.w);
+        }
+        *reinterpret_cast<float4*>(part + (int64_t)blockIdx.x * C + c) = sum;
     }
 }
 
-// z = y + bias (kept, FP32); x = ReLU(z) as BF16 (relu = 0: identity, x as FP32 into y)
-__global__ void k_bias_act(float* __restrict__ y, const float* __restrict__ bias, int64_t rows, int cols,
-                           __nv_bfloat16* __restrict__ x, int relu) {
-    GSTRIDE(i, rows * cols) {
-        const float z = y[i] + bias[i % cols];
-        y[i] = z;
-        if (x) x[i] = __float2bfloat16(relu ? fmaxf(z, 0.0f) : z);
-    }
-}
-
-// dz = dx ⊙ (z > 0), FP32 and BF16 copies
-__global__ void k_relu_back(const float* __restrict__ dx, const float* __restrict__ z, int64_t n, float* __restrict__ dz,
-                            __nv_bfloat16* __restrict__ dzb) {
-    GSTRIDE(i, n) {
-        const float v = z[i] > 0.0f ? dx[i] : 0.0f;
-        dz[i] = v;
-        dzb[i] = __float2bfloat16(v);
-    }
-}
-
-// column sums of rows × cols (FP32): per column, fixed chunks of rows summed in
-// order, then the chunk sums in order
-constexpr int SUM_CHUNK = 4096;
-__global__ void k_colsum_part(const float* __restrict__ m, int64_t rows, int cols, float* __restrict__ part) {
-    const int64_t nchunks = (rows + SUM_CHUNK - 1) / SUM_CHUNK;
-    GSTRIDE(i, nchunks * cols) {
-        const int c = (int)(i % cols);
-        const int64_t ch = i / cols;
-        float acc = 0.0f;
-        const int64_t r1 = min(rows, (ch + 1) * SUM_CHUNK);
-        for (int64_t r = ch * SUM_CHUNK; r < r1; ++r) acc += m[r * cols + c];
-        part[ch * cols + c] = acc;
-    }
-}
-__global__ void k_colsum_fold(const float* __restrict__ part, int64_t nchunks, int cols, float* __restrict__ out) {
-    GSTRIDE(c, cols) {
-        float acc = 0.0f;
-        for (int64_t ch = 0; ch < nchunks; ++ch) acc += part[ch * cols + c];
-        out[c] = acc;
-    }
-}
-
-// loss = mean (out − t)², dout = 2(out − t)/n (one CTA, fixed order)
-__global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t, int n, float* __restrict__ dout,
-                      float* __restrict__ loss) {
+// loss = mean (out − t)², dout = 2(out − t)/n as BF16 rows of ld, its column sums into
+// colsum (one CTA, fixed order)
+__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, const float* __restrict__ t, int rows, int cols,
+                                             __nv_bfloat16* __restrict__ dzb, int ld, float* __restrict__ colsum,
+                                             float* __restrict__ loss) {
     __shared__ float red[256];
+    const int n = rows * cols;
     float acc = 0.0f;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+    for (int i = threadIdx.x; i < n; i += 256) {
         const float d = out[i] - t[i];
-        dout[i] = 2.0f * d / (float)n;
+        dzb[i / cols * ld + i % cols] = __float2bfloat16(2.0f * d / (float)n);
         acc += d * d;
     }
     red[threadIdx.x] = acc;
@@ -269,18 +296,79 @@ __global__ void k_mse(const float* __restrict__ out, const float* __restrict__ t
         __syncthreads();
     }
     if (threadIdx.x == 0) *loss = red[0] / (float)n;
+    __syncthreads();
+    // sixteen threads a column, their sums in order
+    for (int c0 = 0; c0 < cols; c0 += 16) {
+        const int c = c0 + threadIdx.x / 16, q = threadIdx.x % 16;
+        float s = 0.0f;
+        if (c < cols)
+            for (int r = q; r < rows; r += 16) s += 2.0f * (out[r * cols + c] - t[r * cols + c]) / (float)n;
+        red[threadIdx.x] = s;
+        __syncthreads();
+        if (q == 0 && c < cols) {
+            for (int k = 1; k < 16; ++k) s += red[threadIdx.x + k];
+            colsum[c] = s;
+        }
+        __syncthreads();
+    }
 }
 
-__global__ void k_adam(float* __restrict__ w, const float* __restrict__ g, float* __restrict__ m, float* __restrict__ v,
-                       int64_t n, float lr, float b1, float b2, float c1, float c2, float eps) {
-    GSTRIDE(i, n) {
-        const float gi = g[i];
-        const float mi = b1 * m[i] + (1.0f - b1) * gi;
-        const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
-        m[i] = mi;
-        v[i] = vi;
-        w[i] -= lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+// One tensor of parameters at the end of a training step.
+struct Tensor {
+    float *w, *g, *m, *v;
+    __nv_bfloat16* wb;   // its BF16 copy (weights)
+    const float* part;   // partial gradients to sum, n apart (null: g holds the gradient)
+    int n, parts;
+    int block0;          // its first CTA
+};
+struct Tensors {
+    Tensor t[12];
+};
+// Tensors with at least this many partials take eight warps to each element.
+constexpr int WIDE_PARTS = 24;
+inline int tensor_blocks(int n, int parts) { return parts >= WIDE_PARTS ? (n + 31) / 32 : (n + 255) / 256; }
+
+// The gradients' partials summed in a fixed order, then (lr > 0) Adam on the FP32 master
+// values and their BF16 copies: one launch for all layers (it was a sum per split
+// product, twelve Adam launches and twelve conversions and transposes).
+__global__ void __launch_bounds__(256) k_update(const __grid_constant__ Tensors T, float lr, float b1, float b2, float c1,
+                                                float c2, float eps) {
+    __shared__ float red[8][32];
+    int k = 0;
+    while (k < 11 && (int)blockIdx.x >= T.t[k + 1].block0) ++k;
+    const Tensor& t = T.t[k];
+    const int blk = (int)blockIdx.x - t.block0;
+    int i;
+    float g = 0.0f;
+    if (t.parts >= WIDE_PARTS) {
+        const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+        i = blk * 32 + lane;
+        if (i < t.n)
+#pragma unroll 8
+            for (int s = warp; s < t.parts; s += 8) g += __ldg(t.part + (int64_t)s * t.n + i);
+        red[warp][lane] = g;
+        __syncthreads();
+        if (warp > 0) return;
+        for (int q = 1; q < 8; ++q) g += red[q][lane];
+        if (i >= t.n) return;
+    } else {
+        i = blk * 256 + threadIdx.x;
+        if (i >= t.n) return;
+        if (t.part)
+#pragma unroll 4
+            for (int s = 0; s < t.parts; ++s) g += __ldg(t.part + (int64_t)s * t.n + i);
+        else
+            g = t.g[i];
     }
+    if (t.part) t.g[i] = g;
+    if (!(lr > 0.0f)) return;
+    const float mi = b1 * t.m[i] + (1.0f - b1) * g;
+    const float vi = b2 * t.v[i] + (1.0f - b2) * g * g;
+    t.m[i] = mi;
+    t.v[i] = vi;
+    const float w = t.w[i] - lr * (mi / c1) / (sqrtf(vi / c2) + eps);
+    t.w[i] = w;
+    if (t.wb) t.wb[i] = __float2bfloat16(w);
 }
 
 // out[i] = Σ_s part[s·mn + i], slices in order
@@ -331,8 +419,15 @@ __global__ void k_normalise(const float* __restrict__ img, int64_t n, float* __r
 struct Layer {
     int out, in, kp;      // W is out × kp (FP32 master; columns ≥ the true width stay 0)
     float *w, *b, *gw, *gb, *mw, *vw, *mb, *vb;
-    __nv_bfloat16 *wb, *wtb;  // BF16 W (out × kp) and Wᵀ (kp × out)
+    __nv_bfloat16* wb;    // BF16 W
+    __nv_bfloat16* dzb;   // dZ (rows × dz_ld(out)) of the last training step
+    float* wpart;         // the K slices of its weight gradient (null: one slice)
+    float* bpart;         // the CTAs' column sums of dZ
+    int wparts, bparts;   // how many of either
 };
+
+// Row pitch of dZ: TMA wants multiples of 16 bytes.
+inline int dz_ld(int out) { return (out + 7) & ~7; }
 
 }  // namespace
 }  // namespace mi
@@ -340,24 +435,24 @@ struct Layer {
 struct mi_initnet {
     mi_context* ctx = nullptr;
     int max_batch = 0;
-    mi::Layer L[mi::NLAYER];
+    mi::Layer L[mi::NLAYER] = {};
     int step = 0;
     // activations (sized for max_batch)
-    __nv_bfloat16* x0 = nullptr;               // input, BF16 channels-last
     __nv_bfloat16* col[mi::NCONV] = {};        // im2col rows
-    float* z[mi::NLAYER] = {};                 // pre-activations (FP32)
     __nv_bfloat16* xb[mi::NLAYER] = {};        // activations (BF16): conv outputs, fc1
-    float* out = nullptr;                      // fc2 output (alias of z[5])
-    // backward scratch
-    float *dz = nullptr, *dx = nullptr, *dcol = nullptr, *part = nullptr, *loss = nullptr;
-    __nv_bfloat16 *dzb = nullptr, *tA = nullptr, *tB = nullptr;
-    float* slices = nullptr;  // split-K partial products
-    unsigned int* err = nullptr;    // pinned host word a GEMM raises when a wait gives up, and
-    unsigned int* err_dev = nullptr;  // its device address
+    float* out = nullptr;                      // fc2 output
+    float* dcol = nullptr;                     // a layer's input gradient, in im2col columns
+    float* slices = nullptr;                   // split-K partial products of a forward layer
+    // pinned host words and their device addresses: [0] raised by a GEMM whose wait gave up,
+    // [1] the loss
+    unsigned int* host = nullptr;
+    unsigned int* host_dev = nullptr;
 };
 
 namespace mi {
 namespace {
+
+constexpr int BACK_CTAS = 296;  // of k_back_act at most: two on an SM
 
 int64_t rows_of(int l, int B) {  // GEMM rows (output voxels × batch) of layer l
     if (l < NCONV) return (int64_t)B * DIM[l + 1] * DIM[l + 1] * DIM[l + 1];
@@ -368,55 +463,25 @@ void free_net(mi_initnet* n) {
     if (!n) return;
     mi_context* ctx = n->ctx;
     for (auto& l : n->L) {
-        mi::dev_free(ctx, l.w);
-        mi::dev_free(ctx, l.b);
-        mi::dev_free(ctx, l.gw);
-        mi::dev_free(ctx, l.gb);
-        mi::dev_free(ctx, l.mw);
-        mi::dev_free(ctx, l.vw);
-        mi::dev_free(ctx, l.mb);
-        mi::dev_free(ctx, l.vb);
-        mi::dev_free(ctx, l.wb);
-        mi::dev_free(ctx, l.wtb);
+        for (float* p : {l.w, l.b, l.gw, l.gb, l.mw, l.vw, l.mb, l.vb, l.wpart, l.bpart}) dev_free(ctx, p);
+        dev_free(ctx, l.wb);
+        dev_free(ctx, l.dzb);
     }
-    mi::dev_free(ctx, n->x0);
-    for (auto p : n->col) mi::dev_free(ctx, p);
-    for (auto p : n->z) mi::dev_free(ctx, p);
-    for (auto p : n->xb) mi::dev_free(ctx, p);
-    mi::dev_free(ctx, n->dz);
-    mi::dev_free(ctx, n->dx);
-    mi::dev_free(ctx, n->dcol);
-    mi::dev_free(ctx, n->part);
-    mi::dev_free(ctx, n->loss);
-    mi::dev_free(ctx, n->dzb);
-    mi::dev_free(ctx, n->tA);
-    mi::dev_free(ctx, n->tB);
-    mi::dev_free(ctx, n->slices);
-    pinned_free(ctx, n->err);
+    for (auto p : n->col) dev_free(ctx, p);
+    for (auto p : n->xb) dev_free(ctx, p);
+    dev_free(ctx, n->out);
+    dev_free(ctx, n->dcol);
+    dev_free(ctx, n->slices);
+    pinned_free(ctx, n->host);
     delete n;
 }
 
-// BF16 copies of every weight (and of its transpose) after an update
+// BF16 copies of every weight after they were set
 cudaError_t refresh_bf16(mi_initnet* n) {
-    cudaStream_t st = n->ctx->stream;
     for (auto& l : n->L) {
         const int64_t cnt = (int64_t)l.out * l.kp;
-        k_to_bf16<<<grid1(cnt), 256, 0, st>>>(l.w, l.wb, cnt);
-        cudaError_t e = transpose<float>(l.w, l.out, l.kp, l.kp, l.wtb, l.out, st);
-        if (e != cudaSuccess) return e;
+        k_to_bf16<<<grid1(cnt), 256, 0, n->ctx->stream>>>(l.w, l.wb, cnt);
     }
-    return cudaGetLastError();
-}
-
-// C (M × N, contiguous) = A·Bᵀ, split over K where the tiles alone are few
-cudaError_t mm(mi_initnet* n, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B, int ldb,
-               float* C) {
-    cudaStream_t st = n->ctx->stream;
-    const int S = k_splits(M, N, K);
-    if (S == 1) return gemm_dispatch(n->ctx, M, N, K, A, lda, B, ldb, C, N, 1, n->err_dev);
-    cudaError_t e = gemm_dispatch(n->ctx, M, N, K, A, lda, B, ldb, n->slices, N, S, n->err_dev);
-    if (e != cudaSuccess) return e;
-    k_sum_slices<<<grid1((int64_t)M * N), 256, 0, st>>>(n->slices, S, (int64_t)M * N, C);
     return cudaGetLastError();
 }
 
@@ -426,87 +491,108 @@ size_t slice_floats(int M, int N, int K) {
     return S > 1 ? (size_t)S * M * N : 0;
 }
 
-cudaError_t colsum(mi_initnet* n, const float* m, int64_t rows, int cols, float* out) {
-    cudaStream_t st = n->ctx->stream;
-    const int64_t nchunks = (rows + SUM_CHUNK - 1) / SUM_CHUNK;
-    k_colsum_part<<<grid1(nchunks * cols), 256, 0, st>>>(m, rows, cols, n->part);
-    k_colsum_fold<<<grid1(cols), 256, 0, st>>>(n->part, nchunks, cols, out);
+// Layer l's product, bias and ReLU: rows × kp of x into BF16 activations, or for the last
+// layer (no ReLU) FP32 into y.
+cudaError_t layer_forward(mi_initnet* n, int l, int B, const __nv_bfloat16* x, float* y) {
+    const Layer& L = n->L[l];
+    const int M = (int)rows_of(l, B), S = k_splits(M, L.out, L.kp);
+    const Operand a{x, L.kp, false}, w{L.wb, L.kp, false};
+    __nv_bfloat16* act = n->xb[l];
+    if (S == 1)
+        return product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{y, L.out, L.b, act, L.out, 1}, 1, n->host_dev);
+    const cudaError_t e = product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{n->slices, L.out, nullptr, nullptr, 0, 0}, S,
+                                  n->host_dev);
+    if (e != cudaSuccess) return e;
+    const int64_t mn = (int64_t)M * L.out;
+    k_slices_act<<<grid1(mn), 256, 0, n->ctx->stream>>>(n->slices, S, mn, L.b, L.out, act);
     return cudaGetLastError();
 }
 
-// forward pass of B samples (input x: B × 32³ × 2 FP32, channels-last)
-cudaError_t forward(mi_initnet* n, int B, const float* x) {
+// forward pass of B samples (input x: B × 32³ × 2 FP32, channels-last) into out (B × 12)
+cudaError_t forward(mi_initnet* n, int B, const float* x, float* out) {
     cudaStream_t st = n->ctx->stream;
-    const int64_t nin = (int64_t)B * 32 * 32 * 32 * 2;
-    k_to_bf16<<<grid1(nin), 256, 0, st>>>(x, n->x0, nin);
-    const __nv_bfloat16* cur = n->x0;
+    auto grid = [&](int l) { return grid1(rows_of(l, B) * (n->L[l].kp / 8)); };
     cudaError_t e = cudaSuccess;
     for (int l = 0; l < NCONV && e == cudaSuccess; ++l) {
-        const Layer& L = n->L[l];
-        const int64_t rows = rows_of(l, B);
-        k_im2col<<<grid1(rows * L.kp), 256, 0, st>>>(cur, B, DIM[l], CH[l], L.kp, n->col[l]);
-        e = mm(n, (int)rows, L.out, L.kp, n->col[l], L.kp, L.wb, L.kp, n->z[l]);
-        if (e == cudaSuccess) k_bias_act<<<grid1(rows * L.out), 256, 0, st>>>(n->z[l], L.b, rows, L.out, n->xb[l], 1);
-        cur = n->xb[l];
+        __nv_bfloat16* col = n->col[l];
+        switch (l) {
+            case 0: k_im2col<DIM[0], CH[0], 56, float><<<grid(l), 256, 0, st>>>(x, B, col); break;
+            case 1: k_im2col<DIM[1], CH[1], 27 * CH[1], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[0], B, col); break;
+            case 2: k_im2col<DIM[2], CH[2], 27 * CH[2], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[1], B, col); break;
+            default: k_im2col<DIM[3], CH[3], 27 * CH[3], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[2], B, col); break;
+        }
+        e = cudaGetLastError();
+        if (e == cudaSuccess) e = layer_forward(n, l, B, col, nullptr);
     }
     // fc1 on the flattened conv output (B × 1024), fc2 without activation
-    if (e == cudaSuccess) {
-        const Layer& F1 = n->L[NCONV];
-        e = mm(n, B, F1.out, F1.kp, n->xb[NCONV - 1], FC1_IN, F1.wb, F1.kp, n->z[NCONV]);
-        if (e == cudaSuccess)
-            k_bias_act<<<grid1((int64_t)B * F1.out), 256, 0, st>>>(n->z[NCONV], F1.b, B, F1.out, n->xb[NCONV], 1);
-    }
-    if (e == cudaSuccess) {
-        const Layer& F2 = n->L[NCONV + 1];
-        e = mm(n, B, F2.out, F2.kp, n->xb[NCONV], FC1_OUT, F2.wb, F2.kp, n->z[NCONV + 1]);
-        if (e == cudaSuccess)
-            k_bias_act<<<grid1((int64_t)B * F2.out), 256, 0, st>>>(n->z[NCONV + 1], F2.b, B, F2.out, nullptr, 0);
-    }
-    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e == cudaSuccess) e = layer_forward(n, NCONV, B, n->xb[NCONV - 1], nullptr);
+    if (e == cudaSuccess) e = layer_forward(n, NCONV + 1, B, n->xb[NCONV], out);
     return e;
 }
 
-// gradients of the mean squared error against target t (B × 12) into every layer's
-// gw / gb; loss into n->loss
+// The partials of every layer's gradients of the mean squared error against target t
+// (B × 12) on the network's last output; loss into the host word.
 cudaError_t backward(mi_initnet* n, int B, const float* t) {
-    cudaStream_t st = n->ctx->stream;
-    cudaError_t e = cudaSuccess;
-    float* out = n->z[NCONV + 1];
-    // dOut
-    k_mse<<<1, 256, 0, st>>>(out, t, B * FC2_OUT, n->dz, n->loss);
-    // layers from the top; n->dz holds dZ of the current layer (FP32, rows × out)
+    mi_context* ctx = n->ctx;
+    cudaStream_t st = ctx->stream;
+    {
+        Layer& top = n->L[NLAYER - 1];
+        k_mse<<<1, 256, 0, st>>>(n->out, t, B, FC2_OUT, top.dzb, dz_ld(FC2_OUT), top.bpart,
+                                 reinterpret_cast<float*>(n->host_dev + 1));
+        top.bparts = 1;
+    }
+    cudaError_t e = cudaGetLastError();
     for (int l = NLAYER - 1; l >= 0 && e == cudaSuccess; --l) {
         Layer& L = n->L[l];
-        const int64_t rows = rows_of(l, B);
-        // input of the layer (BF16, rows × kp): im2col rows or the previous activation
+        const int rows = (int)rows_of(l, B);
+        // the layer's input (BF16, rows × kp): im2col rows or the previous activation
         const __nv_bfloat16* xin = l < NCONV ? n->col[l] : n->xb[l - 1];
-        const int ldx = l < NCONV ? L.kp : (l == NCONV ? FC1_IN : FC1_OUT);
-        // bias gradient
-        e = colsum(n, n->dz, rows, L.out, L.gb);
-        // dW (out × kp) = dZᵀ · X: both operands transposed to K = rows contiguous
-        if (e == cudaSuccess) e = transpose<float>(n->dz, (int)rows, L.out, L.out, n->tA, (int)rows, st);
-        if (e == cudaSuccess) e = transpose<__nv_bfloat16>(xin, (int)rows, L.kp, ldx, n->tB, (int)rows, st);
-        if (e == cudaSuccess) e = mm(n, L.out, L.kp, (int)rows, n->tA, (int)rows, n->tB, (int)rows, L.gw);
+        const Operand dz{L.dzb, dz_ld(L.out), false}, dzt{L.dzb, dz_ld(L.out), true};
+        // dW (out × kp) = dZᵀ · X, k the rows
+        L.wparts = k_splits(L.out, L.kp, rows);
+        e = product(ctx, L.out, L.kp, rows, dzt, Operand{xin, L.kp, true},
+                    tc::Epilogue{L.wparts > 1 ? L.wpart : L.gw, L.kp, nullptr, nullptr, 0, 0}, L.wparts, n->host_dev);
         if (l == 0 || e != cudaSuccess) break;
-        // dX of the layer input (rows × kp) = dZ · W
-        const int64_t cnt = rows * L.out;
-        k_to_bf16<<<grid1(cnt), 256, 0, st>>>(n->dz, n->dzb, cnt);
-        e = mm(n, (int)rows, L.kp, L.out, n->dzb, L.out, L.wtb, L.out, n->dcol);
+        // the gradient of the layer's input (rows × kp) = dZ · W (out is at most four k tiles, so
+        // never split)
+        e = product(ctx, rows, L.kp, L.out, dz, Operand{L.wb, L.kp, true},
+                    tc::Epilogue{n->dcol, L.kp, nullptr, nullptr, 0, 0}, 1, n->host_dev);
         if (e != cudaSuccess) break;
-        // back to the previous layer's activation layout, then through its ReLU
-        const int pl = l - 1;
-        const int64_t prows = rows_of(pl, B);
-        const int pout = n->L[pl].out;
-        if (l < NCONV) {
-            k_col2im<<<grid1(prows * pout), 256, 0, st>>>(n->dcol, B, DIM[l], CH[l], L.kp, n->dx);
-        } else {
-            // fc layers read the previous activation row by row: dcol already is dX
-            cudaMemcpyAsync(n->dx, n->dcol, (size_t)prows * pout * sizeof(float), cudaMemcpyDeviceToDevice, st);
+        // back to the previous layer's activations, through its ReLU
+        Layer& P = n->L[l - 1];
+        const int64_t prows = rows_of(l - 1, B);
+        const __nv_bfloat16* act = n->xb[l - 1];
+        const int grid = (int)std::min<int64_t>(BACK_CTAS, (prows * (P.out / 4) + 255) / 256);
+        P.bparts = grid;
+        switch (l) {
+            case 1: k_back_act<DIM[1], CH[1], 27 * CH[1]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 2: k_back_act<DIM[2], CH[2], 27 * CH[2]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 3: k_back_act<DIM[3], CH[3], 27 * CH[3]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 4: k_back_act<0, CH[4], 0><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
+            default: k_back_act<0, FC1_OUT, 0><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
         }
-        k_relu_back<<<grid1(prows * pout), 256, 0, st>>>(n->dx, n->z[pl], prows * pout, n->dz, n->dzb);
         e = cudaGetLastError();
     }
     return e;
+}
+
+// The gradients from their partials and, with lr > 0, the Adam step.
+cudaError_t update(mi_initnet* n, float lr) {
+    const float b1 = 0.9f, b2 = 0.999f;
+    const float c1 = 1.0f - std::pow(b1, (float)n->step), c2 = 1.0f - std::pow(b2, (float)n->step);
+    Tensors T;
+    int blocks = 0, k = 0;
+    auto add = [&](const Tensor& t) {
+        T.t[k] = t;
+        T.t[k++].block0 = blocks;
+        blocks += tensor_blocks(t.n, t.parts);
+    };
+    for (const Layer& L : n->L) {
+        add(Tensor{L.w, L.gw, L.mw, L.vw, L.wb, L.wparts > 1 ? L.wpart : nullptr, L.out * L.kp, L.wparts, 0});
+        add(Tensor{L.b, L.gb, L.mb, L.vb, nullptr, L.bpart, L.out, L.bparts, 0});
+    }
+    k_update<<<blocks, 256, 0, n->ctx->stream>>>(T, lr, b1, b2, c1, c2, 1e-8f);
+    return cudaGetLastError();
 }
 
 }  // namespace
@@ -537,7 +623,7 @@ mi_status mi_initnet_create(mi_context* ctx, uint64_t seed, int max_batch, mi_in
         z ^= z >> 31;
         return (double)(z >> 11) * 0x1p-53;
     };
-    size_t max_rows_kp = 0, max_rows_out = 0;
+    size_t max_dcol = 0, max_slices = 0;
     for (int l = 0; l < NLAYER; ++l) {
         Layer& L = n->L[l];
         int fan_in;
@@ -563,41 +649,28 @@ mi_status mi_initnet_create(mi_context* ctx, uint64_t seed, int max_batch, mi_in
         alloc(&L.mb, L.out * 4);
         alloc(&L.vb, L.out * 4);
         alloc(&L.wb, wn * 2);
-        alloc(&L.wtb, wn * 2);
         std::vector<float> hw(wn, 0.0f);
         const double bound = std::sqrt(6.0 / fan_in) * (l == NLAYER - 1 ? 0.1 : 1.0);
         for (int o = 0; o < L.out; ++o)
             for (int k = 0; k < L.in; ++k) hw[(size_t)o * L.kp + k] = (float)((2.0 * next_u() - 1.0) * bound);
         if (e == cudaSuccess) e = cudaMemcpyAsync(L.w, hw.data(), wn * 4, cudaMemcpyHostToDevice, ctx->stream);
+        // for every batch up to max_batch: the slices of a smaller one may be more, but each
+        // holds at least four k tiles
         const int64_t rows = rows_of(l, B);
-        max_rows_kp = std::max(max_rows_kp, (size_t)rows * L.kp);
-        max_rows_out = std::max(max_rows_out, (size_t)rows * L.out);
-        alloc(&n->z[l], (size_t)rows * L.out * 4);
+        const size_t most = std::min<int64_t>(296, std::max<int64_t>(1, (rows + 64 * 4 - 1) / (64 * 4)));
+        if (l > 0) max_dcol = std::max(max_dcol, (size_t)rows * L.kp);
         if (l < NLAYER - 1) alloc(&n->xb[l], (size_t)rows * L.out * 2);
         if (l < NCONV) alloc(&n->col[l], (size_t)rows * L.kp * 2);
-    }
-    size_t max_slices = 0;
-    for (int l = 0; l < NLAYER; ++l) {
-        const Layer& L = n->L[l];
-        const int rows = (int)rows_of(l, B);
-        max_slices = std::max({max_slices, slice_floats(rows, L.out, L.kp), slice_floats(L.out, L.kp, rows),
-                               slice_floats(rows, L.kp, L.out)});
+        alloc(&L.dzb, (size_t)rows * dz_ld(L.out) * 2);
+        alloc(&L.wpart, most * wn * 4);
+        alloc(&L.bpart, (size_t)BACK_CTAS * L.out * 4);
+        for (int q = 1; q <= B; ++q) max_slices = std::max(max_slices, slice_floats((int)rows_of(l, q), L.out, L.kp));
     }
     alloc(&n->slices, std::max<size_t>(max_slices, 1) * 4);
-    size_t max_act = 0;  // largest activation / input of any layer, FP32 elements
-    for (int l = 0; l < NLAYER; ++l) max_act = std::max(max_act, (size_t)rows_of(l, B) * n->L[l].out);
-    max_act = std::max(max_act, (size_t)B * 32 * 32 * 32 * 2);
-    alloc(&n->x0, (size_t)B * 32 * 32 * 32 * 2 * 2);
-    alloc(&n->dz, max_act * 4);
-    alloc(&n->dx, max_act * 4);
-    alloc(&n->dcol, max_rows_kp * 4);
-    alloc(&n->part, (max_rows_out / SUM_CHUNK + 1024) * 4 + 65536 * 4);
-    alloc(&n->loss, 4);
-    alloc(&n->dzb, max_act * 2);
-    alloc(&n->tA, std::max(max_rows_out, max_act) * 2);
-    alloc(&n->tB, max_rows_kp * 2);
-    if (e == cudaSuccess) e = pinned_alloc(ctx, (void**)&n->err, (void**)&n->err_dev);
-    if (e == cudaSuccess) *n->err = 0u;
+    alloc(&n->dcol, max_dcol * 4);
+    alloc(&n->out, (size_t)B * FC2_OUT * 4);
+    if (e == cudaSuccess) e = pinned_alloc(ctx, (void**)&n->host, (void**)&n->host_dev);
+    if (e == cudaSuccess) n->host[0] = n->host[1] = 0u;
     if (e == cudaSuccess) e = mi::refresh_bf16(n);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {
@@ -646,8 +719,8 @@ mi_status mi_initnet_set(mi_initnet* n, int which, const float* w, const float* 
 static mi_status check_err(mi_initnet* n, cudaError_t e, const char* where) {
     if (e == cudaSuccess) e = cudaStreamSynchronize(n->ctx->stream);
     if (e != cudaSuccess) return mi::cuda_status(n->ctx, e, where);
-    if (*n->err) {
-        *n->err = 0u;
+    if (n->host[0]) {
+        n->host[0] = 0u;
         return mi::set_error(n->ctx, MI_ERR_TIMEOUT, "tensor-core GEMM: an mbarrier wait gave up");
     }
     return MI_OK;
@@ -657,10 +730,7 @@ static mi_status check_err(mi_initnet* n, cudaError_t e, const char* where) {
 mi_status mi_initnet_forward(mi_initnet* n, int B, const float* x, float* out) {
     if (!n || B < 1 || B > n->max_batch || !x || !out) return MI_ERR_INVALID_ARGUMENT;
     MI_CHECK_CUDA(n->ctx, cudaSetDevice(n->ctx->device));
-    cudaError_t e = mi::forward(n, B, x);
-    if (e == cudaSuccess)
-        e = cudaMemcpyAsync(out, n->z[mi::NLAYER - 1], (size_t)B * mi::FC2_OUT * 4, cudaMemcpyDeviceToDevice, n->ctx->stream);
-    return check_err(n, e, "mi_initnet_forward");
+    return check_err(n, mi::forward(n, B, x, out), "mi_initnet_forward");
 }
 
 // One training step on B samples: forward, mean squared error against t (device,
@@ -669,23 +739,14 @@ mi_status mi_initnet_train_step(mi_initnet* n, int B, const float* x, const floa
     using namespace mi;
     if (!n || B < 1 || B > n->max_batch || !x || !t) return MI_ERR_INVALID_ARGUMENT;
     MI_CHECK_CUDA(n->ctx, cudaSetDevice(n->ctx->device));
-    cudaStream_t st = n->ctx->stream;
-    cudaError_t e = forward(n, B, x);
+    cudaError_t e = forward(n, B, x, n->out);
     if (e == cudaSuccess) e = backward(n, B, t);
-    if (e == cudaSuccess && lr > 0.0f) {
-        n->step += 1;
-        const float b1 = 0.9f, b2 = 0.999f;
-        const float c1 = 1.0f - std::pow(b1, (float)n->step), c2 = 1.0f - std::pow(b2, (float)n->step);
-        for (auto& L : n->L) {
-            const int64_t wn = (int64_t)L.out * L.kp;
-            k_adam<<<grid1(wn), 256, 0, st>>>(L.w, L.gw, L.mw, L.vw, wn, lr, b1, b2, c1, c2, 1e-8f);
-            k_adam<<<grid1(L.out), 256, 0, st>>>(L.b, L.gb, L.mb, L.vb, L.out, lr, b1, b2, c1, c2, 1e-8f);
-        }
-        e = cudaGetLastError();
-        if (e == cudaSuccess) e = refresh_bf16(n);
+    if (e == cudaSuccess) {
+        if (lr > 0.0f) n->step += 1;
+        e = update(n, lr);
     }
     mi_status s = check_err(n, e, "mi_initnet_train_step");
-    if (s == MI_OK && loss) MI_CHECK_CUDA(n->ctx, cudaMemcpy(loss, n->loss, 4, cudaMemcpyDeviceToHost));
+    if (s == MI_OK && loss) std::memcpy(loss, &n->host[1], 4);
     return s;
 }
 
