@@ -166,11 +166,11 @@ struct Workspace {
 namespace mi {
 // Buffers of the mean-squares and correlation reductions (moments.cu).
 struct MomentsWs {
-    int grid = 0;
-    double* partials = nullptr;      // [grid][slots]
-    double* result = nullptr;        // [2][28]: the folded moments, then correlation's pass-1 sums
-    unsigned int* counter = nullptr; // [2] arrival counters
-    double* host = nullptr;          // pinned, mapped mirror of the folded moments
+    int grid = 0, grid_grad = 0;     // CTAs of the value's pass, and with the derivative
+    double* partials = nullptr;      // [slots][grid]
+    double* shift = nullptr;         // correlation's shift, then that of a repeated pass
+    unsigned int* counter = nullptr; // arrivals
+    double* host = nullptr;          // pinned, mapped mirror of the folded moments, then the tag
     double* host_dev = nullptr;      // the mirror's device address
     float* fval = nullptr;           // each sample's fixed value, in sample order (null: the whole grid)
 };

@@ -1219,7 +1219,7 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
     for (int d = 0; d < 3; ++d) P.msz[d] = (int)moving->geo.size[d];
     P.ms1 = (uint32_t)P.mstride1;
     P.ms2 = (uint32_t)P.mstride2;
-    {
+    if (mattes) {
         // the moving volume behind a point-sampling, clamp-to-edge, unnormalised-coordinate
         // texture (the fast path's corner fetch): a 2-D layered array, one layer per z
         // slice, whose cell corners come in two gathers, when the volume fits the
@@ -1233,7 +1233,7 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         TRY_CUDA(cudaDeviceGetAttribute(&lh, cudaDevAttrMaxTexture2DLayeredHeight, ctx->device));
         TRY_CUDA(cudaDeviceGetAttribute(&ll, cudaDevAttrMaxTexture2DLayeredLayers, ctx->device));
         const bool layered = moving->geo.size[0] <= lw && moving->geo.size[1] <= lh && moving->geo.size[2] <= ll &&
-                             MOVING_LAYERED && texture == MI_TEXTURE_AUTO && mattes;
+                             MOVING_LAYERED && texture == MI_TEXTURE_AUTO;
         P.mlayered = layered ? 1 : 0;
         P.mbf16 = b16 ? 1 : 0;
         TRY_CUDA(array_alloc(ctx, &m->marray, ext, esize, layered));
@@ -1243,13 +1243,7 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         cp.dstArray = m->marray;
         cp.extent = ext;
         cp.kind = cudaMemcpyDeviceToDevice;
-        const cudaError_t ce = cudaMemcpy3DAsync(&cp, st);
-        if (mbits) {
-            cudaStreamSynchronize(st);
-            dev_free(ctx, mbits);
-            mbits = nullptr;
-        }
-        TRY_CUDA(ce);
+        TRY_CUDA(cudaMemcpy3DAsync(&cp, st));
         cudaResourceDesc res = {};
         res.resType = cudaResourceTypeArray;
         res.res.array.array = m->marray;
@@ -1261,6 +1255,8 @@ mi_status mi_metric_create_ex(mi_context* ctx, const mi_image* fixed, const mi_i
         TRY_CUDA(cudaCreateTextureObject(&m->mtex, &res, &td, nullptr));
         P.mtex = m->mtex;
     }
+    dev_free(ctx, mbits);
+    mbits = nullptr;
     P.bins = bins;
     P.fixed_bin_size = info.fixed_bin_size;
     P.moving_bin_size = info.moving_bin_size;
