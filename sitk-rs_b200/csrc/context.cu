@@ -68,11 +68,12 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 //   device memory  a stream-ordered pool of the context, which keeps at most POOL_KEEP
 //                  bytes it has no use for (the rest goes back to the device at the next
 //                  synchronisation), and gives all of it up when an allocation fails
-//   pinned blocks  slabs of 64, kept until the context goes
+//   pinned blocks  slabs of 64 small ones, kept until the context goes; of the larger ones up
+//                  to LARGE_SPARES of each size of at most LARGE_KEEP bytes
 //   arrays         at most SPARE_ARRAYS of SPARE_ARRAY_BYTES together, taken by exact shape
 constexpr unsigned long long POOL_KEEP = 4ull << 30;
 constexpr size_t SPARE_ARRAYS = 64, SPARE_ARRAY_BYTES = (size_t)1 << 30;
-constexpr size_t SLAB_BLOCKS = 64;
+constexpr size_t SLAB_BLOCKS = 64, LARGE_SPARES = 4, LARGE_KEEP = (size_t)16 << 20;
 
 namespace {
 
@@ -122,29 +123,47 @@ void dev_free(mi_context* ctx, void* p) {
     if (p) cudaFreeAsync(p, ctx->stream);
 }
 
-cudaError_t pinned_alloc(mi_context* ctx, void** host, void** dev) {
+// Larger blocks come in powers of two.
+static size_t pinned_class(size_t bytes) {
+    size_t c = 4096;
+    while (c < bytes) c <<= 1;
+    return c;
+}
+
+cudaError_t pinned_alloc(mi_context* ctx, void** host, void** dev, size_t bytes) {
     std::lock_guard<std::mutex> g(ctx->spare_mutex);
-    if (ctx->pinned_spare.empty()) {
+    std::vector<unsigned char*>& spare = bytes <= PINNED_BLOCK ? ctx->pinned_spare : ctx->pinned_large[pinned_class(bytes)];
+    if (spare.empty()) {
+        const size_t block = bytes <= PINNED_BLOCK ? PINNED_BLOCK : pinned_class(bytes);
+        const size_t blocks = bytes <= PINNED_BLOCK ? SLAB_BLOCKS : 1;
         void* slab = nullptr;
-        const cudaError_t e = cudaHostAlloc(&slab, SLAB_BLOCKS * PINNED_BLOCK, cudaHostAllocMapped);
+        const cudaError_t e = cudaHostAlloc(&slab, blocks * block, cudaHostAllocMapped);
         if (e != cudaSuccess) return e;
-        ctx->pinned_slabs.push_back(static_cast<unsigned char*>(slab));
-        for (size_t i = SLAB_BLOCKS; i-- > 0;) ctx->pinned_spare.push_back(ctx->pinned_slabs.back() + i * PINNED_BLOCK);
+        if (bytes <= PINNED_BLOCK) ctx->pinned_slabs.push_back(static_cast<unsigned char*>(slab));
+        for (size_t i = blocks; i-- > 0;) spare.push_back(static_cast<unsigned char*>(slab) + i * block);
     }
-    unsigned char* h = ctx->pinned_spare.back();
+    unsigned char* h = spare.back();
     if (dev) {
         const cudaError_t e = cudaHostGetDevicePointer(dev, h, 0);
         if (e != cudaSuccess) return e;
     }
-    ctx->pinned_spare.pop_back();
+    spare.pop_back();
     *host = h;
     return cudaSuccess;
 }
 
-void pinned_free(mi_context* ctx, void* host) {
+void pinned_free(mi_context* ctx, void* host, size_t bytes) {
     if (!host) return;
     std::lock_guard<std::mutex> g(ctx->spare_mutex);
-    ctx->pinned_spare.push_back(static_cast<unsigned char*>(host));
+    if (bytes <= PINNED_BLOCK) {
+        ctx->pinned_spare.push_back(static_cast<unsigned char*>(host));
+        return;
+    }
+    std::vector<unsigned char*>& spare = ctx->pinned_large[pinned_class(bytes)];
+    if (pinned_class(bytes) <= LARGE_KEEP && spare.size() < LARGE_SPARES)
+        spare.push_back(static_cast<unsigned char*>(host));
+    else
+        cudaFreeHost(host);
 }
 
 cudaError_t array_alloc(mi_context* ctx, cudaArray_t* out, const cudaExtent& ext, size_t element, bool layered) {
@@ -277,6 +296,8 @@ mi_status mi_context_destroy(mi_context* ctx) {
     }
     for (const mi::SpareArray& a : ctx->spare_arrays) cudaFreeArray(a.array);
     for (unsigned char* slab : ctx->pinned_slabs) cudaFreeHost(slab);
+    for (auto& c : ctx->pinned_large)
+        for (unsigned char* p : c.second) cudaFreeHost(p);
     cudaMemPoolDestroy(ctx->pool);
     delete ctx;
     return MI_OK;

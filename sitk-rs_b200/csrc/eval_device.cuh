@@ -680,8 +680,8 @@ __device__ TailCtx tail_finish(int B, double moving_bin_size, const EvalArgs& a,
     const int B2 = B * B;
     if (!a.gcols) {
         const int G = tail_groups(B);
-        if ((int)threadIdx.x < G * B) {
-            const int m = threadIdx.x % B, g = threadIdx.x / B;
+        for (int e = threadIdx.x; e < G * B; e += blockDim.x) {
+            const int m = e % B, g = e / B;
             unsigned long long v = 0ull;
             for (int f = g; f < B; f += G) v += ts.hist[f * B + m];
             ts.part[g * B + m] = v;

@@ -5,6 +5,7 @@
 #include <cudaTypedefs.h>
 #include <cstdint>
 #include <list>
+#include <map>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -31,6 +32,7 @@ struct mi_context {
     cudaMemPool_t pool = nullptr;
     std::mutex spare_mutex;
     std::vector<unsigned char*> pinned_slabs, pinned_spare;
+    std::map<size_t, std::vector<unsigned char*>> pinned_large;  // spare ones by size
     std::list<mi::SpareArray> spare_arrays;  // oldest first
     size_t spare_array_bytes = 0;
 };
@@ -218,6 +220,11 @@ struct mi_metric {
     bool bs_have_key = false;
     uint32_t* bs_order = nullptr;  // sample indices sorted by cell (valid-region samples first)
     uint32_t* bs_off = nullptr;    // [cells + 1] offsets into bs_order
+    uint32_t* bs_flat = nullptr;   // the samples' voxels and fixed bins in that order
+    uint8_t* bs_fbin = nullptr;
+    double* bs_host = nullptr;     // pinned copy of the coefficients in, the derivative out
+    double* bs_host_dev = nullptr; // and its device address
+    void* bs_points = nullptr;     // control points in moving index space (double4 each)
     int64_t bs_ncells = 0;
     float* bs_pr = nullptr;        // the pRatio·nFactor table of the last evaluation
 };
@@ -241,11 +248,11 @@ cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
     return e;
 }
 void dev_free(mi_context* ctx, void* p);
-// A block of PINNED_BLOCK bytes of pinned host memory mapped into the device; `dev` (its
-// device address) may be null.
+// Pinned host memory mapped into the device (`dev`, its device address, may be null), freed
+// with the size it was asked for.
 constexpr size_t PINNED_BLOCK = 512;
-cudaError_t pinned_alloc(mi_context* ctx, void** host, void** dev);
-void pinned_free(mi_context* ctx, void* host);
+cudaError_t pinned_alloc(mi_context* ctx, void** host, void** dev, size_t bytes = PINNED_BLOCK);
+void pinned_free(mi_context* ctx, void* host, size_t bytes = PINNED_BLOCK);
 // A 3-D or layered array of 4-byte float or 2-byte unsigned elements.
 cudaError_t array_alloc(mi_context* ctx, cudaArray_t* out, const cudaExtent& ext, size_t element, bool layered);
 void array_free(mi_context* ctx, cudaArray_t array, const cudaExtent& ext, size_t element, bool layered);

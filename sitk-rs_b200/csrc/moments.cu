@@ -46,6 +46,7 @@
 
 #include "internal.h"
 #include "sampler.cuh"
+#include "sampler64.cuh"
 #include "eval_device.cuh"
 
 namespace mi {
@@ -74,17 +75,9 @@ struct MomArgs {
     double* result_host;       // mapped host mirror the last CTA writes
     unsigned long long seq;    // the evaluation's number
     const double* shift;       // f₀, m₀ (correlation)
-    // thresholds on the upper words of a fraction outside which the sample may lie within
-    // cerr of a cell face
-    int face_lo, face_hi;
-    int half_lo, half_hi;      // and of 1/2 ∓ 2·cerr
+    FracWords words;
     double mid[3];             // the fixed grid's centre in index units
-    int easy;                  // cerr is small enough for the interior test
 };
-
-// floor and int conversions by addition: 1.5·2^52 + x has x's integer part in its low word
-constexpr double BIG = 6755399441055744.0;
-__device__ __forceinline__ double u32_to_f64(uint32_t v) { return __hiloint2double(0x43300000, (int)v) - 4503599627370496.0; }
 
 // A sample's place in the moving volume: the cell, the fractions, and the grid index.
 struct Place {
@@ -136,98 +129,21 @@ __device__ __forceinline__ bool locate(const SamplerParams& P, const MomArgs& a,
 #pragma unroll
     for (int r = 0; r < 3; ++r)
         c[r] = fma(P.cA[r * 3 + 2], p.idx[2], fma(P.cA[r * 3 + 1], p.idx[1], fma(P.cA[r * 3], p.idx[0], P.cb[r])));
-    // The decisions by integers: the cell, and the upper word of the fraction against those of
-    // cerr, 1 − cerr and 1/2 ∓ 2·cerr (a word equal to the threshold's counts as near it).
-    bool inner = true, sure = a.easy != 0;
-    int h[3];
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const double t = __dadd_rd(c[d], BIG);
-        p.cell[d] = __double2loint(t);
-        p.fr[d] = c[d] - (t - BIG);
-        h[d] = __double2hiint(p.fr[d]);
-        inner = inner && __double2hiint(t) == 0x43380000 && (unsigned)p.cell[d] < (unsigned)(P.msz[d] - 1);
-        if (GRAD) sure = sure && h[d] > a.face_lo && h[d] < a.face_hi;
-        if (P.has_mmask) sure = sure && (h[d] < a.half_lo || h[d] > a.half_hi);
-    }
-    if (!inner) {
-        // off the interior: c ∈ [−1/2, 0) and [size − 1, size − 1/2) are still inside
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int hi = __double2hiint(__dadd_rd(c[d], BIG)), n = p.cell[d];
-            if (hi != 0x43380000 && hi != 0x4337ffff) {
-                sure = false;  // past 32 bits, or not a number
-            } else if (n == -1 || n == P.msz[d] - 1) {
-                if (a.easy && (n == -1 ? h[d] < a.half_lo : h[d] > a.half_hi)) return false;
-                sure = sure && (h[d] < a.half_lo || h[d] > a.half_hi);
-            } else if ((unsigned)n >= (unsigned)P.msz[d]) {
-                if (a.easy) return false;
-            }
-        }
-    }
-    if (!sure) {
+    const int st = place64<GRAD>(P, a.words, c, p.cell, p.fr);
+    if (st == SAMPLE_OFF) return false;
+    if (st == SAMPLE_UNSURE) {
         // (copies: what a call takes by address lives in memory, here only on this path)
         double e[3] = {c[0], c[1], c[2]};
         int cell[3];
         if (!locate_edge<GRAD>(P, i, j, k, e, cell)) return false;
 #pragma unroll
         for (int d = 0; d < 3; ++d) {
-            c[d] = e[d];
             p.cell[d] = cell[d];
-            p.fr[d] = c[d] - floor(c[d]);
-            h[d] = __double2hiint(p.fr[d]);
+            p.fr[d] = e[d] - floor(e[d]);
         }
+        return !P.has_mmask || mask_exact(P, a.mmask, e);
     }
-    if (P.has_mmask) {
-        // the nearest voxel, halves up; an exact c (locate_edge) decides at 1/2 itself
-        uint32_t at = 0;
-#pragma unroll
-        for (int d = 0; d < 3; ++d) {
-            const int r = p.cell[d] + (h[d] >= 0x3fe00000 ? 1 : 0);
-            if ((unsigned)r >= (unsigned)P.msz[d]) return false;
-            at += (uint32_t)r * (d == 0 ? 1u : (d == 1 ? P.ms1 : P.ms2));
-        }
-        if (!__ldg(a.mmask + at)) return false;
-    }
-    return true;
-}
-
-// The cell's corners (order of fetch_corners, each clamped to the volume) by plain loads from
-// the x-fastest volume: 3–7 % faster here than eight point fetches of a 3-D texture, on the
-// whole grid and on sampled lists, at any rotation, and no array to fill at set-up.
-__device__ __forceinline__ void load_corners(const SamplerParams& P, const float* __restrict__ moving, const int* cell,
-                                             float* v) {
-    uint32_t lo[3], up[3];  // the lower corner's offset, and from it to the upper one's
-#pragma unroll
-    for (int d = 0; d < 3; ++d) {
-        const uint32_t step = d == 0 ? 1u : (d == 1 ? P.ms1 : P.ms2);
-        lo[d] = (uint32_t)max(cell[d], 0) * step;
-        up[d] = (unsigned)cell[d] < (unsigned)(P.msz[d] - 1) ? step : 0u;
-    }
-    const uint32_t o = lo[0] + lo[1] + lo[2];
-#pragma unroll
-    for (int t = 0; t < 8; ++t)
-        v[t] = __ldg(moving + (o + (t & 1 ? up[0] : 0u) + (t & 2 ? up[1] : 0u) + (t & 4 ? up[2] : 0u)));
-}
-
-// transform/interpolator.rs:103-152: the linear interpolant at the fractions of the cell
-// with corners v, and its gradient in index space
-template <bool GRAD>
-__device__ __forceinline__ double interpolate(const float* v, const double* fr, double* g) {
-    const double v0 = v[0], v2 = v[2], v4 = v[4], v6 = v[6];
-    const double d00 = (double)v[1] - v0, d10 = (double)v[3] - v2, d01 = (double)v[5] - v4, d11 = (double)v[7] - v6;
-    const double x00 = fma(fr[0], d00, v0), x10 = fma(fr[0], d10, v2);
-    const double x01 = fma(fr[0], d01, v4), x11 = fma(fr[0], d11, v6);
-    const double e0 = x10 - x00, e1 = x11 - x01;
-    const double y0 = fma(fr[1], e0, x00), y1 = fma(fr[1], e1, x01);
-    const double z = y1 - y0;
-    if (GRAD) {
-        const double a0 = fma(fr[1], d10 - d00, d00), a1 = fma(fr[1], d11 - d01, d01);
-        g[0] = fma(fr[2], a1 - a0, a0);
-        g[1] = fma(fr[2], e1 - e0, e0);
-        g[2] = z;
-    }
-    return fma(fr[2], z, y0);
+    return !P.has_mmask || mask64(P, a.mmask, p.cell, p.fr);
 }
 
 // acc[0..2] += w·g, acc[3 + 3j + m] += w·g_j·x_m
@@ -477,20 +393,8 @@ static mi_status moments_pass(mi_metric* m, const SamplerParams& P, const double
     a.result_host = w.host_dev;
     a.seq = ++ws.seq;
     a.shift = shift;
-    // upper words of cerr and 1 − cerr; equality counts as near a face
-    long long lo, hi;
-    const double ce = P.cerr, top = 1.0 - P.cerr;
-    std::memcpy(&lo, &ce, 8);
-    std::memcpy(&hi, &top, 8);
-    a.face_lo = (int)(lo >> 32);
-    a.face_hi = (int)(hi >> 32);
-    const double below = 0.5 - 2.0 * ce, above = 0.5 + 2.0 * ce;
-    std::memcpy(&lo, &below, 8);
-    std::memcpy(&hi, &above, 8);
-    a.half_lo = (int)(lo >> 32);
-    a.half_hi = (int)(hi >> 32);
+    a.words = frac_words(P.cerr);
     for (int d = 0; d < 3; ++d) a.mid[d] = (double)P.xmid[d];
-    a.easy = P.cerr < 0.01 ? 1 : 0;
     const bool timing = ws.timing != 0;
     if (timing) MI_CHECK_CUDA(ctx, cudaEventRecord(ws.ev[0], st));
     const int grid = grad ? w.grid_grad : w.grid;
