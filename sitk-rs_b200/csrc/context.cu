@@ -65,15 +65,19 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // pair takes 0.65–0.75 ms at any size up to 128 MB, a 128-byte cudaHostAlloc / cudaFreeHost
 // pair 2.2 ms and a layered array 0.45 ms; the pool hands a block out and back in 4 µs.
 // A metric holds about twenty blocks, so its set-up was mostly these calls.
-//   device memory  a stream-ordered pool of the context, which keeps at most POOL_KEEP
-//                  bytes it has no use for (the rest goes back to the device at the next
-//                  synchronisation), and gives all of it up when an allocation fails
+//   device memory  a stream-ordered pool of the context for blocks below LARGE, and spare
+//                  blocks of at most LARGE_BYTES together above it, taken by the nearest
+//                  size (the pool maps freed pages anew where a block of another size takes
+//                  their place: 0.2–5 ms for 64–128 MB)
 //   pinned blocks  slabs of 64 small ones, kept until the context goes; of the larger ones up
-//                  to LARGE_SPARES of each size of at most LARGE_KEEP bytes
+//                  to PINNED_SPARES of each size of at most PINNED_KEEP bytes
 //   arrays         at most SPARE_ARRAYS of SPARE_ARRAY_BYTES together, taken by exact shape
-constexpr unsigned long long POOL_KEEP = 4ull << 30;
+// All of it goes back to the device when an allocation does not fit beside it, and with the
+// context. A block is reused in the order of the context's one stream, so nothing waits.
+constexpr unsigned long long POOL_KEEP = 256ull << 20;  // what the pool keeps of freed pages
+constexpr size_t LARGE = (size_t)1 << 20, LARGE_BYTES = (size_t)4 << 30;
 constexpr size_t SPARE_ARRAYS = 64, SPARE_ARRAY_BYTES = (size_t)1 << 30;
-constexpr size_t SLAB_BLOCKS = 64, LARGE_SPARES = 4, LARGE_KEEP = (size_t)16 << 20;
+constexpr size_t SLAB_BLOCKS = 64, PINNED_SPARES = 4, PINNED_KEEP = (size_t)16 << 20;
 
 namespace {
 
@@ -97,19 +101,29 @@ void drop_arrays(mi_context* ctx, size_t count, size_t bytes) {
     }
 }
 
+// The spare large blocks beyond `bytes` together go to the pool, oldest first (spare_mutex
+// held).
+void drop_blocks(mi_context* ctx, size_t bytes) {
+    while (!ctx->spare_blocks.empty() && ctx->spare_block_bytes > bytes) {
+        const auto oldest = ctx->spare_blocks.begin();
+        ctx->spare_block_bytes -= oldest->bytes;
+        ctx->large_blocks.erase(oldest->p);
+        cudaFreeAsync(oldest->p, ctx->stream);
+        ctx->spare_blocks.erase(oldest);
+    }
+}
+
 // Everything kept goes back to the device, for an allocation that did not fit beside it.
 void give_back(mi_context* ctx) {
     cudaGetLastError();
+    std::lock_guard<std::mutex> g(ctx->spare_mutex);
+    drop_blocks(ctx, 0);
+    drop_arrays(ctx, 0, 0);
     cudaStreamSynchronize(ctx->stream);
     cudaMemPoolTrimTo(ctx->pool, 0);
-    std::lock_guard<std::mutex> g(ctx->spare_mutex);
-    drop_arrays(ctx, 0, 0);
 }
 
-}  // namespace
-
-cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
-    if (bytes == 0) bytes = 1;
+cudaError_t pool_alloc(mi_context* ctx, void** p, size_t bytes) {
     cudaError_t e = cudaMallocFromPoolAsync(p, bytes, ctx->pool, ctx->stream);
     if (e == cudaErrorMemoryAllocation) {
         give_back(ctx);
@@ -119,8 +133,44 @@ cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
     return e;
 }
 
+}  // namespace
+
+cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
+    if (bytes < LARGE) return pool_alloc(ctx, p, bytes ? bytes : 1);
+    bytes = (bytes + LARGE - 1) & ~(LARGE - 1);
+    {
+        std::lock_guard<std::mutex> g(ctx->spare_mutex);
+        auto best = ctx->spare_blocks.end();
+        for (auto it = ctx->spare_blocks.begin(); it != ctx->spare_blocks.end(); ++it)
+            if (it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
+                (best == ctx->spare_blocks.end() || it->bytes < best->bytes))
+                best = it;
+        if (best != ctx->spare_blocks.end()) {
+            *p = best->p;
+            ctx->spare_block_bytes -= best->bytes;
+            ctx->spare_blocks.erase(best);
+            return cudaSuccess;
+        }
+    }
+    const cudaError_t e = pool_alloc(ctx, p, bytes);
+    if (e == cudaSuccess) {
+        std::lock_guard<std::mutex> g(ctx->spare_mutex);
+        ctx->large_blocks[*p] = bytes;
+    }
+    return e;
+}
+
 void dev_free(mi_context* ctx, void* p) {
-    if (p) cudaFreeAsync(p, ctx->stream);
+    if (!p) return;
+    std::lock_guard<std::mutex> g(ctx->spare_mutex);
+    const auto large = ctx->large_blocks.find(p);
+    if (large == ctx->large_blocks.end()) {
+        cudaFreeAsync(p, ctx->stream);
+        return;
+    }
+    ctx->spare_blocks.push_back(SpareBlock{p, large->second});
+    ctx->spare_block_bytes += large->second;
+    drop_blocks(ctx, LARGE_BYTES);
 }
 
 // Larger blocks come in powers of two.
@@ -160,7 +210,7 @@ void pinned_free(mi_context* ctx, void* host, size_t bytes) {
         return;
     }
     std::vector<unsigned char*>& spare = ctx->pinned_large[pinned_class(bytes)];
-    if (pinned_class(bytes) <= LARGE_KEEP && spare.size() < LARGE_SPARES)
+    if (pinned_class(bytes) <= PINNED_KEEP && spare.size() < PINNED_SPARES)
         spare.push_back(static_cast<unsigned char*>(host));
     else
         cudaFreeHost(host);
@@ -295,6 +345,7 @@ mi_status mi_context_destroy(mi_context* ctx) {
         cudaStreamDestroy(ctx->stream);
     }
     for (const mi::SpareArray& a : ctx->spare_arrays) cudaFreeArray(a.array);
+    for (const mi::SpareBlock& b : ctx->spare_blocks) cudaFree(b.p);
     for (unsigned char* slab : ctx->pinned_slabs) cudaFreeHost(slab);
     for (auto& c : ctx->pinned_large)
         for (unsigned char* p : c.second) cudaFreeHost(p);

@@ -8,6 +8,7 @@
 #include <map>
 #include <mutex>
 #include <string>
+#include <unordered_map>
 #include <vector>
 
 #include "mi_b200.h"
@@ -19,6 +20,11 @@ struct SpareArray {
     size_t extent[3], element;
     bool layered;
     size_t bytes() const { return extent[0] * extent[1] * extent[2] * element; }
+};
+// A large block of device memory waiting for its next use.
+struct SpareBlock {
+    void* p;
+    size_t bytes;
 };
 }  // namespace mi
 
@@ -33,6 +39,9 @@ struct mi_context {
     std::mutex spare_mutex;
     std::vector<unsigned char*> pinned_slabs, pinned_spare;
     std::map<size_t, std::vector<unsigned char*>> pinned_large;  // spare ones by size
+    std::list<mi::SpareBlock> spare_blocks;  // oldest first
+    size_t spare_block_bytes = 0;
+    std::unordered_map<void*, size_t> large_blocks;  // every large block, in use or spare
     std::list<mi::SpareArray> spare_arrays;  // oldest first
     size_t spare_array_bytes = 0;
 };
