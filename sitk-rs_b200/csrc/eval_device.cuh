@@ -72,14 +72,6 @@ constexpr int HIST_CLUSTER = MI_HIST_CLUSTER;
 #ifndef MI_HIST_FINE_T
 #define MI_HIST_FINE_T 10
 #endif
-// Order of a materialised sample list: 0 sorts by voxel index (x-fastest rows);
-// b > 0 sorts into bricks of 2^b voxels per axis, so that a warp's samples, and the
-// moving cells they map to, are spatially close. 8³ bricks measured k_hist 40.9 µs
-// against 43.0 for row order on the 256³ workload (4³ and 16³ within 0.2 µs of 8³).
-#ifndef MI_SAMPLE_BRICK_LOG2
-#define MI_SAMPLE_BRICK_LOG2 3
-#endif
-constexpr int SAMPLE_BRICK_LOG2 = MI_SAMPLE_BRICK_LOG2;
 // The moving volume's texture: 1 stores it 2-D layered (one layer per z slice, a cell's
 // corners in two gathers) wherever the volume fits the layered limits, 0 always 3-D
 // (eight point fetches).

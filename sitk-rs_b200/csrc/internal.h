@@ -191,7 +191,7 @@ struct mi_metric {
     mi_context* ctx = nullptr;
     int metric_kind = 0;          // MI_METRIC_MATTES, MI_METRIC_MEAN_SQUARES, MI_METRIC_CORRELATION
     mi_geometry fgeo{}, mgeo{};
-    float* fixed = nullptr;       // device copy of the fixed volume
+    float* fixed = nullptr;       // device copy of the fixed volume (whole-grid mean squares and correlation)
     float* moving = nullptr;      // device copy of the moving volume
     uint8_t* mmask = nullptr;     // device moving mask or null
     cudaArray_t marray = nullptr; // the moving volume in a block-linear 3-D array
@@ -282,7 +282,7 @@ mi_status transform_jacobian(int kind, const double* params, int nparams, const 
                              const double* x, double* jac);
 
 // Mean squares and correlation (moments.cu).
-mi_status moments_setup(mi_metric* m);
+mi_status moments_setup(mi_metric* m, const float* fixed);  // fixed: the fixed volume
 void moments_free(mi_metric* m);
 mi_status evaluate_moments(mi_metric* m, const SamplerParams& P, const double* jac0, const double* jacc, int nparams,
                            bool want_derivative, double* value, double* derivative, int64_t* valid);

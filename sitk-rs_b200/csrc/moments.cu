@@ -336,7 +336,7 @@ int grid_of(mi_context* ctx, int64_t n) {
 
 }  // namespace
 
-mi_status moments_setup(mi_metric* m) {
+mi_status moments_setup(mi_metric* m, const float* fixed) {
     mi_context* ctx = m->ctx;
     MomentsWs& w = m->mom;
     const int64_t n = m->n_samples;
@@ -351,12 +351,12 @@ mi_status moments_setup(mi_metric* m) {
     if (m->samples && m->n_samples > 0) {
         MI_CHECK_CUDA(ctx, dev_alloc(ctx, &w.fval, (size_t)m->n_samples * sizeof(float)));
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>((m->n_samples + 255) / 256, (int64_t)ctx->num_sms * 8));
-        k_gather_fixed<<<g, 256, 0, st>>>(m->fixed, m->samples, m->n_samples, w.fval);
+        k_gather_fixed<<<g, 256, 0, st>>>(fixed, m->samples, m->n_samples, w.fval);
         MI_CHECK_CUDA(ctx, cudaGetLastError());
     }
     if (ncc) {
         const int64_t nm = m->mgeo.size[0] * m->mgeo.size[1] * m->mgeo.size[2];
-        k_shift<<<1, 256, 0, st>>>(w.fval ? w.fval : m->fixed, n, m->moving, nm, w.shift);
+        k_shift<<<1, 256, 0, st>>>(w.fval ? w.fval : fixed, n, m->moving, nm, w.shift);
         MI_CHECK_CUDA(ctx, cudaGetLastError());
     }
     static_assert((NCC_SLOTS + 1) * sizeof(double) <= PINNED_BLOCK, "the moments' mirror is one pinned block");
