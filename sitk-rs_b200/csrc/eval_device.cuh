@@ -15,6 +15,7 @@
 #include <cstdint>
 
 #include "internal.h"
+#include "pdl.cuh"
 #include "sampler.cuh"
 
 namespace mi {
@@ -287,14 +288,6 @@ __device__ __forceinline__ void publish_seq(const EvalArgs& a, int np) {
             *reinterpret_cast<volatile unsigned long long*>(a.result_host + RESULT_ERR + 1) = h ^ publish_mix(a.seq);
     }
 }
-
-// Programmatic dependent launch: the histogram pass lets the launch that follows it
-// (launched with programmatic stream serialisation) be scheduled as its CTAs retire;
-// that launch waits here for the histogram pass to complete, with its writes
-// visible, before it reads any of them. Without the attribute the wait returns at
-// once.
-__device__ __forceinline__ void pdl_launch_dependents() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
 // ---------------------------------------------------------------------------
 // Pass 1: joint histogram (+ per-sample records for pass 2). The CTA histogram is

@@ -8,8 +8,8 @@
 //           a ring of shared-memory stages, as far ahead as the ring goes
 //   warp 1  one lane issues four tcgen05.mma per stage into one of two accumulators in
 //           tensor memory and commits the stage back to warp 0
-//   warps 2–5  read the other accumulator (tcgen05.ld, 32 rows a warp), turn 32 × 32
-//           blocks in shared memory and store whole 128-byte rows of C
+//   warps 2–5  read the other accumulator (tcgen05.ld, 32 rows a warp) and store 32 × 32
+//           blocks by TMA from shared memory, two in flight a warp
 // so copies, products and stores of neighbouring items overlap. Rows, columns and k past
 // the operands' ends arrive as zeros. Every element's products are accumulated in k
 // order, as in gemm_tc.cuh: same bits.
@@ -17,8 +17,11 @@
 // Bound: a 128 × 256 tile does 2·128·256·64 operations for 48 KB brought in and 48 KB read
 // by the tensor core, so shared-memory bandwidth and the tensor pipe are close; the ring
 // (four stages) covers L2's latency. Narrow products (NT ≤ 64) are bound by the bytes of A.
-// 4096³: 137 µs a call (1,005 TFLOP/s, 0.63 of 1.59 PFLOP/s; four rounds of CTAs for 3.46
-// rounds of tiles); the one-stage kernel of gemm_tc.cuh took 1,489 µs.
+// 4096³: 133 µs a call (1,033 TFLOP/s, 0.65 of 1.59 PFLOP/s; four rounds of CTAs for 3.46
+// rounds of tiles); the one-stage kernel of gemm_tc.cuh took 1,489 µs. Products of few k are
+// bound by their output: 32,768 × 432 × 32 writes 57 MB in 18 µs by TMA stores, 32 µs when
+// the four warps turned the blocks in shared memory and stored rows themselves (290
+// instructions a block).
 //
 // An operand may also be stored the other way round, k slowest ("k-rows": element (r, k) at
 // k·ld + r, as a product's transpose needs it): its tiles come as boxes of 64 rows × 64 k
@@ -33,6 +36,7 @@
 #include <cuda.h>
 
 #include "gemm_tc.cuh"
+#include "pdl.cuh"
 
 namespace mi {
 namespace tc {
@@ -44,8 +48,8 @@ template <int NT>
 struct TmaShape {
     static constexpr uint32_t A_BYTES = TILE_M * TILE_K * 2, B_BYTES = NT * TILE_K * 2;
     static constexpr uint32_t STAGE = A_BYTES + B_BYTES;
-    static constexpr uint32_t EPI = 4 * 32 * 36 * 4;  // four warps' 32 × 32 blocks, rows of 36 floats
-    static constexpr int FIT = (int)((220 * 1024 - EPI) / STAGE);
+    static constexpr uint32_t EPI = 4 * 2 * 32 * 32 * 4;  // four warps' 32 × 32 blocks, two each
+    static constexpr int FIT = (int)((225 * 1024 - EPI) / STAGE);
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
     static constexpr uint32_t BARS = STAGES * STAGE + EPI;
     static constexpr uint32_t SMEM = BARS + (2 * STAGES + 5) * 8 + 1024;  // and the alignment of the base
@@ -103,9 +107,11 @@ __device__ __forceinline__ uint64_t swizzled_desc_mn(uint32_t addr) {
            (2ull << 61);
 }
 
-// What becomes of an element z of the product: stored in C (where not null), and with X as
-// BF16 of z + bias[column], negative values cut off when relu is set. With a bias C gets
-// z + bias. Splits store the plain partial products.
+// What becomes of an element z of the product: stored in C, or where that is null as BF16 in
+// X; z + bias[column] with a bias (the layers' widths are multiples of four), negative
+// values cut off when relu is set. Splits store the plain partial products in C. With
+// `tma` the blocks leave by TMA through the output's map: pitch and base multiples of 16
+// bytes. X always goes that way.
 struct Epilogue {
     float* C;
     int ldc;
@@ -113,7 +119,25 @@ struct Epilogue {
     __nv_bfloat16* X;
     int ldx;
     int relu;
+    int tma;
 };
+
+// 16-byte chunk q of row `row` in a block of rows of ROW bytes, by TMA's swizzle of that width
+template <int ROW>
+__device__ __forceinline__ uint32_t block_chunk(int row, int q) {
+    static_assert(ROW == 32 || ROW == 64 || ROW == 128, "");
+    const int x = ROW == 128 ? row & 7 : (ROW == 64 ? (row >> 1) & 3 : (row >> 2) & 1);
+    return (uint32_t)(row * ROW + ((q ^ x) << 4));
+}
+__device__ __forceinline__ void st_shared16(uint32_t at, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+    asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};" ::"r"(at), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+}
+__device__ __forceinline__ void tma_store(const CUtensorMap* map, uint32_t src, int col, int row, int z) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(map), "r"(src),
+                 "r"(col), "r"(row), "r"(z)
+                 : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
 
 // Work item `item`: K slices slowest, then columns, rows fastest (CTAs that run together
 // share a B tile and the A tiles stay in L2).
@@ -144,8 +168,8 @@ __device__ __forceinline__ void request_tile(uint32_t dst, const CUtensorMap* ma
 
 template <int NT, bool A_KROWS, bool B_KROWS>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
-k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB, int M, int N, int K,
-           const Epilogue E, int splits, unsigned int* __restrict__ err) {
+k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+           const __grid_constant__ CUtensorMap mapOut, int M, int N, int K, const Epilogue E, int splits, unsigned int* __restrict__ err) {
     static_assert(!B_KROWS || NT % 64 == 0, "k-rows tiles come in boxes of 64");
     using S = TmaShape<NT>;
     extern __shared__ uint8_t raw[];
@@ -156,6 +180,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     const uint32_t full = bars, empty = bars + S::STAGES * 8, tfull = bars + S::STAGES * 16, tempty = tfull + 16,
                    drained = tempty + 16;
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    pdl::launch_dependents();
     if (threadIdx.x == 0) {
         for (int s = 0; s < S::STAGES; ++s) {
             bar_init(full + s * 8, 1);
@@ -178,6 +203,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = tmem_slot;
+    pdl::wait_previous();
 
     const int mt = (M + TILE_M - 1) / TILE_M, nt = (N + NT - 1) / NT;
     const int ktiles = (K + TILE_K - 1) / TILE_K, per = (ktiles + splits - 1) / splits;
@@ -263,10 +289,10 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         __syncwarp();
     } else {
         const int quad = warp & 3;  // the tensor-memory lanes this warp can read
-        float* block = reinterpret_cast<float*>(raw + (epi - smem_u32(raw))) + (warp - 2) * 32 * 36;
+        const uint32_t blocks = epi + (warp - 2) * 2 * 4096;
+        float* block = reinterpret_cast<float*>(raw + (blocks - smem_u32(raw)));
         const int ldc = E.ldc;
-        const bool vec = (ldc & 3) == 0 && ((uintptr_t)E.C & 15) == 0;
-        uint32_t tiles = 0;
+        uint32_t tiles = 0, stored = 0;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
             const Item w = item_at<NT>(it, mt, nt, ktiles, per);
             const bool any = w.kt0 < w.kt1;
@@ -275,7 +301,6 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                 if (!__all_sync(0xffffffffu, bar_wait(tfull + a * 8, (tiles >> 1) & 1, &quit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
-            float* out = E.C + (size_t)w.z * M * ldc;
             constexpr int W = NT < 32 ? NT : 32;  // columns a block
             const int row0 = w.m0 + quad * 32;
 #pragma unroll 1
@@ -301,44 +326,62 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 #pragma unroll
                     for (int q = 0; q < W; ++q) r[q] = 0u;
                 }
-                if (w.n0 + c0 >= N) continue;
+                const int col0 = w.n0 + c0;
+                if (col0 >= N || row0 >= M) continue;
+                if (E.bias) {
 #pragma unroll
-                for (int q = 0; q < W; q += 4)
-                    *reinterpret_cast<uint4*>(block + lane * 36 + q) = make_uint4(r[q], r[q + 1], r[q + 2], r[q + 3]);
-                __syncwarp();
-                constexpr int PER_ROW = W / 4, ROWS = 32 / PER_ROW;  // lanes a row, rows at once
-                const int q = (lane % PER_ROW) * 4, col = w.n0 + c0 + q;
+                    for (int q = 0; q < W; q += 4) {
+                        if (col0 + q >= N) break;
+                        const float4 b = __ldg(reinterpret_cast<const float4*>(E.bias + col0 + q));
+                        const float add[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
-                for (int i = 0; i < 32; i += ROWS) {
-                    const int rr = i + lane / PER_ROW, row = row0 + rr;
-                    if (row < M) {
-                        float4 v = *reinterpret_cast<const float4*>(block + rr * 36 + q);
-                        float* dst = out + (size_t)row * ldc + col;
-                        if (E.bias && col + 4 <= N) {  // the layers' widths are multiples of four
-                            const float4 b = __ldg(reinterpret_cast<const float4*>(E.bias + col));
-                            v = make_float4(v.x + b.x, v.y + b.y, v.z + b.z, v.w + b.w);
-                            if (E.X) {
-                                if (E.relu) v = make_float4(fmaxf(v.x, 0.f), fmaxf(v.y, 0.f), fmaxf(v.z, 0.f), fmaxf(v.w, 0.f));
-                                const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
-                                *reinterpret_cast<uint2*>(E.X + (size_t)row * E.ldx + col) =
-                                    make_uint2(*reinterpret_cast<const uint32_t*>(&lo), *reinterpret_cast<const uint32_t*>(&hi));
-                            }
-                        }
-                        if (!E.C) {
-                        } else if (vec && col + 4 <= N) {
-                            *reinterpret_cast<float4*>(dst) = v;
-                        } else {
-                            if (col < N) dst[0] = v.x;
-                            if (col + 1 < N) dst[1] = v.y;
-                            if (col + 2 < N) dst[2] = v.z;
-                            if (col + 3 < N) dst[3] = v.w;
+                        for (int k = 0; k < 4; ++k) {
+                            const float v = __uint_as_float(r[q + k]) + add[k];
+                            r[q + k] = __float_as_uint(E.relu ? fmaxf(v, 0.f) : v);
                         }
                     }
                 }
-                __syncwarp();
+                if (E.tma) {
+                    // the block of two stores ago has been read
+                    if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+                    __syncwarp();
+                    const uint32_t at = blocks + (stored++ & 1) * 4096;
+                    if (E.C) {
+#pragma unroll
+                        for (int q = 0; q < W / 4; ++q)
+                            st_shared16(at + block_chunk<W * 4>(lane, q), r[4 * q], r[4 * q + 1], r[4 * q + 2], r[4 * q + 3]);
+                    } else {
+                        uint32_t h[W / 2];
+#pragma unroll
+                        for (int q = 0; q < W / 2; ++q) {
+                            const __nv_bfloat162 v =
+                                __floats2bfloat162_rn(__uint_as_float(r[2 * q]), __uint_as_float(r[2 * q + 1]));
+                            h[q] = *reinterpret_cast<const uint32_t*>(&v);
+                        }
+#pragma unroll
+                        for (int q = 0; q < W / 8; ++q)
+                            st_shared16(at + block_chunk<W * 2>(lane, q), h[4 * q], h[4 * q + 1], h[4 * q + 2], h[4 * q + 3]);
+                    }
+                    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+                    __syncwarp();
+                    if (lane == 0) tma_store(&mapOut, at, col0, row0, w.z);
+                } else {
+                    // any pitch and base: each row's columns by the lanes in turn
+#pragma unroll
+                    for (int q = 0; q < W; q += 4)
+                        *reinterpret_cast<uint4*>(block + lane * 36 + q) = make_uint4(r[q], r[q + 1], r[q + 2], r[q + 3]);
+                    __syncwarp();
+                    float* out = E.C + ((size_t)w.z * M + row0) * ldc + col0;
+                    if (lane < W && col0 + lane < N)
+#pragma unroll 8
+                        for (int i = 0; i < 32; ++i)
+                            if (row0 + i < M) out[(size_t)i * ldc + lane] = block[i * 36 + lane];
+                    __syncwarp();
+                }
             }
             if (any) ++tiles;
         }
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");  // its memory is read, C written
     }
     __syncthreads();
     if (threadIdx.x == 0 && quit) *reinterpret_cast<volatile unsigned int*>(err) = 1u;

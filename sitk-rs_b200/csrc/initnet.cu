@@ -8,11 +8,13 @@
 //
 // Every convolution runs as a GEMM over im2col rows (channels-last activations; the
 // column index of an im2col row is ((kz·3 + ky)·3 + kx)·Cin + c), forward and
-// backward, on the tcgen05 BF16 GEMM (gemm_tc.cuh) with FP32 accumulation: forward
+// backward, on the tcgen05 BF16 GEMM (gemm_tma.cuh) with FP32 accumulation: forward
 // Y = Xcol·Wᵀ; weight gradient dW = dYᵀ·Xcol; input gradient dXcol = dY·W, gathered
-// back to the input grid (col2im as a gather, so deterministic). Operands that a TN
-// GEMM needs K-contiguous are transposed into BF16 first. Master weights, biases and
-// Adam moments are FP32. No reference counterpart.
+// back to the input grid (col2im as a gather, so deterministic). Master weights, biases
+// and Adam moments are FP32. The 31 launches of a step are programmatic dependents of one
+// another, so that each one's launch and set-up overlap the end of the one before: with
+// the stores by TMA a step takes 274 µs for 64 pairs and 140 µs for one (about 390 µs for 64
+// before both). No reference counterpart.
 #include <cuda_bf16.h>
 
 #include <algorithm>
@@ -24,6 +26,7 @@
 #include "gemm_tc.cuh"
 #include "gemm_tma.cuh"
 #include "internal.h"
+#include "pdl.cuh"
 
 namespace mi {
 
@@ -63,15 +66,34 @@ bool operand_map(CUtensorMap* map, const Operand& o, int rows, int K, int box) {
                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
 }
 
+// The map of a product's output (rows × N, `splits` of them one after another) in blocks of 32
+// rows × min(nt, 32) columns, swizzled by their rows' bytes. False where TMA cannot
+// write it.
+bool output_map(CUtensorMap* map, const tc::Epilogue& E, int M, int N, int splits, int nt) {
+    const bool f32 = E.C != nullptr;
+    const cuuint64_t size = f32 ? 4 : 2, pitch = (cuuint64_t)(f32 ? E.ldc : E.ldx) * size;
+    void* p = f32 ? (void*)E.C : (void*)E.X;
+    // a row that ended inside 16 bytes would clear the rest of them
+    if (pitch % 16 != 0 || (cuuint64_t)N * size % 16 != 0 || ((uintptr_t)p & 15) != 0 || !tensor_map_encoder()) return false;
+    const cuuint32_t w = (cuuint32_t)std::min(nt, 32), row = w * (cuuint32_t)size;
+    const cuuint64_t dim[3] = {(cuuint64_t)N, (cuuint64_t)M, (cuuint64_t)splits}, stride[2] = {pitch, pitch * (cuuint64_t)M};
+    const cuuint32_t bx[3] = {w, 32, 1}, es[3] = {1, 1, 1};
+    return tensor_map_encoder()(map, f32 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, p, dim,
+                                stride, bx, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                                row == 128  ? CU_TENSOR_MAP_SWIZZLE_128B
+                                : row == 64 ? CU_TENSOR_MAP_SWIZZLE_64B
+                                            : CU_TENSOR_MAP_SWIZZLE_32B,
+                                CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 template <int NT, bool AK, bool BK>
 cudaError_t launch_tma(mi_context* ctx, int M, int N, int K, const CUtensorMap& a, const CUtensorMap& b,
-                       const tc::Epilogue& E, int splits, unsigned int* err) {
+                       const CUtensorMap& out, const tc::Epilogue& E, int splits, unsigned int* err) {
     constexpr uint32_t sm = tc::TmaShape<NT>::SMEM;
     if (raise_smem_limit(ctx, (const void*)tc::k_gemm_tma<NT, AK, BK>, sm) != MI_OK) return cudaErrorInvalidValue;
     const int64_t items = (int64_t)((M + tc::TILE_M - 1) / tc::TILE_M) * ((N + NT - 1) / NT) * splits;
     const int grid = (int)std::min<int64_t>(items, ctx->num_sms);
-    tc::k_gemm_tma<NT, AK, BK><<<grid, tc::TMA_THREADS, sm, ctx->stream>>>(a, b, M, N, K, E, splits, err);
-    return cudaGetLastError();
+    return pdl::launch(tc::k_gemm_tma<NT, AK, BK>, grid, tc::TMA_THREADS, sm, ctx->stream, a, b, out, M, N, K, E, splits, err);
 }
 
 // The N tile of the TMA kernel. Its tiles are 128 × 256 where that leaves at least as few
@@ -90,13 +112,15 @@ int tma_n_tile(mi_context* ctx, int M, int N, int splits) {
 // The product by TMA: E's outputs, or with splits > 1 the K slices' partial products one
 // after another in E.C (M × ldc each). cudaErrorNotSupported where TMA cannot read an
 // operand. Both operands may be k_rows, or B alone.
-cudaError_t product(mi_context* ctx, int M, int N, int K, const Operand& A, const Operand& B, const tc::Epilogue& E,
+cudaError_t product(mi_context* ctx, int M, int N, int K, const Operand& A, const Operand& B, tc::Epilogue E,
                     int splits, unsigned int* err) {
     int nt = tma_n_tile(ctx, M, N, splits);
     if (B.k_rows) nt = std::max(nt, 64);
-    CUtensorMap a, b;
+    CUtensorMap a, b, out = {};
     if (!operand_map(&a, A, M, K, tc::TILE_M) || !operand_map(&b, B, N, K, nt)) return cudaErrorNotSupported;
-#define MI_PRODUCT(NT, AK, BK) return launch_tma<NT, AK, BK>(ctx, M, N, K, a, b, E, splits, err)
+    E.tma = output_map(&out, E, M, N, splits, nt);
+    if (!E.tma && !E.C) return cudaErrorNotSupported;
+#define MI_PRODUCT(NT, AK, BK) return launch_tma<NT, AK, BK>(ctx, M, N, K, a, b, out, E, splits, err)
     if (A.k_rows) {
         switch (nt) {
             case 64: MI_PRODUCT(64, true, true);
@@ -126,7 +150,7 @@ cudaError_t product(mi_context* ctx, int M, int N, int K, const Operand& A, cons
 cudaError_t gemm_dispatch(mi_context* ctx, int M, int N, int K, const __nv_bfloat16* A, int lda, const __nv_bfloat16* B,
                           int ldb, float* C, int ldc, int splits, unsigned int* err) {
     const cudaError_t e = product(ctx, M, N, K, Operand{A, lda, false}, Operand{B, ldb, false},
-                                  tc::Epilogue{C, ldc, nullptr, nullptr, 0, 0}, splits, err);
+                                  tc::Epilogue{C, ldc, nullptr, nullptr, 0, 0, 0}, splits, err);
     if (e != cudaErrorNotSupported) return e;
     cudaStream_t st = ctx->stream;
     switch (n_tile(N)) {
@@ -144,7 +168,10 @@ constexpr int FC1_IN = 128 * 8, FC1_OUT = 256, FC2_OUT = 12;
 constexpr int NLAYER = NCONV + 2;
 
 inline int kraw(int l) { return 27 * CH[l]; }          // im2col width of conv l (0-based)
-inline int kpad(int l) { return (kraw(l) + 7) & ~7; }  // padded to 16-byte rows
+// padded to 16-byte rows, the first layer's to a whole tile: its 262,144 rows' product (64
+// pairs) takes 18.5–20.3 µs where TMA fills 56 columns up to 64, 12.7 µs with 64 stored (the
+// others' last tiles are one in seven or fewer)
+inline int kpad(int l) { return l == 0 ? 64 : (kraw(l) + 7) & ~7; }
 
 inline int grid1(int64_t n) {
     const int64_t g = (n + 255) / 256;
@@ -165,39 +192,43 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // im2col of a channels-last volume (B × D³ × CIN) for a 3³ stride-2 pad-1 convolution: row
 // (b, z, y, x) of the D/2 output grid, column ((kz·3+ky)·3+kx)·CIN + c, zeros to KP columns.
 // A thread fills eight columns (16 bytes): eight channels of one tap, or, in the first
-// layer, both channels of four taps, read from the FP32 input and rounded here. With
-// one column a thread and divisions by run-time sizes the two large layers took 138
-// and 131 µs for 64 pairs (29 MB written each).
+// layer, both channels of four taps, read from the FP32 input and rounded here. Bound by
+// the bytes written (34 and 28 MB in the two large layers for 64 pairs: 17 and 10.5 µs with
+// cold caches; 22.6 and 13.2 µs with 64-bit indices over all pairs). A CTA's rows are the
+// same in every pair, blockIdx.y.
 template <int D, int CIN, int KP, typename T>
 __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, __nv_bfloat16* __restrict__ col) {
-    constexpr int Do = D / 2, PARTS = KP / 8;
-    const int64_t n = (int64_t)B * Do * Do * Do * PARTS;
-    GSTRIDE(i, n) {
-        const int part = (int)(i % PARTS);
-        const int64_t row = i / PARTS;
-        const int xo = (int)(row % Do), yo = (int)(row / Do % Do), zo = (int)(row / (Do * Do) % Do);
-        const int64_t b = row / (Do * Do * Do);
-        auto at = [&](int t) -> const T* {  // the input voxel under tap t, or null
-            const int xi = 2 * xo + t % 3 - 1, yi = 2 * yo + t / 3 % 3 - 1, zi = 2 * zo + t / 9 - 1;
-            if (t >= 27 || (unsigned)xi >= (unsigned)D || (unsigned)yi >= (unsigned)D || (unsigned)zi >= (unsigned)D)
-                return nullptr;
-            return x + (((b * D + zi) * D + yi) * D + xi) * CIN;
-        };
+    constexpr uint32_t Do = D / 2, PARTS = KP / 8, N = Do * Do * Do * PARTS;
+    pdl::launch_dependents();
+    const uint32_t i = blockIdx.x * 256 + threadIdx.x;  // of a sample's rows
+    pdl::wait_previous();
+    if (i >= N) return;
+    const uint32_t part = i % PARTS, row = i / PARTS;
+    const int xo = (int)(row % Do), yo = (int)(row / Do % Do), zo = (int)(row / (Do * Do));
+    int off[CIN == 2 ? 4 : 1];  // the input voxel under the tap, -1: none
+#pragma unroll
+    for (int q = 0; q < (CIN == 2 ? 4 : 1); ++q) {
+        const int t = CIN == 2 ? (int)part * 4 + q : (int)(part / (CIN / 8));
+        const int xi = 2 * xo + t % 3 - 1, yi = 2 * yo + t / 3 % 3 - 1, zi = 2 * zo + t / 9 - 1;
+        off[q] = t < 27 && (unsigned)xi < (unsigned)D && (unsigned)yi < (unsigned)D && (unsigned)zi < (unsigned)D
+                     ? (zi * D + yi) * D + xi
+                     : -1;
+    }
+    for (int b = blockIdx.y; b < B; b += gridDim.y) {
+        const T* in = x + (size_t)b * (D * D * D * CIN);
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
         if constexpr (CIN == 2) {
             uint32_t w[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const T* p = at(part * 4 + q);
-                const float2 f = p ? __ldg(reinterpret_cast<const float2*>(p)) : make_float2(0.f, 0.f);
+                const float2 f = off[q] >= 0 ? __ldg(reinterpret_cast<const float2*>(in) + off[q]) : make_float2(0.f, 0.f);
                 w[q] = pack_bf16(f.x, f.y);
             }
             v = make_uint4(w[0], w[1], w[2], w[3]);
         } else {
-            const T* p = at(part / (CIN / 8));
-            if (p) v = __ldg(reinterpret_cast<const uint4*>(p + part % (CIN / 8) * 8));
+            if (off[0] >= 0) v = __ldg(reinterpret_cast<const uint4*>(in + (size_t)off[0] * CIN + part % (CIN / 8) * 8));
         }
-        reinterpret_cast<uint4*>(col)[i] = v;
+        reinterpret_cast<uint4*>(col)[(size_t)b * N + i] = v;
     }
 }
 
@@ -205,6 +236,8 @@ __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, 
 // the bias, ReLU, BF16.
 __global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t mn, const float* __restrict__ bias,
                              int cols, __nv_bfloat16* __restrict__ x) {
+    pdl::launch_dependents();
+    pdl::wait_previous();
     GSTRIDE(i, mn) {
         float acc = 0.0f;
         for (int s = 0; s < splits; ++s) acc += part[(int64_t)s * mn + i];
@@ -218,14 +251,18 @@ __global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t
 // from the layer's product dcol: for a fully connected layer it is dcol itself (D = 0); for
 // a convolution over D³ inputs of C channels it is the transpose of im2col as a gather,
 // the output voxels and taps that read the input voxel, in a fixed order. A thread keeps
-// four channels, so that its sums stay in registers. (Gather, ReLU, conversion and sums
-// were five launches; the sums, 4,096 rows a thread in order, took 0.9–1.1 ms each.)
+// four channels, so that its sums stay in registers, and requests all of a voxel's up to
+// eight values before it adds them: 57 MB of the first layer's dcol in 30 µs with cold
+// caches, 43 µs tap by tap. (Gather, ReLU, conversion and sums were five launches; the
+// sums, 4,096 rows a thread in order, took 0.9–1.1 ms each.)
 template <int D, int C, int KP>
 __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol, const __nv_bfloat16* __restrict__ a,
                                                   int64_t rows, __nv_bfloat16* __restrict__ dzb, float* __restrict__ part) {
     constexpr int G = C / 4;  // threads a row
     static_assert(256 % G == 0, "a thread's channels stay the same");
     __shared__ float4 sums[256];
+    pdl::launch_dependents();
+    pdl::wait_previous();
     const int c = (threadIdx.x % G) * 4;
     float4 sum = make_float4(0.f, 0.f, 0.f, 0.f);
     for (int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) / G; r < rows; r += (int64_t)gridDim.x * (256 / G)) {
@@ -234,27 +271,36 @@ __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol
             v = __ldg(reinterpret_cast<const float4*>(dcol + r * C + c));
         } else {
             constexpr int Do = D / 2;
-            const int xi = (int)(r % D), yi = (int)(r / D % D), zi = (int)(r / (D * D) % D);
+            const uint32_t in = (uint32_t)(r % (D * D * D));
+            const int xi = (int)(in % D), yi = (int)(in / D % D), zi = (int)(in / (D * D));
             const int64_t b = r / (D * D * D);
+            // Per axis an even input voxel is read by tap 1 of output i/2 alone, an odd one by tap
+            // 0 of the output after it (if there is one) and by tap 2 of the one before: two
+            // slots an axis, eight loads at once.
+            int o[3][2], tap[3][2];
+            const int at[3] = {zi, yi, xi};
 #pragma unroll
-            for (int kz = 0; kz < 3; ++kz) {
-                const int tz = zi + 1 - kz;
-                if (tz < 0 || (tz & 1) || tz / 2 >= Do) continue;
+            for (int d = 0; d < 3; ++d) {
+                const int odd = at[d] & 1;
+                o[d][0] = (at[d] + odd) >> 1;
+                tap[d][0] = odd ? 0 : 1;
+                if (o[d][0] >= Do) tap[d][0] = -1;
+                o[d][1] = at[d] >> 1;
+                tap[d][1] = odd ? 2 : -1;
+            }
+            float4 t[8];
 #pragma unroll
-                for (int ky = 0; ky < 3; ++ky) {
-                    const int ty = yi + 1 - ky;
-                    if (ty < 0 || (ty & 1) || ty / 2 >= Do) continue;
-#pragma unroll
-                    for (int kx = 0; kx < 3; ++kx) {
-                        const int tx = xi + 1 - kx;
-                        if (tx < 0 || (tx & 1) || tx / 2 >= Do) continue;
-                        const int64_t row = ((b * Do + tz / 2) * Do + ty / 2) * Do + tx / 2;
-                        const float4 t =
-                            __ldg(reinterpret_cast<const float4*>(dcol + row * KP + ((kz * 3 + ky) * 3 + kx) * C + c));
-                        v = make_float4(v.x + t.x, v.y + t.y, v.z + t.z, v.w + t.w);
-                    }
+            for (int q = 0; q < 8; ++q) {
+                const int z = q >> 2, y = (q >> 1) & 1, xx = q & 1;
+                t[q] = make_float4(0.f, 0.f, 0.f, 0.f);
+                if (tap[0][z] >= 0 && tap[1][y] >= 0 && tap[2][xx] >= 0) {
+                    const int64_t row = ((b * Do + o[0][z]) * Do + o[1][y]) * Do + o[2][xx];
+                    t[q] = __ldg(reinterpret_cast<const float4*>(dcol + row * KP +
+                                                                 ((tap[0][z] * 3 + tap[1][y]) * 3 + tap[2][xx]) * C + c));
                 }
             }
+#pragma unroll
+            for (int q = 0; q < 8; ++q) v = make_float4(v.x + t[q].x, v.y + t[q].y, v.z + t[q].z, v.w + t[q].w);
         }
         const uint2 act = __ldg(reinterpret_cast<const uint2*>(a + r * C + c));
         // ReLU outputs: not negative, so positive means not zero
@@ -282,6 +328,8 @@ __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, cons
                                              __nv_bfloat16* __restrict__ dzb, int ld, float* __restrict__ colsum,
                                              float* __restrict__ loss) {
     __shared__ float red[256];
+    pdl::launch_dependents();
+    pdl::wait_previous();
     const int n = rows * cols;
     float acc = 0.0f;
     for (int i = threadIdx.x; i < n; i += 256) {
@@ -340,6 +388,8 @@ __global__ void __launch_bounds__(256) k_update(const __grid_constant__ Tensors 
     const int blk = (int)blockIdx.x - t.block0;
     int i;
     float g = 0.0f;
+    pdl::launch_dependents();
+    pdl::wait_previous();
     if (t.parts >= WIDE_PARTS) {
         const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
         i = blk * 32 + lane;
@@ -499,29 +549,27 @@ cudaError_t layer_forward(mi_initnet* n, int l, int B, const __nv_bfloat16* x, f
     const Operand a{x, L.kp, false}, w{L.wb, L.kp, false};
     __nv_bfloat16* act = n->xb[l];
     if (S == 1)
-        return product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{y, L.out, L.b, act, L.out, 1}, 1, n->host_dev);
-    const cudaError_t e = product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{n->slices, L.out, nullptr, nullptr, 0, 0}, S,
+        return product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{y, L.out, L.b, act, L.out, y ? 0 : 1, 0}, 1, n->host_dev);
+    const cudaError_t e = product(n->ctx, M, L.out, L.kp, a, w, tc::Epilogue{n->slices, L.out, nullptr, nullptr, 0, 0, 0}, S,
                                   n->host_dev);
     if (e != cudaSuccess) return e;
     const int64_t mn = (int64_t)M * L.out;
-    k_slices_act<<<grid1(mn), 256, 0, n->ctx->stream>>>(n->slices, S, mn, L.b, L.out, act);
-    return cudaGetLastError();
+    return pdl::launch(k_slices_act, grid1(mn), 256, 0, n->ctx->stream, n->slices, S, mn, L.b, L.out, act);
 }
 
 // forward pass of B samples (input x: B × 32³ × 2 FP32, channels-last) into out (B × 12)
 cudaError_t forward(mi_initnet* n, int B, const float* x, float* out) {
     cudaStream_t st = n->ctx->stream;
-    auto grid = [&](int l) { return grid1(rows_of(l, B) * (n->L[l].kp / 8)); };
+    auto grid = [&](int l) { return dim3((unsigned)((rows_of(l, 1) * (n->L[l].kp / 8) + 255) / 256), (unsigned)std::min(B, 65535)); };
     cudaError_t e = cudaSuccess;
     for (int l = 0; l < NCONV && e == cudaSuccess; ++l) {
         __nv_bfloat16* col = n->col[l];
         switch (l) {
-            case 0: k_im2col<DIM[0], CH[0], 56, float><<<grid(l), 256, 0, st>>>(x, B, col); break;
-            case 1: k_im2col<DIM[1], CH[1], 27 * CH[1], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[0], B, col); break;
-            case 2: k_im2col<DIM[2], CH[2], 27 * CH[2], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[1], B, col); break;
-            default: k_im2col<DIM[3], CH[3], 27 * CH[3], __nv_bfloat16><<<grid(l), 256, 0, st>>>(n->xb[2], B, col); break;
+            case 0: e = pdl::launch(k_im2col<DIM[0], CH[0], 64, float>, grid(l), 256, 0, st, x, B, col); break;
+            case 1: e = pdl::launch(k_im2col<DIM[1], CH[1], 27 * CH[1], __nv_bfloat16>, grid(l), 256, 0, st, n->xb[0], B, col); break;
+            case 2: e = pdl::launch(k_im2col<DIM[2], CH[2], 27 * CH[2], __nv_bfloat16>, grid(l), 256, 0, st, n->xb[1], B, col); break;
+            default: e = pdl::launch(k_im2col<DIM[3], CH[3], 27 * CH[3], __nv_bfloat16>, grid(l), 256, 0, st, n->xb[2], B, col); break;
         }
-        e = cudaGetLastError();
         if (e == cudaSuccess) e = layer_forward(n, l, B, col, nullptr);
     }
     // fc1 on the flattened conv output (B × 1024), fc2 without activation
@@ -535,13 +583,10 @@ cudaError_t forward(mi_initnet* n, int B, const float* x, float* out) {
 cudaError_t backward(mi_initnet* n, int B, const float* t) {
     mi_context* ctx = n->ctx;
     cudaStream_t st = ctx->stream;
-    {
-        Layer& top = n->L[NLAYER - 1];
-        k_mse<<<1, 256, 0, st>>>(n->out, t, B, FC2_OUT, top.dzb, dz_ld(FC2_OUT), top.bpart,
-                                 reinterpret_cast<float*>(n->host_dev + 1));
-        top.bparts = 1;
-    }
-    cudaError_t e = cudaGetLastError();
+    Layer& top = n->L[NLAYER - 1];
+    cudaError_t e = pdl::launch(k_mse, 1, 256, 0, st, n->out, t, B, FC2_OUT, top.dzb, dz_ld(FC2_OUT), top.bpart,
+                                reinterpret_cast<float*>(n->host_dev + 1));
+    top.bparts = 1;
     for (int l = NLAYER - 1; l >= 0 && e == cudaSuccess; --l) {
         Layer& L = n->L[l];
         const int rows = (int)rows_of(l, B);
@@ -551,12 +596,12 @@ cudaError_t backward(mi_initnet* n, int B, const float* t) {
         // dW (out × kp) = dZᵀ · X, k the rows
         L.wparts = k_splits(L.out, L.kp, rows);
         e = product(ctx, L.out, L.kp, rows, dzt, Operand{xin, L.kp, true},
-                    tc::Epilogue{L.wparts > 1 ? L.wpart : L.gw, L.kp, nullptr, nullptr, 0, 0}, L.wparts, n->host_dev);
+                    tc::Epilogue{L.wparts > 1 ? L.wpart : L.gw, L.kp, nullptr, nullptr, 0, 0, 0}, L.wparts, n->host_dev);
         if (l == 0 || e != cudaSuccess) break;
         // the gradient of the layer's input (rows × kp) = dZ · W (out is at most four k tiles, so
         // never split)
         e = product(ctx, rows, L.kp, L.out, dz, Operand{L.wb, L.kp, true},
-                    tc::Epilogue{n->dcol, L.kp, nullptr, nullptr, 0, 0}, 1, n->host_dev);
+                    tc::Epilogue{n->dcol, L.kp, nullptr, nullptr, 0, 0, 0}, 1, n->host_dev);
         if (e != cudaSuccess) break;
         // back to the previous layer's activations, through its ReLU
         Layer& P = n->L[l - 1];
@@ -565,13 +610,12 @@ cudaError_t backward(mi_initnet* n, int B, const float* t) {
         const int grid = (int)std::min<int64_t>(BACK_CTAS, (prows * (P.out / 4) + 255) / 256);
         P.bparts = grid;
         switch (l) {
-            case 1: k_back_act<DIM[1], CH[1], 27 * CH[1]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
-            case 2: k_back_act<DIM[2], CH[2], 27 * CH[2]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
-            case 3: k_back_act<DIM[3], CH[3], 27 * CH[3]><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
-            case 4: k_back_act<0, CH[4], 0><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
-            default: k_back_act<0, FC1_OUT, 0><<<grid, 256, 0, st>>>(n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 1: e = pdl::launch(k_back_act<DIM[1], CH[1], 27 * CH[1]>, grid, 256, 0, st, n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 2: e = pdl::launch(k_back_act<DIM[2], CH[2], 27 * CH[2]>, grid, 256, 0, st, n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 3: e = pdl::launch(k_back_act<DIM[3], CH[3], 27 * CH[3]>, grid, 256, 0, st, n->dcol, act, prows, P.dzb, P.bpart); break;
+            case 4: e = pdl::launch(k_back_act<0, CH[4], 0>, grid, 256, 0, st, n->dcol, act, prows, P.dzb, P.bpart); break;
+            default: e = pdl::launch(k_back_act<0, FC1_OUT, 0>, grid, 256, 0, st, n->dcol, act, prows, P.dzb, P.bpart); break;
         }
-        e = cudaGetLastError();
     }
     return e;
 }
@@ -591,8 +635,7 @@ cudaError_t update(mi_initnet* n, float lr) {
         add(Tensor{L.w, L.gw, L.mw, L.vw, L.wb, L.wparts > 1 ? L.wpart : nullptr, L.out * L.kp, L.wparts, 0});
         add(Tensor{L.b, L.gb, L.mb, L.vb, nullptr, L.bpart, L.out, L.bparts, 0});
     }
-    k_update<<<blocks, 256, 0, n->ctx->stream>>>(T, lr, b1, b2, c1, c2, 1e-8f);
-    return cudaGetLastError();
+    return pdl::launch(k_update, blocks, 256, 0, n->ctx->stream, T, lr, b1, b2, c1, c2, 1e-8f);
 }
 
 }  // namespace

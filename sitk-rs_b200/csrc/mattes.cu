@@ -117,7 +117,7 @@ template <bool RECORD>
 __global__ void __launch_bounds__(HIST_BLOCK, HIST_MIN_BLOCKS)
 k_hist(const __grid_constant__ SamplerParams P, EvalArgs a) {
     extern __shared__ __align__(16) unsigned int sh[];
-    pdl_launch_dependents();
+    pdl::launch_dependents();
     hist_phase<RECORD, (HIST_CLUSTER > 1)>(P, a, sh, grid_samples(a.n), exact_queue(a));
     // the value+derivative evaluation's tail is formed by k_deriv's CTAs; a value-only
     // evaluation ends here, with its tail in the CTA that flushes last
@@ -132,7 +132,7 @@ k_hist(const __grid_constant__ SamplerParams P, EvalArgs a) {
 __global__ void __launch_bounds__(DERIV_BLOCK, DERIV_MIN_BLOCKS)
 k_deriv(const __grid_constant__ SamplerParams P, const __grid_constant__ JacobianForm J, EvalArgs a) {
     extern __shared__ double dsh[];
-    pdl_wait();
+    pdl::wait_previous();
     const TailCtx t = stream_phase(P, a, dsh, grid_groups(a));
     if (!last_to_arrive(a.sync)) return;
     // every CTA has read the histogram and written its value slices and moments; the
@@ -152,7 +152,7 @@ __global__ void __launch_bounds__(TILE_BLOCK, 1)
 k_hist_tile(const __grid_constant__ SamplerParams P, EvalArgs a, const __grid_constant__ CUtensorMap tmap,
             TileArgs T) {
     extern __shared__ __align__(128) unsigned char tsh[];
-    pdl_launch_dependents();
+    pdl::launch_dependents();
     tile_hist_phase<RECORD>(P, a, &tmap, T, tsh);
     if (RECORD || !last_to_arrive(a.sync + 1)) return;
     tail_once(P.bins, P.moving_bin_size, a, tsh, true);

@@ -51,3 +51,18 @@ def test_both_forms_give_the_same_bits(M, N, K):
     A1[:, :K] = A
     C, C1 = torch.empty((M, N), device="cuda"), torch.empty((M, N), device="cuda")
     assert np.array_equal(_gemm(A, B, C).cpu().numpy(), _gemm(A1[:, :K], B, C1).cpu().numpy())
+
+
+@pytest.mark.parametrize("M,N,pitch,first", [
+    (33, 20, 24, 0), (161, 36, 48, 4), (31, 44, 64, 8), (129, 148, 152, 4), (97, 260, 264, 0),  # blocks stored by TMA
+    (33, 20, 25, 0), (161, 36, 48, 1), (31, 43, 48, 0)])                                        # by lanes
+def test_output_blocks_end_where_the_product_does(M, N, pitch, first):
+    import torch
+    g = torch.Generator().manual_seed(M * N)
+    A = torch.randint(-3, 4, (M, 72), generator=g).to(torch.bfloat16).cuda()
+    B = torch.randint(-3, 4, (N, 72), generator=g).to(torch.bfloat16).cuda()
+    C = torch.full((M + 2, pitch), -7.0, device="cuda")
+    want = C.clone()
+    want[1:M + 1, first:first + N] = (A.double() @ B.double().T).float()  # integers below 2^24: exact
+    _gemm(A, B, C[1:M + 1, first:first + N])
+    assert torch.equal(C, want)
