@@ -1,17 +1,17 @@
 // Batched registration: many pairs of uneven sizes advance one optimizer iteration
-// per pass of three launches — the histogram pass over every active pair's chunks,
-// the tail and derivative pass over the same chunks, and the optimizer step of every
-// pair — with all optimizer state on the device. A pass is captured in a CUDA graph
+// per pass of two launches — the histogram pass over every active pair's chunks, then
+// the tail and derivative pass over the same chunks, in which the CTA that finishes a
+// pair makes its optimizer step — with all optimizer state on the device. A pass is captured in a CUDA graph
 // (several passes per graph) and replayed until every pair has stopped; the host
 // only reads how many pairs are still active after each replay.
 //
 // Per pair the arithmetic is the single-pair path's: the same sampler, histogram,
 // tail and moment code (eval_device.cuh), the same regular-step gradient descent
 // (rsgd.h) and the same point-map constants (point_map.h). What differs is the
-// launch shape: a pair's samples are cut into chunks of `chunk` samples, each CTA
-// takes chunks in turn (a persistent grid over the chunk list), and the fixed-point
-// unit of the histogram follows from the chunk size, so values agree with the
-// single-pair path to that unit.
+// launch shape: a pair's samples are cut into chunks of `chunk` samples, whose moments are
+// summed chunk by chunk, the CTAs take equal shares of the active pairs' samples and
+// chunks, and the fixed-point unit of the histogram follows from the chunk size, so
+// values agree with the single-pair path to that unit.
 //
 // The chunk size and the number of privatised histogram copies are chosen by a small
 // autotuner that times the candidates on the batch itself and caches the choice per
@@ -40,11 +40,15 @@ mi_status shift_corners(int kind, const double* params, int nparams, const doubl
 namespace mi {
 namespace {
 
-struct Chunk {
-    int pair;
-    int local;  // index among the pair's chunks
-    uint32_t begin, end;
+// What is left of a pair: nothing once it has stopped. Two lists: the first is read by the
+// histogram pass and cleared, entry by entry, by the steps in the derivative pass; that
+// pass reads the second, the histogram pass's copy, so that no list changes under its readers.
+struct Work {
+    unsigned int samples;  // rounded up to UNIT
+    unsigned int chunks;   // derivative chunks
 };
+constexpr unsigned int UNIT = 128;          // samples: a histogram share starts on whole 512-byte lines
+constexpr unsigned int LEAST_SHARE = 1024;  // samples a histogram CTA takes at least, two a thread
 
 struct PairDev {
     SamplerParams P;
@@ -93,84 +97,265 @@ __device__ void family_stage(int kind, const double* p, const double* center, do
     }
 }
 
-// Copies a pair's sampler constants into shared memory (read by every sample).
-__device__ __forceinline__ void load_params(const SamplerParams& src, SamplerParams& dst) {
-    const unsigned int* s = reinterpret_cast<const unsigned int*>(&src);
-    unsigned int* d = reinterpret_cast<unsigned int*>(&dst);
-    for (int i = threadIdx.x; i < (int)(sizeof(SamplerParams) / 4); i += blockDim.x) d[i] = s[i];
+// What a chunk's samples read of its pair, in shared memory (every pointer and constant would
+// otherwise be fetched from global memory again after each store).
+struct PairShared {
+    alignas(16) unsigned char params[sizeof(SamplerParams)];
+    alignas(16) unsigned char args[sizeof(EvalArgs)];
+    __device__ SamplerParams& P() { return *reinterpret_cast<SamplerParams*>(params); }
+    __device__ const EvalArgs& a() const { return *reinterpret_cast<const EvalArgs*>(args); }
+};
+__device__ __forceinline__ void copy_words(void* dst, const void* src, size_t bytes) {
+    const unsigned int* s = static_cast<const unsigned int*>(src);
+    unsigned int* d = static_cast<unsigned int*>(dst);
+    for (int i = threadIdx.x; i < (int)(bytes / 4); i += blockDim.x) d[i] = s[i];
+}
+static_assert(sizeof(SamplerParams) % 4 == 0 && sizeof(EvalArgs) % 4 == 0, "whole words");
+
+// The whole CTA.
+__device__ __forceinline__ void load_pair(const PairDev& pd, PairShared& sh) {
+    copy_words(sh.params, &pd.P, sizeof(SamplerParams));
+    copy_words(sh.args, &pd.a, sizeof(EvalArgs));
     __syncthreads();
 }
 
+// Positions along the pairs' remaining work, one after another: the whole CTA computes the
+// prefix sums of `key` over the pairs (thread t a run of consecutive ones), and locate()
+// finds the pair under a position.
+struct Line {
+    unsigned long long total;
+    unsigned long long first;  // of this thread's run
+    int lo, hi;                // the run
+};
+template <class Key>
+__device__ __forceinline__ Line lay_out(const Work* __restrict__ work, int npairs, Key key) {
+    __shared__ unsigned long long sums[32];
+    const int per = (npairs + (int)blockDim.x - 1) / (int)blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    Line l;
+    l.lo = min(npairs, (int)threadIdx.x * per);
+    l.hi = min(npairs, l.lo + per);
+    unsigned long long own = 0;
+    for (int p = l.lo; p < l.hi; ++p) own += key(work[p]);
+    unsigned long long scan = own;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        const unsigned long long o = __shfl_up_sync(0xffffffffu, scan, off);
+        if (lane >= off) scan += o;
+    }
+    if (lane == 31) sums[warp] = scan;
+    __syncthreads();
+    unsigned long long before = 0, total = 0;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) {
+        if (w < warp) before += sums[w];
+        total += sums[w];
+    }
+    l.first = before + scan - own;
+    l.total = total;
+    return l;
+}
+struct Place {
+    int pair;
+    unsigned long long start;  // the pair's first position
+};
+// at < l.total; the whole CTA
+template <class Key>
+__device__ __forceinline__ Place locate(const Work* __restrict__ work, const Line& l, unsigned long long at, Key key) {
+    __shared__ Place found;
+    __syncthreads();  // the last one was read
+    unsigned long long x = l.first;
+    for (int p = l.lo; p < l.hi; ++p) {
+        const unsigned long long n = key(work[p]);
+        if (at >= x && at - x < n) found = Place{p, x};
+        x += n;
+    }
+    __syncthreads();
+    return found;
+}
+
+// The histograms of every active pair. Integer sums, so any split of the samples gives the
+// same counts: the active pairs' samples are laid end to end and every CTA takes an equal
+// share, pair by pair, in segments short enough for the fixed-point unit (seg_max). A
+// pass of 24 pairs, 2.45 M samples: 55 µs; 61 µs with whole chunks of 4,096 in turn (610
+// over 296 CTAs, so three rounds for 2.06).
 __global__ void __launch_bounds__(HIST_BLOCK, HIST_MIN_BLOCKS)
-k_batch_hist(PairDev* __restrict__ pairs, const Chunk* __restrict__ chunks, int nchunks, uint32_t* __restrict__ exq,
-             uint32_t exq_cap) {
-    extern __shared__ unsigned int sh[];
-    __shared__ SamplerParams sP;
-    // this CTA's queue for the exact chain: a chunk at a time, so at most a chunk's samples
-    const ExactQueue q{MI_EXACT_DEFERRED ? exq + (size_t)blockIdx.x * exq_cap : nullptr, exq_cap};
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const Chunk ch = chunks[c];
-        PairDev& pd = pairs[ch.pair];
-        if (!pd.active) continue;
-        load_params(pd.P, sP);
-        hist_phase<true>(sP, pd.a, sh, SampleRange{ch.begin, ch.end, threadIdx.x & ~31u, blockDim.x}, q);
-        __syncthreads();
+k_batch_hist(PairDev* __restrict__ pairs, Work* __restrict__ work, int npairs, unsigned int seg_max,
+             uint32_t* __restrict__ exq) {
+    extern __shared__ __align__(16) unsigned int sh[];
+    __shared__ PairShared sp;
+    pdl::launch_dependents();
+    pdl::wait_previous();
+    // this CTA's queue for the exact chain: a segment at a time, so at most its samples
+    const ExactQueue q{MI_EXACT_DEFERRED ? exq + (size_t)blockIdx.x * seg_max : nullptr, seg_max};
+    const auto samples = [](const Work& w) { return w.samples; };
+    const Line line = lay_out(work, npairs, samples);
+    if (blockIdx.x == 0)  // the derivative pass's copy
+        for (int p = threadIdx.x; p < npairs; p += blockDim.x) work[npairs + p] = work[p];
+    unsigned long long share = (line.total + gridDim.x - 1) / gridDim.x;
+    share = max((share + UNIT - 1) / UNIT * UNIT, (unsigned long long)LEAST_SHARE);
+    const unsigned long long end = min(line.total, share * (blockIdx.x + 1));
+    for (unsigned long long at = share * blockIdx.x; at < end;) {
+        const Place pl = locate(work, line, at, samples);
+        const PairDev& pd = pairs[pl.pair];
+        load_pair(pd, sp);
+        const uint32_t n = sp.a().n;
+        const uint32_t first = (uint32_t)(at - pl.start);
+        const uint32_t last = (uint32_t)(min(pl.start + (n + UNIT - 1) / UNIT * UNIT, end) - pl.start);
+        const uint32_t len = last - first, segs = (len + seg_max - 1) / seg_max;
+        const uint32_t seg = ((len + segs - 1) / segs + UNIT - 1) / UNIT * UNIT;  // seg_max is a multiple of UNIT
+        for (uint32_t b = first; b < last; b += seg) {
+            const uint32_t e = min(min(b + seg, last), n);
+            if (b < e) hist_phase<true>(sp.P(), sp.a(), sh, SampleRange{b, e, threadIdx.x & ~31u, blockDim.x}, q);
+            __syncthreads();
+        }
+        at = pl.start + last;
     }
 }
 
-__global__ void __launch_bounds__(DERIV_BLOCK)
-k_batch_deriv(PairDev* __restrict__ pairs, const Chunk* __restrict__ chunks, int nchunks) {
-    extern __shared__ double dsh[];
-    __shared__ SamplerParams sP;
-    __shared__ bool last;
-    for (int c = blockIdx.x; c < nchunks; c += gridDim.x) {
-        const Chunk ch = chunks[c];
-        PairDev& pd = pairs[ch.pair];
-        if (!pd.active) continue;
-        load_params(pd.P, sP);
-        const uint32_t gend = ch.end == pd.a.n ? pd.a.npad >> 2 : ch.end >> 2;
-        const GroupWork w{ch.begin >> 2, gend, threadIdx.x, blockDim.x, pd.a.partials + ch.local,
-                          (int64_t)pd.nchunks, ch.local, pd.nchunks};
-        const TailCtx t = deriv_phase(sP, pd.a, dsh, w);
-        // the last chunk of the pair to finish folds the pair's moments and value
-        __threadfence();
-        __syncthreads();
-        if (threadIdx.x == 0) last = atomicAdd(&pd.done, 1u) == (unsigned int)pd.nchunks - 1u;
-        __syncthreads();
-        if (last) {
-            __threadfence();
-            deriv_fold(sP, pd.J, pd.a, t, pd.a.partials, (unsigned int)pd.nchunks);
-            if (threadIdx.x < 32) fold_value(sP.bins, pd.a, t);
-            if (threadIdx.x == 0) pd.done = 0u;
-            const int nb = sP.bins * sP.bins + sP.bins;
-            for (int i = threadIdx.x; i < nb; i += blockDim.x) pd.a.ghist[i] = 0ull;
+// The optimizer's part of a pair, staged for one thread.
+struct StepShared {
+    rsgd::State state;
+    double scaled[MI_MAX_PARAMS], params[MI_MAX_PARAMS], center[3], cmax;
+    int go;
+};
+
+// The optimizer's decision on the evaluation just made, then the next point map, by the CTA
+// that finished the pair's derivative, on copies in shared memory: one thread decides, the
+// divisions and the point map's bound are spread (9.6 µs with all of it by one thread, 10–14 µs as a launch of its
+// own of one thread a pair). P is that CTA's copy of the pair's constants.
+__device__ void step_pair(PairDev& pd, Work& work, SamplerParams& P, const mi_rsgd_config& cfg, unsigned int* active_count) {
+    __shared__ StepShared s;
+    const int np = pd.nparams;
+    copy_words(&s.state, &pd.state, sizeof(rsgd::State));
+    if ((int)threadIdx.x < np) {
+        s.scaled[threadIdx.x] = rsgd::div(pd.a.result[2 + threadIdx.x], pd.scales[threadIdx.x]);
+        s.params[threadIdx.x] = pd.params[threadIdx.x];
+    }
+    if (threadIdx.x < 3) s.center[threadIdx.x] = pd.center[threadIdx.x];
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        pd.evaluations += 1;
+        pd.value = pd.a.result[0];
+        pd.valid = pd.a.result[1];
+        s.go = rsgd::after_scaled(s.state, cfg, pd.corners, s.scaled, s.params) ? 0 : 1;
+        if (s.go) {
+            double stage[12];
+            family_stage(pd.kind, s.params, s.center, stage);
+            pm_stages(P, stage, 1);
+        } else {
+            pd.active = 0;
+            work = Work{0u, 0u};
+            pd.stop_ns = global_ns();
+            atomicSub(active_count, 1u);
+        }
+    }
+    __syncthreads();
+    copy_words(&pd.state, &s.state, sizeof(rsgd::State));
+    if (s.go) {
+        // point_map_fill, the corners in one warp beside the composite map
+        if (threadIdx.x == 0) pm_compose(P);
+        if (threadIdx.x >= 32 && threadIdx.x < 64) {
+            double m = pm_corner(P, threadIdx.x & 7);
+#pragma unroll
+            for (int off = 4; off; off >>= 1) m = fmax(m, __shfl_xor_sync(0xffffffffu, m, off));
+            if (threadIdx.x == 32) s.cmax = m;
         }
         __syncthreads();
+        if (threadIdx.x == 0) pm_bounds(P, s.cmax);
+        __syncthreads();
+        if ((int)threadIdx.x < np) pd.params[threadIdx.x] = s.params[threadIdx.x];
+        copy_words(&pd.P, &P, sizeof(SamplerParams));
     }
 }
 
-// One thread per pair: the optimizer's decision on the evaluation just made, then
-// the next point map.
-__global__ void k_batch_update(PairDev* __restrict__ pairs, int npairs, mi_rsgd_config cfg,
-                               unsigned int* __restrict__ active_count) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= npairs) return;
-    PairDev& pd = pairs[i];
-    if (!pd.active) return;
-    pd.evaluations += 1;
-    pd.value = pd.a.result[0];
-    pd.valid = pd.a.result[1];
-    double grad[MI_MAX_PARAMS];
-    for (int k = 0; k < pd.nparams; ++k) grad[k] = pd.a.result[2 + k];
-    if (rsgd::after_evaluation(pd.state, cfg, pd.corners, pd.scales, grad, pd.params)) {
-        pd.active = 0;
-        pd.stop_ns = global_ns();
-        atomicSub(active_count, 1u);
-        return;
+// A pair whose last chunk this CTA finished.
+struct Finished {
+    int pair;
+    TailCtx t;
+};
+constexpr int FINISHED_MAX = 4;
+
+// The tail and derivative of every active pair's chunks; with STEP the CTA that finishes a
+// pair also makes its optimizer step. A chunk's FP32 sums are its own, whoever forms them:
+// every CTA takes an equal run of consecutive chunks, so that a pair's table (k_deriv's,
+// stream_table: one round of requests and two barriers) is formed once for all of its
+// chunks here, and folds and steps the pairs it finished after its chunks, not between
+// them (up to FINISHED_MAX of them waiting). 24 pairs, 610 chunks: 40 µs; 65 µs with a tail
+// for every chunk, the steps a launch of their own.
+template <bool STEP>
+__global__ void __launch_bounds__(DERIV_BLOCK, DERIV_MIN_BLOCKS)
+k_batch_deriv(PairDev* __restrict__ pairs, Work* __restrict__ work, int npairs, unsigned int chunk, mi_rsgd_config cfg,
+              unsigned int* __restrict__ active_count) {
+    extern __shared__ double dsh[];
+    __shared__ PairShared sp;
+    __shared__ Finished done[FINISHED_MAX];
+    __shared__ bool last;
+    pdl::launch_dependents();
+    pdl::wait_previous();
+    // a pair's table weighs about as much as a chunk: its first position is the table's
+    const auto chunks = [](const Work& w) { return w.chunks ? w.chunks + 1u : 0u; };
+    const Work* left = work + npairs;
+    const Line line = lay_out(left, npairs, chunks);
+    const unsigned long long begin = line.total * blockIdx.x / gridDim.x, end = line.total * (blockIdx.x + 1) / gridDim.x;
+    int nfinished = 0, loaded = -1;
+    auto finish = [&]() {
+        for (int k = 0; k < nfinished; ++k) {
+            const int p = done[k].pair;
+            PairDev& pd = pairs[p];
+            if (p != loaded) load_pair(pd, sp);
+            loaded = p;
+            __threadfence();  // the other CTAs' moments and value slices
+            const EvalArgs& a = sp.a();
+            static_assert(DERIV_BLOCK >= 18 * NMOM + 32, "deriv_fold's value warp");
+            deriv_fold<true>(sp.P(), pd.J, a, done[k].t, a.partials, (unsigned int)pd.nchunks);
+            if (threadIdx.x == 0) pd.done = 0u;
+            const int B = sp.P().bins, nb = B * B + 2 * B;  // joint, counts, column sums
+            for (int i = threadIdx.x; i < nb; i += blockDim.x) a.ghist[i] = 0ull;
+            __syncthreads();
+            if (STEP) step_pair(pd, work[p], sp.P(), cfg, active_count);
+            __syncthreads();
+        }
+        nfinished = 0;
+    };
+    Place pl{-1, 0ull};
+    TableCtx tab;
+    unsigned int count = 0, mine = 0;  // the pair's chunks, and those done here
+    for (unsigned long long c = begin; c < end; ++c) {
+        const bool fresh = pl.pair < 0 || c - pl.start > count;
+        if (fresh) {
+            pl = locate(left, line, c, chunks);
+            if (c == pl.start && ++c == end) break;  // the first position is no chunk
+            count = (unsigned int)pairs[pl.pair].nchunks;
+            load_pair(pairs[pl.pair], sp);
+            loaded = pl.pair;
+        }
+        const EvalArgs& a = sp.a();
+        const unsigned int local = (unsigned int)(c - pl.start) - 1u, first = local * chunk;
+        const uint32_t gend = a.n - first <= chunk ? a.npad >> 2 : (first + chunk) >> 2;
+        const GroupWork w{first >> 2, gend, threadIdx.x, blockDim.x, a.partials + local, (int64_t)count, (int)local, (int)count};
+        RecordGroup cur;
+        if (fresh)
+            tab = stream_table<GridRecords>(sp.P(), a, dsh, w, cur);
+        else if (w.begin + w.first < w.end)
+            load_group(a, w.begin + w.first, cur);
+        stream_rows<GridRecords>(sp.P(), a, dsh, w, cur, tab);
+        ++mine;
+        __syncthreads();
+        if (c + 1 < end && local + 1 < count) continue;
+        // the pair's chunks here are done: with them the pair, if no other CTA has more to come
+        __threadfence();
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            last = atomicAdd(&pairs[pl.pair].done, mine) + mine == count;
+            if (last) done[nfinished] = Finished{pl.pair, tab.t};
+        }
+        mine = 0;
+        __syncthreads();
+        if (last && ++nfinished == FINISHED_MAX) {
+            finish();
+            pl.pair = -1;  // the table and the pair's constants may be another's now
+        }
     }
-    double stage[12];
-    family_stage(pd.kind, pd.params, pd.center, stage);
-    point_map_fill(pd.P, stage, 1);
+    finish();
 }
 
 // Autotuner cache: (bins, log2 of the total sample count) → (chunk, coarse copies).
@@ -187,8 +372,9 @@ struct mi_batch {
     std::vector<std::vector<double>> fixed_params;
     std::vector<mi::PairDev> host;  // host mirror of the device pair array
     mi::PairDev* d_pairs = nullptr;
-    mi::Chunk* d_chunks = nullptr;
+    mi::Work* d_work = nullptr;   // two lists
     int nchunks = 0;
+    unsigned int seg_max = 0;     // samples a histogram CTA may add before it flushes
     double* d_partials = nullptr;
     size_t partials_cap = 0;      // doubles
     unsigned int* d_active = nullptr;
@@ -208,9 +394,11 @@ struct mi_batch {
 namespace mi {
 namespace {
 
-size_t batch_hist_smem(int B, int copies, int fine) {
+// The copies alone, by which their number is chosen, and with the column sums after them.
+size_t batch_hist_copies(int B, int copies, int fine) {
     return ((size_t)copies * hist_copy_stride(B) + (size_t)fine * hist_fine_stride(B)) * sizeof(unsigned int);
 }
+size_t batch_hist_smem(int B, int copies, int fine) { return hist_region_bytes(B, copies, fine); }
 
 void release_graph(mi_batch* b) {
     if (b->exec) cudaGraphExecDestroy(b->exec);
@@ -226,17 +414,18 @@ mi_status shape_batch(mi_batch* b, int chunk, int copies) {
     mi_context* ctx = b->ctx;
     const int B = b->bins;
     int fine = std::max(1, copies / 2);
-    while (fine > 1 && batch_hist_smem(B, copies, fine) > 52 * 1024) fine >>= 1;
-    if (batch_hist_smem(B, copies, fine) > 200 * 1024)
+    while (fine > 1 && batch_hist_copies(B, copies, fine) > 52 * 1024) fine >>= 1;
+    if (batch_hist_copies(B, copies, fine) > 200 * 1024)
         return set_error(ctx, MI_ERR_INVALID_ARGUMENT, "histogram copies do not fit in shared memory");
-    std::vector<Chunk> chunks;
+    int nchunks = 0, per_thread_max = 1 << 20;
+    int64_t total = 0;
     size_t poff = 0;
     for (int p = 0; p < b->npairs; ++p) {
         mi_metric* m = b->metrics[p];
         const uint32_t n = (uint32_t)m->n_samples;
         const int nc = std::max<int>(1, (int)((n + chunk - 1) / chunk));
-        for (int c = 0; c < nc; ++c)
-            chunks.push_back(Chunk{p, c, (uint32_t)c * (uint32_t)chunk, std::min<uint32_t>(n, (uint32_t)(c + 1) * chunk)});
+        nchunks += nc;
+        total += n;
         PairDev& pd = b->host[p];
         pd.nchunks = nc;
         pd.a.partials = b->d_partials + poff;
@@ -253,6 +442,16 @@ mi_status shape_batch(mi_batch* b, int chunk, int copies) {
         while (kf > k && (std::ldexp(1.0, kf - FINE_T) * fine_max + fine_max >= lim ||
                           std::ldexp(1.0, kf) * (double)(m->n_samples + 1) >= 0x1p63))
             --kf;
+        // the most samples a thread may add with these units (any n or chunk: the pair's own
+        // number fits)
+        int most = (int)per_thread;
+        while (most < (1 << 20) &&
+               std::ldexp(1.0, k) * (2.0 / 3.0) * (double)(most + 1) * (HIST_BLOCK / copies) +
+                       (double)(most + 1) * (HIST_BLOCK / copies) < lim &&
+               std::ldexp(1.0, kf - FINE_T) * (double)(most + 1) * (HIST_BLOCK / fine) +
+                       (double)(most + 1) * (HIST_BLOCK / fine) < lim)
+            ++most;
+        per_thread_max = std::min(per_thread_max, most);
         pd.a.hist_scale = (float)std::ldexp(1.0, k);
         pd.a.fine_scale = (float)std::ldexp(1.0, kf);
         pd.a.fine_shift = kf - k;
@@ -261,52 +460,54 @@ mi_status shape_batch(mi_batch* b, int chunk, int copies) {
         pd.a.fine_copies = fine;
     }
     if (poff > b->partials_cap) return set_error(ctx, MI_ERR_INVALID_ARGUMENT, "batch chunk shape too fine");
-    dev_free(ctx, b->d_chunks);
-    b->d_chunks = nullptr;
-    MI_CHECK_CUDA(ctx, dev_alloc(ctx, &b->d_chunks, chunks.size() * sizeof(Chunk)));
-    MI_CHECK_CUDA(ctx, cudaMemcpyAsync(b->d_chunks, chunks.data(), chunks.size() * sizeof(Chunk), cudaMemcpyHostToDevice,
-                                       ctx->stream));
-    b->nchunks = (int)chunks.size();
+    b->nchunks = nchunks;
+    b->seg_max = (unsigned int)per_thread_max * HIST_BLOCK;
     b->chunk = chunk;
     b->copies = copies;
     b->fine_copies = fine;
-    const size_t hs = batch_hist_smem(B, copies, fine), ds = deriv_smem(B);
+    const size_t hs = batch_hist_smem(B, copies, fine), ds = stream_smem(B);
     // raise-only limits: another batch with fewer bins must not lower them under this one
     {
         mi_status ls = raise_smem_limit(ctx, (const void*)k_batch_hist, hs);
-        if (ls == MI_OK) ls = raise_smem_limit(ctx, (const void*)k_batch_deriv, ds);
+        if (ls == MI_OK) ls = raise_smem_limit(ctx, (const void*)k_batch_deriv<true>, ds);
+        if (ls == MI_OK) ls = raise_smem_limit(ctx, (const void*)k_batch_deriv<false>, ds);
         if (ls != MI_OK) return ls;
     }
     int occ_h = 0, occ_d = 0;
     MI_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_h, k_batch_hist, HIST_BLOCK, hs));
-    MI_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k_batch_deriv, DERIV_BLOCK, ds));
-    b->grid_hist = std::max(1, std::min(b->nchunks, ctx->num_sms * std::max(occ_h, 1)));
+    MI_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k_batch_deriv<true>, DERIV_BLOCK, ds));
+    b->grid_hist = (int)std::max<int64_t>(1, std::min<int64_t>((total + LEAST_SHARE - 1) / LEAST_SHARE + b->npairs,
+                                                               ctx->num_sms * std::max(occ_h, 1)));
     b->grid_deriv = std::max(1, std::min(b->nchunks, ctx->num_sms * std::max(occ_d, 1)));
-    if ((size_t)b->grid_hist * chunk > b->exq_len) {
+    if (MI_EXACT_DEFERRED && (size_t)b->grid_hist * b->seg_max > b->exq_len) {
         dev_free(ctx, b->d_exq);
         b->d_exq = nullptr;
         b->exq_len = 0;
-        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &b->d_exq, (size_t)b->grid_hist * chunk * sizeof(uint32_t)));
-        b->exq_len = (size_t)b->grid_hist * chunk;
+        MI_CHECK_CUDA(ctx, dev_alloc(ctx, &b->d_exq, (size_t)b->grid_hist * b->seg_max * sizeof(uint32_t)));
+        b->exq_len = (size_t)b->grid_hist * b->seg_max;
     }
     release_graph(b);
     return MI_OK;
 }
 
 mi_status upload_pairs(mi_batch* b) {
+    std::vector<Work> work(b->npairs);
+    for (int p = 0; p < b->npairs; ++p)
+        work[p] = Work{((unsigned int)b->metrics[p]->n_samples + UNIT - 1) / UNIT * UNIT, (unsigned int)b->host[p].nchunks};
     MI_CHECK_CUDA(b->ctx, cudaMemcpyAsync(b->d_pairs, b->host.data(), b->host.size() * sizeof(PairDev),
                                           cudaMemcpyHostToDevice, b->ctx->stream));
+    MI_CHECK_CUDA(b->ctx, cudaMemcpyAsync(b->d_work, work.data(), work.size() * sizeof(Work), cudaMemcpyHostToDevice,
+                                          b->ctx->stream));
     return MI_OK;
 }
 
 mi_status launch_pass(mi_batch* b, const mi_rsgd_config& cfg, bool update) {
     cudaStream_t st = b->ctx->stream;
     const int B = b->bins;
-    k_batch_hist<<<b->grid_hist, HIST_BLOCK, batch_hist_smem(B, b->copies, b->fine_copies), st>>>(
-        b->d_pairs, b->d_chunks, b->nchunks, b->d_exq, (uint32_t)b->chunk);
-    k_batch_deriv<<<b->grid_deriv, DERIV_BLOCK, deriv_smem(B), st>>>(b->d_pairs, b->d_chunks, b->nchunks);
-    if (update) k_batch_update<<<(b->npairs + 63) / 64, 64, 0, st>>>(b->d_pairs, b->npairs, cfg, b->d_active);
-    MI_CHECK_CUDA(b->ctx, cudaGetLastError());
+    MI_CHECK_CUDA(b->ctx, pdl::launch(k_batch_hist, b->grid_hist, HIST_BLOCK, batch_hist_smem(B, b->copies, b->fine_copies), st,
+                                      b->d_pairs, b->d_work, b->npairs, b->seg_max, b->d_exq));
+    MI_CHECK_CUDA(b->ctx, pdl::launch(update ? k_batch_deriv<true> : k_batch_deriv<false>, b->grid_deriv, DERIV_BLOCK,
+                                      stream_smem(B), st, b->d_pairs, b->d_work, b->npairs, (unsigned int)b->chunk, cfg, b->d_active));
     return MI_OK;
 }
 
@@ -360,10 +561,10 @@ mi_status autotune(mi_batch* b, const mi_rsgd_config& cfg, const double* params)
     float best = 1e30f;
     int best_chunk = 4096, best_copies = 4;
     mi_status st = MI_OK;
-    const size_t coarse_cap = std::max<size_t>(48 * 1024, batch_hist_smem(b->bins, hist_copies(b->bins), 0));
+    const size_t coarse_cap = std::max<size_t>(48 * 1024, batch_hist_copies(b->bins, hist_copies(b->bins), 0));
     for (int ch : chunks) {
         for (int cp : copies_c) {
-            if (batch_hist_smem(b->bins, cp, 0) > coarse_cap) continue;
+            if (batch_hist_copies(b->bins, cp, 0) > coarse_cap) continue;
             if ((st = shape_batch(b, ch, cp)) != MI_OK) break;
             if ((st = seed_pairs(b, cfg, params)) != MI_OK) break;
             if ((st = launch_pass(b, cfg, false)) != MI_OK) break;  // warm-up
@@ -437,7 +638,7 @@ void free_batch(mi_batch* b) {
     cudaStreamSynchronize(ctx->stream);
     release_graph(b);
     dev_free(ctx, b->d_pairs);
-    dev_free(ctx, b->d_chunks);
+    dev_free(ctx, b->d_work);
     dev_free(ctx, b->d_partials);
     dev_free(ctx, b->d_active);
     dev_free(ctx, b->d_marks);
@@ -512,6 +713,8 @@ mi_status mi_batch_create(mi_context* ctx, int npairs, const mi_image* const* fi
         a.n = (uint32_t)m->n_samples;
         a.npad = (a.n + 3u) & ~3u;
         a.ghist = m->ws.hist;
+        a.gcols = m->ws.hist + (size_t)bins * bins + bins;
+        a.reps = 1;
         a.rec_bins = m->ws.rec_bins;
         a.rec_f = m->ws.rec_f;
         a.rec_g = m->ws.rec_g;
@@ -522,6 +725,7 @@ mi_status mi_batch_create(mi_context* ctx, int npairs, const mi_image* const* fi
     }
     if (s == MI_OK) {
         cudaError_t e = dev_alloc(ctx, &b->d_pairs, (size_t)npairs * sizeof(PairDev));
+        if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_work, (size_t)2 * npairs * sizeof(Work));
         if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_partials, max_chunks * NMOM * sizeof(double));
         if (e == cudaSuccess) e = dev_alloc(ctx, &b->d_active, sizeof(unsigned int));
         if (e == cudaSuccess) e = pinned_alloc(ctx, reinterpret_cast<void**>(&b->h_active), nullptr);

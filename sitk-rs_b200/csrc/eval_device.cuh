@@ -507,15 +507,26 @@ __device__ __forceinline__ void hist_phase(const SamplerParams& P, const EvalArg
         cl.sync();  // no CTA leaves while another still reads its shared memory
         return;
     }
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) {
-        unsigned long long v = 0ull;
-        for (int c = 0; c < copies; ++c) v += sh[c * cstride + i];
-        if (i < B * B) {
-            unsigned long long f = 0ull;
+    // A thread adds the rows f ≡ g of one column m, so that a column's sum leaves it once: a
+    // 64-bit add to shared memory is a compare-and-swap loop, and one per bin (2,500 at 50
+    // bins, ten threads a column at a time) held the flush back.
+    const int groups = max(1, (int)blockDim.x / B);
+    for (int e = threadIdx.x; e < groups * B; e += blockDim.x) {
+        const int m = e % B;
+        unsigned long long col = 0ull;
+        for (int i = e; i < B * B; i += groups * B) {
+            unsigned long long v = 0ull, f = 0ull;
+            for (int c = 0; c < copies; ++c) v += sh[c * cstride + i];
             for (int c = 0; c < fine_copies; ++c) f += sh_fine[c * fstride + i];
             v = (v << a.fine_shift) + f;
-            if (a.gcols && v) atomicAdd(&colacc[i % B], v);
+            col += v;
+            if (v) atomicAdd(&rep_hist[i], v);
         }
+        if (a.gcols && col) atomicAdd(&colacc[m], col);
+    }
+    for (int i = B * B + threadIdx.x; i < nb; i += blockDim.x) {
+        unsigned long long v = 0ull;
+        for (int c = 0; c < copies; ++c) v += sh[c * cstride + i];
         if (v) atomicAdd(&rep_hist[i], v);
     }
     if (a.gcols) {
@@ -1097,11 +1108,16 @@ __host__ __device__ inline size_t stream_smem(int B) {
     return 32 * (size_t)NMOM * sizeof(double) + (size_t)B * B * sizeof(float) + (size_t)2 * B * 8;
 }
 
-// Returns the tail state (for the last CTA's fold).
-template <class Src = GridRecords>
-__device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, double* dsh, const GroupWork w) {
+// Its first part: the table, margins and counts in dsh, the tail state returned, and the
+// first record group requested into `cur`.
+struct TableCtx {
+    TailCtx t;
+    unsigned long long jmin, fmin;  // the least passing joint count or column sum, and fixed count
+};
+template <class Src>
+__device__ __forceinline__ TableCtx stream_table(const SamplerParams& P, const EvalArgs& a, double* dsh, const GroupWork& w,
+                                                 typename Src::Group& cur) {
     const int B = P.bins, B2 = B * B;
-    double* red = dsh;
     float* pr = reinterpret_cast<float*>(dsh + 32 * NMOM);
     unsigned long long* col = reinterpret_cast<unsigned long long*>(pr + B2);
     unsigned long long* cnt = col + B;
@@ -1109,9 +1125,6 @@ __device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, doubl
     const int bd = (int)blockDim.x;
     const int wfirst = (int)threadIdx.x - lane;
     const int ns = value_slices(B);
-    float acc[NMOM];
-#pragma unroll
-    for (int i = 0; i < NMOM; ++i) acc[i] = 0.0f;
     const uint32_t q = w.begin + w.first;
     // one round of requests: the first R·bd bins (bin i0 + u·bd + lane for warp base
     // i0), the margins, the first record group
@@ -1129,7 +1142,6 @@ __device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, doubl
         col[i] = __ldcg(a.gcols + i);
         cnt[i] = __ldcg(a.ghist + B2 + i);
     }
-    typename Src::Group cur;
     if (q < w.end) Src::load(a, q, cur);
     __syncthreads();
     // The pRatio table needs the ε tests of the joint counts and the margins, not the
@@ -1167,11 +1179,32 @@ __device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, doubl
         }
     }
     __syncthreads();
-    if (!t.degenerate) Src::stream(P, a, pr, q, w.end, w.stride, cur, acc);
+    return TableCtx{t, jmin, fmin};
+}
+
+// Its second part, on the table that stream_table left in dsh: the moments of this CTA's
+// records and its value slices.
+template <class Src>
+__device__ __forceinline__ void stream_rows(const SamplerParams& P, const EvalArgs& a, double* dsh, const GroupWork& w,
+                                            const typename Src::Group& cur, const TableCtx& tab) {
+    const TailCtx& t = tab.t;
+    const int B = P.bins, B2 = B * B;
+    double* red = dsh;
+    const float* pr = reinterpret_cast<const float*>(dsh + 32 * NMOM);
+    const unsigned long long* col = reinterpret_cast<const unsigned long long*>(pr + B2);
+    const unsigned long long* cnt = col + B;
+    const int lane = threadIdx.x & 31;
+    const int bd = (int)blockDim.x;
+    const int ns = value_slices(B);
+    float acc[NMOM];
+#pragma unroll
+    for (int i = 0; i < NMOM; ++i) acc[i] = 0.0f;
+    if (!t.degenerate) Src::stream(P, a, pr, w.begin + w.first, w.end, w.stride, cur, acc);
     // the value slices that fall to this CTA (slices unit + units·(u + k·warps) to warp
     // u), each bin's term from the logarithms the other forms take (margin_terms,
     // value_term)
     if (!t.degenerate) {
+        const unsigned long long jmin = tab.jmin, fmin = tab.fmin;
         const int nwarp = bd >> 5;
         for (int sl = (int)(threadIdx.x >> 5) * (int)w.units + (int)w.unit; sl < ns;
              sl += nwarp * (int)w.units) {
@@ -1191,7 +1224,15 @@ __device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, doubl
         }
     }
     store_moments(acc, red, w.part, w.part_stride);
-    return t;
+}
+
+// Both. Returns the tail state (for the last CTA's fold).
+template <class Src = GridRecords>
+__device__ TailCtx stream_phase(const SamplerParams& P, const EvalArgs& a, double* dsh, const GroupWork w) {
+    typename Src::Group cur;
+    const TableCtx tab = stream_table<Src>(P, a, dsh, w, cur);
+    stream_rows<Src>(P, a, dsh, w, cur, tab);
+    return tab.t;
 }
 
 // Run by the last CTA to finish the derivative phase: fold the `count` partials of

@@ -45,15 +45,20 @@ MI_HD inline float f32_up(double x) {
     return f;
 }
 
-// P holds the metric's fixed part (grids, moving image, histogram geometry); this
-// fills the stage-dependent part. Returns false when the map is not finite.
-MI_HD inline bool point_map_fill(SamplerParams& P, const double* stages, int nstage) {
-    using rsgd::add;
-    using rsgd::mul;
-    using rsgd::sub;
+// P holds the metric's fixed part (grids, moving image, histogram geometry);
+// point_map_fill fills the stage-dependent part in three: the composite map, the
+// magnitude bound (per corner, so a device caller can spread them), and what follows
+// from it.
+MI_HD inline void pm_stages(SamplerParams& P, const double* stages, int nstage) {
     P.nstage = nstage;
     for (int s = 0; s < nstage; ++s)
         for (int i = 0; i < 12; ++i) P.stage[s][i] = stages[s * 12 + i];
+}
+
+MI_HD inline void pm_compose(SamplerParams& P) {
+    using rsgd::add;
+    using rsgd::sub;
+    const int nstage = P.nstage;
     // T(x) = MT·x + tT, the stages folded (for the fast path only; the exact chain
     // replays them one by one)
     double MT[9] = {1, 0, 0, 0, 1, 0, 0, 0, 1}, tT[3] = {0, 0, 0};
@@ -74,33 +79,46 @@ MI_HD inline bool point_map_fill(SamplerParams& P, const double* stages, int nst
     pm_mat3_vec(P.mp2i, tmp, b);
     for (int i = 0; i < 9; ++i) P.cA[i] = A[i];
     for (int d = 0; d < 3; ++d) P.cb[d] = b[d];
-    // Magnitude bound of every intermediate of the exact chain, in moving voxels,
-    // over the fixed grid's corners; the chain's rounding is ≲ 20·2^-53 of it and
-    // cerr allows 2^-40 (≈ 400× margin).
+}
+
+// Magnitude bound of every intermediate of the exact chain, in moving voxels, at a corner
+// of the fixed grid; the chain's rounding is ≲ 20·2^-53 of the largest and cerr allows
+// 2^-40 (≈ 400× margin).
+MI_HD inline double pm_corner(const SamplerParams& P, int corner) {
+    using rsgd::add;
+    using rsgd::mul;
+    const int nstage = P.nstage;
     double cmax = 0.0;
-    for (int corner = 0; corner < 8; ++corner) {
-        const double idx[3] = {(corner & 1) ? (double)(P.fsize0 - 1) : 0.0, (corner & 2) ? (double)(P.fsize1 - 1) : 0.0,
-                               (corner & 4) ? (double)(P.fsize2 - 1) : 0.0};
-        double mag[3];
+    const double idx[3] = {(corner & 1) ? (double)(P.fsize0 - 1) : 0.0, (corner & 2) ? (double)(P.fsize1 - 1) : 0.0,
+                           (corner & 4) ? (double)(P.fsize2 - 1) : 0.0};
+    double mag[3];
+    for (int r = 0; r < 3; ++r)
+        mag[r] = add(add(add(fabs(P.forigin[r]), mul(fabs(P.fi2p[r * 3]), idx[0])), mul(fabs(P.fi2p[r * 3 + 1]), idx[1])),
+                     mul(fabs(P.fi2p[r * 3 + 2]), idx[2]));
+    for (int s = 0; s < nstage; ++s) {
+        const double* S = P.stage[s];
+        double nmag[3];
         for (int r = 0; r < 3; ++r)
-            mag[r] = add(add(add(fabs(P.forigin[r]), mul(fabs(P.fi2p[r * 3]), idx[0])), mul(fabs(P.fi2p[r * 3 + 1]), idx[1])),
-                         mul(fabs(P.fi2p[r * 3 + 2]), idx[2]));
-        for (int s = 0; s < nstage; ++s) {
-            const double* S = P.stage[s];
-            double nmag[3];
-            for (int r = 0; r < 3; ++r)
-                nmag[r] = add(add(add(mul(fabs(S[r * 3]), mag[0]), mul(fabs(S[r * 3 + 1]), mag[1])),
-                                  mul(fabs(S[r * 3 + 2]), mag[2])),
-                              fabs(S[9 + r]));
-            for (int r = 0; r < 3; ++r) mag[r] = nmag[r];
-        }
-        for (int r = 0; r < 3; ++r) mag[r] = add(mag[r], fabs(P.morigin[r]));
-        for (int r = 0; r < 3; ++r) {
-            const double cm = add(add(mul(fabs(P.mp2i[r * 3]), mag[0]), mul(fabs(P.mp2i[r * 3 + 1]), mag[1])),
-                                  mul(fabs(P.mp2i[r * 3 + 2]), mag[2]));
-            cmax = fmax(cmax, cm);
-        }
+            nmag[r] = add(add(add(mul(fabs(S[r * 3]), mag[0]), mul(fabs(S[r * 3 + 1]), mag[1])),
+                              mul(fabs(S[r * 3 + 2]), mag[2])),
+                          fabs(S[9 + r]));
+        for (int r = 0; r < 3; ++r) mag[r] = nmag[r];
     }
+    for (int r = 0; r < 3; ++r) mag[r] = add(mag[r], fabs(P.morigin[r]));
+    for (int r = 0; r < 3; ++r) {
+        const double cm = add(add(mul(fabs(P.mp2i[r * 3]), mag[0]), mul(fabs(P.mp2i[r * 3 + 1]), mag[1])),
+                              mul(fabs(P.mp2i[r * 3 + 2]), mag[2]));
+        cmax = fmax(cmax, cm);
+    }
+    return cmax;
+}
+
+// Returns false when the map is not finite.
+MI_HD inline bool pm_bounds(SamplerParams& P, double cmax) {
+    using rsgd::add;
+    using rsgd::mul;
+    using rsgd::sub;
+    const int nstage = P.nstage;
     if (!(cmax <= DBL_MAX)) return false;
     P.cerr = mul(mul(0x1p-40, add(1.0, cmax)), (double)(1 + nstage));
     {
@@ -152,6 +170,14 @@ MI_HD inline bool point_map_fill(SamplerParams& P, const double* stages, int nst
     }
     P.bin_hi = (double)(P.bins - 3);  // bins − PADDING − 1
     return true;
+}
+
+MI_HD inline bool point_map_fill(SamplerParams& P, const double* stages, int nstage) {
+    pm_stages(P, stages, nstage);
+    pm_compose(P);
+    double cmax = 0.0;
+    for (int corner = 0; corner < 8; ++corner) cmax = fmax(cmax, pm_corner(P, corner));
+    return pm_bounds(P, cmax);
 }
 
 }  // namespace mi

@@ -163,13 +163,10 @@ MI_HD inline void start(State& s, const mi_rsgd_config& cfg, int P) {
     s.lr_pending = cfg.estimate_learning_rate ? 1 : 0;
 }
 
-// One decision after an evaluation (optimizer.rs:383-440): with the derivative at p,
+// One decision after an evaluation (optimizer.rs:383-440): with the scaled derivative at p,
 // either stop (returns true, s.stop set) or step p in place (returns false).
-MI_HD inline bool after_evaluation(State& s, const mi_rsgd_config& cfg, const Corners& c, const double* scales,
-                                   const double* grad, double* p) {
+MI_HD inline bool after_scaled(State& s, const mi_rsgd_config& cfg, const Corners& c, const double* scaled, double* p) {
     const int n = c.P;
-    double scaled[MI_MAX_PARAMS];
-    for (int k = 0; k < n; ++k) scaled[k] = div(grad[k], scales[k]);
     if (s.lr_pending) {
         // method.rs: EstimateLearningRate::Once — lr = est(g0/scales)·|g0/scales|
         double sq = 0.0;
@@ -201,6 +198,13 @@ MI_HD inline bool after_evaluation(State& s, const mi_rsgd_config& cfg, const Co
     for (int k = 0; k < n; ++k) s.prev[k] = scaled[k];
     s.taken += 1;
     return false;
+}
+// The same with the derivative at p.
+MI_HD inline bool after_evaluation(State& s, const mi_rsgd_config& cfg, const Corners& c, const double* scales,
+                                   const double* grad, double* p) {
+    double scaled[MI_MAX_PARAMS];
+    for (int k = 0; k < c.P; ++k) scaled[k] = div(grad[k], scales[k]);
+    return after_scaled(s, cfg, c, scaled, p);
 }
 
 }  // namespace rsgd
