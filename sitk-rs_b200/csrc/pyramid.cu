@@ -138,7 +138,8 @@ struct Recursion {
 // sample sums, and the shared-memory rows are numbered by step, so that a block's
 // accesses are constant offsets from one address. The volume stays FP64 between axes and
 // is f32 on both ends: the first pass widens as it reads, the last narrows as it writes.
-// 251×256×243: 108, 120 and 113 µs for the three axes; one line per thread with the
+// 251×256×243: 108 µs for the x axis (y and z, 120 and 113 µs, are k_gauss_segments' now: 106
+// and 84 µs); one line per thread with the
 // partial results in global memory took 285 µs an axis, and widening and narrowing
 // passes of their own another 58 µs.
 constexpr int GL = 16;       // lines a warp
@@ -311,6 +312,157 @@ __global__ void __launch_bounds__(32) k_gauss_rows(const TI* __restrict__ in, TO
     }
 }
 
+// Axes 1 and 2 of volumes with many lines: a lane walks a whole line, and neither pass leaves
+// its results anywhere. The causal pass runs once up to the last segment and keeps its four
+// v before every segment of 16; then, segment by segment from the far end, it is run
+// again from there into registers and the anti-causal pass follows over the same samples.
+// Half as many FP64 operations again as k_gauss_strided (45 an element, whose pipe is 40–50 %
+// busy; 22 % there), but 4 doubles of shared memory a line and segment of 16 instead of
+// 16, and coefficients from the constant bank: fourteen warps of 32 lines an SM at n = 256
+// for seven of 16. Samples are requested a segment ahead, as the steps free the registers
+// of the last. n ≥ 20.
+constexpr int SEG = 16;
+constexpr int SEG_LAST = 20;  // the last segment holds 4 + (n − 4) mod 16 elements, so that the
+                              // anti-causal border lies inside it
+
+__host__ __device__ inline int segments(int64_t n) { return (int)((n - 4) / SEG) + 1; }
+
+// A pass's state; its coefficients stay in the constant bank.
+struct Walk {
+    double w1, w2, w3, q1, q2, q3, q4;
+};
+// One step (Recursion::step) with coefficients c, denominators d; BORDER below 4: the v before
+// the border enter as e·b.
+template <int BORDER>
+__device__ __forceinline__ double walk(Walk& s, double x, const double* c, const double* d, const double* b, double e) {
+    const double a = dot4(x, c[0], s.w1, c[1], s.w2, c[2], s.w3, c[3]);
+    const double r = dot4(BORDER >= 1 ? s.q1 : e, BORDER >= 1 ? d[0] : b[0], BORDER >= 2 ? s.q2 : e, BORDER >= 2 ? d[1] : b[1],
+                          BORDER >= 3 ? s.q3 : e, BORDER >= 3 ? d[2] : b[2], BORDER >= 4 ? s.q4 : e, BORDER >= 4 ? d[3] : b[3]);
+    const double v = __dsub_rn(a, r);
+    s.w3 = s.w2;
+    s.w2 = s.w1;
+    s.w1 = x;
+    s.q4 = s.q3;
+    s.q3 = s.q2;
+    s.q2 = s.q1;
+    s.q1 = v;
+    return v;
+}
+// The step at the fixed distance `u` from the border, unrolled.
+__device__ __forceinline__ double walk_at(int u, Walk& s, double x, const double* c, const double* d, const double* b,
+                                          double e) {
+    return u == 0 ? walk<0>(s, x, c, d, b, e)
+                  : (u == 1 ? walk<1>(s, x, c, d, b, e)
+                            : (u == 2 ? walk<2>(s, x, c, d, b, e)
+                                      : (u == 3 ? walk<3>(s, x, c, d, b, e) : walk<4>(s, x, c, d, b, e))));
+}
+
+template <typename TI, typename TO>
+__global__ void __launch_bounds__(32, 14) k_gauss_segments(const TI* __restrict__ in, TO* __restrict__ out, int64_t nlines,
+                                                           int n, int64_t stride, int64_t na, int64_t sb,
+                                                           const __grid_constant__ Deriche C) {
+    extern __shared__ double kept[];  // the causal v before segment k, row 4(k − 1) + l
+    const double *cc = C.c, *cd = C.c + 4, *cb = C.c + 12, *ac = C.c + 8, *ab = C.c + 16;
+    const int lane = threadIdx.x;
+    const int64_t L = min((int64_t)blockIdx.x * 32 + lane, nlines - 1);
+    const int64_t first = (L % na) + (L / na) * sb;
+    const TI* __restrict__ from = in + first;
+    TO* __restrict__ to = out + first;
+    const int nseg = segments(n), last = (nseg - 1) * SEG, count = n - last;  // count in [4, 19]
+    const double e = (double)from[0];
+    // the causal pass up to the last segment
+    Walk f{e, e, e, 0.0, 0.0, 0.0, 0.0};
+    {
+        // each sample is replaced by the next segment's as it is used
+        const TI* p = from;
+        const int64_t ahead = SEG * stride;
+        TI x[SEG];
+#pragma unroll
+        for (int u = 0; u < SEG; ++u) x[u] = p[u * stride];
+        for (int k = 0; k < nseg - 1; ++k, p += ahead) {
+            const bool more = k + 2 < nseg;
+            const TI* q = more ? p + ahead : p;
+            if (k == 0) {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) walk_at(u, f, (double)x[u], cc, cd, cb, e);
+            } else {
+#pragma unroll
+                for (int u = 0; u < 4; ++u) walk<4>(f, (double)x[u], cc, cd, cb, e);
+            }
+#pragma unroll
+            for (int u = 0; u < 4; ++u) x[u] = q[u * stride];
+#pragma unroll
+            for (int u = 4; u < SEG; ++u) {
+                walk<4>(f, (double)x[u], cc, cd, cb, e);
+                x[u] = q[u * stride];
+            }
+            double* row = kept + k * 128 + lane;
+            row[0] = f.q1;
+            row[32] = f.q2;
+            row[64] = f.q3;
+            row[96] = f.q4;
+        }
+    }
+    // the next segment's samples and the three before them, requested one by one as the
+    // anti-causal steps free the registers of the last ones
+    TI x[SEG], w[3];
+    auto request = [&](int k, int u) {
+        if (k < 0) return;
+        const TI* p = from + (int64_t)(k * SEG) * stride;
+        x[u] = p[u * stride];
+        if (u < 3) w[u] = p[k > 0 ? -(u + 1) * stride : 0];
+    };
+    const double z = (double)from[(int64_t)(n - 1) * stride];
+    Walk g{z, z, z, 0.0, 0.0, 0.0, 0.0};
+    double after;  // the sample after the segment
+    {
+        // the last segment, at the end of SEG_LAST places; f stands before it
+        double t[SEG_LAST], v[SEG_LAST];
+        const int skip = SEG_LAST - count;
+#pragma unroll
+        for (int u = 0; u < SEG_LAST; ++u) t[u] = (double)from[(int64_t)max(n - SEG_LAST + u, 0) * stride];
+#pragma unroll
+        for (int u = 0; u < SEG_LAST; ++u) {
+            if (u < skip) continue;
+            v[u] = walk<4>(f, t[u], cc, cd, cb, e);
+        }
+#pragma unroll
+        for (int u = SEG_LAST - 1; u >= 0; --u) {
+            if (u < skip) continue;
+            const double y = walk_at(SEG_LAST - 1 - u, g, u + 1 < SEG_LAST ? t[u + 1 < SEG_LAST ? u + 1 : u] : z, ac, cd, ab, z);
+            to[(int64_t)(n - SEG_LAST + u) * stride] = (TO)__dadd_rn(v[u], y);
+        }
+        after = (double)from[(int64_t)last * stride];
+#pragma unroll
+        for (int u = 0; u < SEG; ++u) request(nseg - 2, u);
+    }
+    for (int k = nseg - 2; k >= 0; --k) {
+        double t[SEG], v[SEG];
+#pragma unroll
+        for (int u = 0; u < SEG; ++u) t[u] = (double)x[u];
+        if (k > 0) {
+            const double* row = kept + (k - 1) * 128 + lane;
+            f = Walk{(double)w[0], (double)w[1], (double)w[2], row[0], row[32], row[64], row[96]};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = walk<4>(f, t[u], cc, cd, cb, e);
+        } else {
+            f = Walk{e, e, e, 0.0, 0.0, 0.0, 0.0};
+#pragma unroll
+            for (int u = 0; u < 4; ++u) v[u] = walk_at(u, f, t[u], cc, cd, cb, e);
+        }
+#pragma unroll
+        for (int u = 4; u < SEG; ++u) v[u] = walk<4>(f, t[u], cc, cd, cb, e);
+        TO* p = to + (int64_t)(k * SEG) * stride;
+#pragma unroll
+        for (int u = SEG - 1; u >= 0; --u) {
+            const double y = walk<4>(g, u + 1 < SEG ? t[u + 1 < SEG ? u + 1 : u] : after, ac, cd, ab, z);
+            p[u * stride] = (TO)__dadd_rn(v[u], y);
+            request(k - 1, SEG - 1 - u);
+        }
+        after = t[0];
+    }
+}
+
 // Lines too long for a warp's partial results in shared memory: one line per thread, the
 // causal pass left in `mid` (FP64) and read back by the anti-causal one.
 template <typename TI, typename TO>
@@ -448,6 +600,15 @@ bool long_line(mi_context* ctx, int axis, int64_t n, size_t esize) {
     return gauss_smem(axis, n, esize) > (size_t)optin || n > (1 << 20);
 }
 
+// Which of the two strided kernels takes an axis: with `fit` warps of k_gauss_strided on an
+// SM and `warps` in all. Its lines' partial results leave room for seven warps or fewer
+// from n = 220 on, and with more than two rounds of them k_gauss_segments' half as many
+// FP64 operations more cost less than the idle pipe: 83–86 against 62–66 µs at 224³,
+// 122–125 against 95 at 256³, 260–265 against 183–191 at 320³, 216 against 113 at
+// 512×512×64 (y). With eight warps or two rounds it is the other way round: 37–38 against
+// 41–44 µs at 192³, 72 against 91 at 512×512×64 (z), 22 against 40 at 256×256×40 (y).
+bool many_lines(int fit, int64_t warps, int sms) { return fit <= 7 && warps > (int64_t)2 * fit * sms; }
+
 // One axis of one volume. `mid`: FP64 scratch for long lines.
 template <typename TI, typename TO>
 mi_status gauss_axis(mi_context* ctx, const TI* in, double* mid, TO* out, const int64_t* sz, int axis, const Deriche& C) {
@@ -468,8 +629,18 @@ mi_status gauss_axis(mi_context* ctx, const TI* in, double* mid, TO* out, const 
         }
     } else {
         const size_t sm = gauss_smem(axis, n, sizeof(TI));
-        const mi_status s = mi::raise_smem_limit(ctx, (const void*)k_gauss_strided<TI, TO>, sm);
+        mi_status s = mi::raise_smem_limit(ctx, (const void*)k_gauss_strided<TI, TO>, sm);
         if (s != MI_OK) return s;
+        int fit = 0;
+        MI_CHECK_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&fit, k_gauss_strided<TI, TO>, 32, sm));
+        if (many_lines(fit, ctas, ctx->num_sms)) {
+            const size_t kept = (size_t)(segments(n) - 1) * 4 * 32 * 8;
+            s = mi::raise_smem_limit(ctx, (const void*)k_gauss_segments<TI, TO>, kept);
+            if (s != MI_OK) return s;
+            k_gauss_segments<TI, TO><<<(unsigned)((nlines + 31) / 32), 32, kept, st>>>(in, out, nlines, (int)n, stride, na, sb, C);
+            MI_CHECK_CUDA(ctx, cudaGetLastError());
+            return MI_OK;
+        }
         k_gauss_strided<TI, TO><<<(unsigned)ctas, 32, sm, st>>>(in, out, nlines, (int)n, stride, na, sb, C);
     }
     MI_CHECK_CUDA(ctx, cudaGetLastError());
