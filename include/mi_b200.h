@@ -416,7 +416,7 @@ mi_status mi_pyramid_level(mi_context* ctx, const mi_image* fixed, const mi_imag
 /* ---- batched registration (no reference counterpart) ----------------------- */
 
 /* Many registrations of uneven image sizes advanced together: every optimizer
- * iteration is one pass of three launches over all still-active pairs (histogram
+ * iteration is one pass of two launches over all still-active pairs (histogram
  * pass, tail and derivative pass, the regular-step gradient descent step of every
  * pair, with all optimizer state on the device), several passes captured in one CUDA
  * graph that is replayed until every pair has stopped. Per pair the sampler,

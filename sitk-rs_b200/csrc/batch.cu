@@ -220,8 +220,9 @@ struct StepShared {
 
 // The optimizer's decision on the evaluation just made, then the next point map, by the CTA
 // that finished the pair's derivative, on copies in shared memory: one thread decides, the
-// divisions and the point map's bound are spread (9.6 µs with all of it by one thread, 10–14 µs as a launch of its
-// own of one thread a pair). P is that CTA's copy of the pair's constants.
+// divisions and the point map's bound are spread (9.6 µs with all of it by one thread,
+// 10–14 µs as a launch of its own of one thread a pair). P is that CTA's copy of the
+// pair's constants.
 __device__ void step_pair(PairDev& pd, Work& work, SamplerParams& P, const mi_rsgd_config& cfg, unsigned int* active_count) {
     __shared__ StepShared s;
     const int np = pd.nparams;
