@@ -7,18 +7,19 @@
 //   warp 0  one lane requests A and B tiles of 64 k (128-byte rows, 128-byte swizzle) into
 //           a ring of shared-memory stages, as far ahead as the ring goes
 //   warp 1  one lane issues four tcgen05.mma per stage into one of two accumulators in
-//           tensor memory and commits the stage back to warp 0
+//           tensor memory and commits the stage back to warp 0 (MT = 2: eight, one accumulator)
 //   warps 2–5  read the other accumulator (tcgen05.ld, 32 rows a warp) and store 32 × 32
 //           blocks by TMA from shared memory, two in flight a warp
 // so copies, products and stores of neighbouring items overlap. Rows, columns and k past
 // the operands' ends arrive as zeros. Every element's products are accumulated in k
 // order, as in gemm_tc.cuh: same bits.
 //
-// Bound: a 128 × 256 tile does 2·128·256·64 operations for 48 KB brought in and 48 KB read
-// by the tensor core, so shared-memory bandwidth and the tensor pipe are close; the ring
-// (four stages) covers L2's latency. Narrow products (NT ≤ 64) are bound by the bytes of A.
-// 4096³: 133 µs a call (1,033 TFLOP/s, 0.65 of 1.59 PFLOP/s; four rounds of CTAs for 3.46
-// rounds of tiles); the one-stage kernel of gemm_tc.cuh took 1,489 µs. Products of few k are
+// Bound: a 128 × 256 tile brings 48 KB from L2 for 2·128·256·64 operations, so 148 CTAs ask it
+// for more than it gives (12 TB/s seen) before the tensor pipe is full; with MT = 2 a CTA
+// takes two blocks of 128 rows on one B tile, 64 KB for twice the operations, and one
+// accumulator (of 512 columns) instead of two. Narrow products (NT ≤ 64) are bound by the
+// bytes of A. 4096³: 109 µs a call with two blocks (1,263 TFLOP/s, 0.79 of 1.59 PFLOP/s), 118
+// with one; the one-stage kernel of gemm_tc.cuh took 1,489 µs. Products of few k are
 // bound by their output: 32,768 × 432 × 32 writes 57 MB in 18 µs by TMA stores, 32 µs when
 // the four warps turned the blocks in shared memory and stored rows themselves (290
 // instructions a block).
@@ -44,16 +45,18 @@ namespace tc {
 constexpr int TMA_THREADS = 192;
 constexpr unsigned int TMA_POLLS = 1u << 20;  // of mbarrier.try_wait, each suspending up to 2 µs
 
-template <int NT>
+// MT: blocks of 128 rows in a tile, one or two.
+template <int NT, int MT = 1>
 struct TmaShape {
-    static constexpr uint32_t A_BYTES = TILE_M * TILE_K * 2, B_BYTES = NT * TILE_K * 2;
+    static constexpr uint32_t A_BYTES = MT * TILE_M * TILE_K * 2, B_BYTES = NT * TILE_K * 2;
     static constexpr uint32_t STAGE = A_BYTES + B_BYTES;
     static constexpr uint32_t EPI = 4 * 2 * 32 * 32 * 4;  // four warps' 32 × 32 blocks, two each
     static constexpr int FIT = (int)((225 * 1024 - EPI) / STAGE);
     static constexpr int STAGES = FIT < 8 ? FIT : 8;
     static constexpr uint32_t BARS = STAGES * STAGE + EPI;
     static constexpr uint32_t SMEM = BARS + (2 * STAGES + 5) * 8 + 1024;  // and the alignment of the base
-    static constexpr uint32_t COLS = 2 * NT < 32 ? 32 : 2 * NT;           // two accumulators, a power of two
+    static constexpr int ACCS = MT == 1 ? 2 : 1;                          // accumulators of MT · NT columns
+    static constexpr uint32_t COLS = 2 * NT < 32 ? 32 : 2 * NT;           // all of them, a power of two
 };
 
 __device__ __forceinline__ void bar_init(uint32_t bar, uint32_t count) {
@@ -144,10 +147,10 @@ __device__ __forceinline__ void tma_store(const CUtensorMap* map, uint32_t src, 
 struct Item {
     int m0, n0, z, kt0, kt1;
 };
-template <int NT>
+template <int NT, int MT>
 __device__ __forceinline__ Item item_at(int item, int mt, int nt, int ktiles, int per) {
     Item w;
-    w.m0 = (item % mt) * TILE_M;
+    w.m0 = (item % mt) * (MT * TILE_M);
     w.n0 = (item / mt) % nt * NT;
     w.z = item / (mt * nt);
     w.kt0 = min(ktiles, w.z * per);
@@ -166,12 +169,14 @@ __device__ __forceinline__ void request_tile(uint32_t dst, const CUtensorMap* ma
     }
 }
 
-template <int NT, bool A_KROWS, bool B_KROWS>
+template <int NT, bool A_KROWS, bool B_KROWS, int MT = 1>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
 k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
            const __grid_constant__ CUtensorMap mapOut, int M, int N, int K, const Epilogue E, int splits, unsigned int* __restrict__ err) {
     static_assert(!B_KROWS || NT % 64 == 0, "k-rows tiles come in boxes of 64");
-    using S = TmaShape<NT>;
+    static_assert(MT == 1 || (!A_KROWS && 2 * NT <= 512), "two blocks of rows fill the tensor memory");
+    using S = TmaShape<NT, MT>;
+    constexpr uint32_t ACCS = S::ACCS;
     extern __shared__ uint8_t raw[];
     __shared__ uint32_t tmem_slot;
     __shared__ volatile int quit;
@@ -205,7 +210,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
     const uint32_t tmem = tmem_slot;
     pdl::wait_previous();
 
-    const int mt = (M + TILE_M - 1) / TILE_M, nt = (N + NT - 1) / NT;
+    const int mt = (M + MT * TILE_M - 1) / (MT * TILE_M), nt = (N + NT - 1) / NT;
     const int ktiles = (K + TILE_K - 1) / TILE_K, per = (ktiles + splits - 1) / splits;
     const int items = mt * nt * splits;
 
@@ -214,7 +219,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
             uint32_t count = 0;  // tiles requested
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const Item w = item_at<NT>(it, mt, nt, ktiles, per);
+                const Item w = item_at<NT, MT>(it, mt, nt, ktiles, per);
                 for (int kt = w.kt0; kt < w.kt1; ++kt, ++count) {
                     const uint32_t s = count % S::STAGES, round = count / S::STAGES;
                     if (!bar_wait(empty + s * 8, (round & 1) ^ 1, &quit)) {
@@ -224,6 +229,8 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                     const uint32_t dst = base + s * S::STAGE;
                     bar_expect(full + s * 8, S::STAGE);
                     request_tile<TILE_M, A_KROWS>(dst, &mapA, full + s * 8, kt * TILE_K, w.m0);
+                    if (MT == 2)
+                        request_tile<TILE_M, A_KROWS>(dst + TILE_M * TILE_K * 2, &mapA, full + s * 8, kt * TILE_K, w.m0 + TILE_M);
                     request_tile<NT, B_KROWS>(dst + S::A_BYTES, &mapB, full + s * 8, kt * TILE_K, w.n0);
                 }
             }
@@ -244,10 +251,10 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
             uint32_t count = 0, tiles = 0;
             bool ok = true;
             for (int it = blockIdx.x; it < items && ok; it += gridDim.x) {
-                const Item w = item_at<NT>(it, mt, nt, ktiles, per);
+                const Item w = item_at<NT, MT>(it, mt, nt, ktiles, per);
                 if (w.kt0 >= w.kt1) continue;  // an empty slice has no product
-                const uint32_t a = tiles & 1;
-                if (!bar_wait(tempty + a * 8, ((tiles >> 1) & 1) ^ 1, &quit)) break;
+                const uint32_t a = tiles % ACCS;
+                if (!bar_wait(tempty + a * 8, ((tiles / ACCS) & 1) ^ 1, &quit)) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 for (int kt = w.kt0; kt < w.kt1; ++kt, ++count) {
                     const uint32_t s = count % S::STAGES;
@@ -260,14 +267,15 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                     const uint64_t ad = A_KROWS ? swizzled_desc_mn(at) : swizzled_desc(at);
                     const uint64_t bd = B_KROWS ? swizzled_desc_mn(bt) : swizzled_desc(bt);
 #pragma unroll
-                    for (int q = 0; q < TILE_K / 16; ++q) {
+                    for (int qh = 0; qh < TILE_K / 16 * MT; ++qh) {
+                        const int q = qh / MT, h = qh % MT;  // both blocks of rows for each of B's 16 k
                         const uint32_t acc = (kt > w.kt0 || q > 0) ? 1u : 0u;
                         asm volatile(
                             "{\n\t.reg .pred p;\n\t"
                             "setp.ne.b32 p, %4, 0;\n\t"
                             "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t"
-                            "}" ::"r"(tmem + a * NT),
-                            "l"(ad + q * A_STEP), "l"(bd + q * B_STEP), "r"(idesc), "r"(acc));
+                            "}" ::"r"(tmem + (a * MT + h) * NT),
+                            "l"(ad + h * (TILE_M * TILE_K * 2 >> 4) + q * A_STEP), "l"(bd + q * B_STEP), "r"(idesc), "r"(acc));
                     }
                     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                                      empty + s * 8)
@@ -294,20 +302,20 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
         const int ldc = E.ldc;
         uint32_t tiles = 0, stored = 0;
         for (int it = blockIdx.x; it < items; it += gridDim.x) {
-            const Item w = item_at<NT>(it, mt, nt, ktiles, per);
+            const Item w = item_at<NT, MT>(it, mt, nt, ktiles, per);
             const bool any = w.kt0 < w.kt1;
-            const uint32_t a = tiles & 1;
+            const uint32_t a = tiles % ACCS;
             if (any) {
-                if (!__all_sync(0xffffffffu, bar_wait(tfull + a * 8, (tiles >> 1) & 1, &quit))) break;
+                if (!__all_sync(0xffffffffu, bar_wait(tfull + a * 8, (tiles / ACCS) & 1, &quit))) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             }
             constexpr int W = NT < 32 ? NT : 32;  // columns a block
-            const int row0 = w.m0 + quad * 32;
 #pragma unroll 1
-            for (int c0 = 0; c0 < NT; c0 += W) {
+            for (int ch = 0; ch < MT * NT; ch += W) {
+                const int c0 = ch % NT, row0 = w.m0 + (ch / NT) * TILE_M + quad * 32;
                 uint32_t r[W];
                 if (any) {
-                    const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + a * NT + c0;
+                    const uint32_t at = tmem + ((uint32_t)(quad * 32) << 16) + a * (MT * NT) + ch;
 #pragma unroll
                     for (int q = 0; q < W; q += 16)
                         asm volatile(
@@ -318,7 +326,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
                               "=r"(r[q + 11]), "=r"(r[q + 12]), "=r"(r[q + 13]), "=r"(r[q + 14]), "=r"(r[q + 15])
                             : "r"(at + q));
                     asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                    if (c0 + W >= NT) {  // the accumulator has been read
+                    if (ch + W >= MT * NT) {  // the accumulator has been read
                         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
                         if (lane == 0) bar_arrive(tempty + a * 8);
                     }

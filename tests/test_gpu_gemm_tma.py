@@ -66,3 +66,17 @@ def test_output_blocks_end_where_the_product_does(M, N, pitch, first):
     want[1:M + 1, first:first + N] = (A.double() @ B.double().T).float()  # integers below 2^24: exact
     _gemm(A, B, C[1:M + 1, first:first + N])
     assert torch.equal(C, want)
+
+
+@pytest.mark.parametrize("M,N,K,pad", [
+    (1300, 4100, 1032, 0),   # the last pair of row blocks: one full, one of 20 rows; a last column tile of 4
+    (2432, 3999, 1024, 8),   # a last pair without its second block; outputs by lanes
+    (4096, 2304, 2056, 0)])
+def test_two_row_blocks_a_tile(M, N, K, pad):
+    import torch
+    g = torch.Generator().manual_seed(M + N)
+    A = torch.randint(-3, 4, (M, K + pad), generator=g).to(torch.bfloat16).cuda()[:, :K]
+    B = torch.randint(-3, 4, (N, K + pad), generator=g).to(torch.bfloat16).cuda()[:, :K]
+    C = torch.full((M, N), -7.0, device="cuda")
+    _gemm(A, B, C)
+    assert torch.equal(C.double(), A.double() @ B.double().T)  # integers below 2^24: exact
