@@ -213,7 +213,8 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // layer, both channels of four taps, read from the FP32 input and rounded here. Bound by
 // the bytes written (34 and 28 MB in the two large layers for 64 pairs: 17 and 10.5 µs with
 // cold caches; 22.6 and 13.2 µs with 64-bit indices over all pairs). A CTA's rows are the
-// same in every pair, blockIdx.y.
+// same in every pair, blockIdx.y. The caller's input may start on any float: a voxel's two
+// channels are one load only where it starts on eight bytes.
 template <int D, int CIN, int KP, typename T>
 __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, __nv_bfloat16* __restrict__ col) {
     constexpr uint32_t Do = D / 2, PARTS = KP / 8, N = Do * Do * Do * PARTS;
@@ -232,6 +233,7 @@ __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, 
                      ? (zi * D + yi) * D + xi
                      : -1;
     }
+    const bool paired = CIN != 2 || (reinterpret_cast<uintptr_t>(x) & 7) == 0;
     for (int b = blockIdx.y; b < B; b += gridDim.y) {
         const T* in = x + (size_t)b * (D * D * D * CIN);
         uint4 v = make_uint4(0u, 0u, 0u, 0u);
@@ -239,7 +241,11 @@ __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, 
             uint32_t w[4];
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-                const float2 f = off[q] >= 0 ? __ldg(reinterpret_cast<const float2*>(in) + off[q]) : make_float2(0.f, 0.f);
+                float2 f = make_float2(0.f, 0.f);
+                if (off[q] >= 0) {
+                    const T* at = in + 2 * off[q];
+                    f = paired ? __ldg(reinterpret_cast<const float2*>(at)) : make_float2(__ldg(at), __ldg(at + 1));
+                }
                 w[q] = pack_bf16(f.x, f.y);
             }
             v = make_uint4(w[0], w[1], w[2], w[3]);
