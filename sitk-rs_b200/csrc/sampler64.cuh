@@ -114,7 +114,8 @@ __device__ __forceinline__ void load_corners(const SamplerParams& P, const float
 }
 
 // transform/interpolator.rs:103-152: the linear interpolant at the fractions of the cell
-// with corners v, and its gradient in index space
+// with corners v, and its gradient in index space. Infinite (or NaN) wherever a corner is, but
+// not always the infinity of the reference's weighted sum: see interpolate_weighted.
 template <bool GRAD>
 __device__ __forceinline__ double interpolate(const float* v, const double* fr, double* g) {
     const double v0 = v[0], v2 = v[2], v4 = v[4], v6 = v[6];
@@ -131,6 +132,27 @@ __device__ __forceinline__ double interpolate(const float* v, const double* fr, 
         g[2] = z;
     }
     return fma(fr[2], z, y0);
+}
+
+// The same as the reference forms it, corner by corner: what the interpolant is where a corner
+// is infinite (its differences from the others are NaN above). 130 FP64 operations for 22.
+template <bool GRAD>
+__device__ __forceinline__ double interpolate_weighted(const float* v, const double* fr, double* g) {
+    double val = 0.0, gi[3] = {0.0, 0.0, 0.0};
+#pragma unroll
+    for (int t = 0; t < 8; ++t) {
+        const double w0 = t & 1 ? fr[0] : 1.0 - fr[0], w1 = t & 2 ? fr[1] : 1.0 - fr[1], w2 = t & 4 ? fr[2] : 1.0 - fr[2];
+        const double b = (double)v[t];
+        val += w0 * w1 * w2 * b;
+        gi[0] += (t & 1 ? 1.0 : -1.0) * (w1 * w2) * b;
+        gi[1] += (t & 2 ? 1.0 : -1.0) * (w0 * w2) * b;
+        gi[2] += (t & 4 ? 1.0 : -1.0) * (w0 * w1) * b;
+    }
+    if (GRAD) {
+#pragma unroll
+        for (int d = 0; d < 3; ++d) g[d] = gi[d];
+    }
+    return val;
 }
 
 }  // namespace
