@@ -173,6 +173,22 @@ void dev_free(mi_context* ctx, void* p) {
     drop_blocks(ctx, LARGE_BYTES);
 }
 
+// Waits for the work of every stream as cudaFree of a cudaMalloc'd block does, which is allowed
+// while another thread captures a graph on another stream; cudaDeviceSynchronize then
+// fails and invalidates that capture (a batch in another thread lost its registration so).
+void wait_for_device(mi_context* ctx) {
+    void* word = nullptr;
+    cudaError_t e = cudaMalloc(&word, 1);
+    if (e == cudaErrorMemoryAllocation) {
+        give_back(ctx);
+        e = cudaMalloc(&word, 1);
+    }
+    if (e == cudaSuccess)
+        cudaFree(word);
+    else
+        cudaDeviceSynchronize();
+}
+
 // Larger blocks come in powers of two.
 static size_t pinned_class(size_t bytes) {
     size_t c = 4096;
@@ -468,13 +484,18 @@ mi_status mi_image_geometry(const mi_image* img, mi_geometry* out) {
     return MI_OK;
 }
 
-const float* mi_image_device_ptr(const mi_image* img) { return img ? img->data : nullptr; }
+const float* mi_image_device_ptr(const mi_image* img) {
+    if (!img) return nullptr;
+    img->lent = true;
+    return img->data;
+}
 
 mi_status mi_image_free(mi_image* img) {
     if (!img) return MI_ERR_INVALID_ARGUMENT;
     cudaSetDevice(img->ctx->device);
-    // the voxels are lent out (mi_image_device_ptr): work of any stream may still read them
-    cudaDeviceSynchronize();
+    // Voxels that were lent out (mi_image_device_ptr) may still be read by work of any stream;
+    // the library's own calls are done with them, or come before the block's next use.
+    if (img->lent) mi::wait_for_device(img->ctx);
     mi::dev_free(img->ctx, img->data);
     delete img;
     return MI_OK;

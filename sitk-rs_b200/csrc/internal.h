@@ -51,6 +51,7 @@ struct mi_image {
     mi_geometry geo{};
     float* data = nullptr;  // device, x-fastest
     int64_t n = 0;
+    mutable bool lent = false;  // its device address was given out
 };
 
 namespace mi {
@@ -257,6 +258,7 @@ cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
     return e;
 }
 void dev_free(mi_context* ctx, void* p);
+void wait_for_device(mi_context* ctx);  // for the work of all of its streams
 // Pinned host memory mapped into the device (`dev`, its device address, may be null), freed
 // with the size it was asked for.
 constexpr size_t PINNED_BLOCK = 512;
