@@ -108,7 +108,9 @@ typedef struct mi_metric mi_metric;
 
 /* ---- context (cuda/backend.rs:30-160: Backend / backend()) ---------------- */
 
-/* One context per device; owns one CUDA stream. MI_ERR_NO_DEVICE when absent. */
+/* One context per device; owns one CUDA stream. MI_ERR_NO_DEVICE when absent. Destroying it
+ * ends its use for new calls; objects made from it may still be freed afterwards, and its
+ * memory goes with the last of them. */
 mi_status mi_context_create(int device, mi_context** out);
 mi_status mi_context_destroy(mi_context* ctx);
 mi_status mi_context_sync(mi_context* ctx);

@@ -367,7 +367,7 @@ std::map<std::pair<int, int>, std::pair<int, int>> g_tune;
 }  // namespace mi
 
 struct mi_batch {
-    mi_context* ctx = nullptr;
+    mi::Held ctx;
     int npairs = 0, bins = 0, kind = 0, nparams = 0;
     std::vector<mi_metric*> metrics;
     std::vector<std::vector<double>> fixed_params;

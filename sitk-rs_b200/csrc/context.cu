@@ -189,6 +189,20 @@ void wait_for_device(mi_context* ctx) {
         cudaDeviceSynchronize();
 }
 
+void context_release(mi_context* ctx) {
+    if (ctx->holders.fetch_sub(1, std::memory_order_acq_rel) != 1) return;
+    cudaSetDevice(ctx->device);
+    cudaStreamSynchronize(ctx->stream);
+    cudaStreamDestroy(ctx->stream);
+    for (const SpareArray& a : ctx->spare_arrays) cudaFreeArray(a.array);
+    for (const SpareBlock& b : ctx->spare_blocks) cudaFree(b.p);
+    for (unsigned char* slab : ctx->pinned_slabs) cudaFreeHost(slab);
+    for (auto& c : ctx->pinned_large)
+        for (unsigned char* p : c.second) cudaFreeHost(p);
+    cudaMemPoolDestroy(ctx->pool);
+    delete ctx;
+}
+
 // Larger blocks come in powers of two.
 static size_t pinned_class(size_t bytes) {
     size_t c = 4096;
@@ -356,17 +370,8 @@ mi_status mi_context_create(int device, mi_context** out) {
 mi_status mi_context_destroy(mi_context* ctx) {
     if (!ctx) return MI_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
-    if (ctx->stream) {
-        cudaStreamSynchronize(ctx->stream);
-        cudaStreamDestroy(ctx->stream);
-    }
-    for (const mi::SpareArray& a : ctx->spare_arrays) cudaFreeArray(a.array);
-    for (const mi::SpareBlock& b : ctx->spare_blocks) cudaFree(b.p);
-    for (unsigned char* slab : ctx->pinned_slabs) cudaFreeHost(slab);
-    for (auto& c : ctx->pinned_large)
-        for (unsigned char* p : c.second) cudaFreeHost(p);
-    cudaMemPoolDestroy(ctx->pool);
-    delete ctx;
+    cudaStreamSynchronize(ctx->stream);
+    mi::context_release(ctx);
     return MI_OK;
 }
 

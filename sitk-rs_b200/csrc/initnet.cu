@@ -507,7 +507,7 @@ inline int dz_ld(int out) { return (out + 7) & ~7; }
 }  // namespace mi
 
 struct mi_initnet {
-    mi_context* ctx = nullptr;
+    mi::Held ctx;
     int max_batch = 0;
     mi::Layer L[mi::NLAYER] = {};
     int step = 0;

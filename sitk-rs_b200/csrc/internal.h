@@ -3,6 +3,7 @@
 
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
+#include <atomic>
 #include <cstdint>
 #include <list>
 #include <map>
@@ -29,6 +30,8 @@ struct SpareBlock {
 }  // namespace mi
 
 struct mi_context {
+    // its owner's until mi_context_destroy, and every object's that lives from it
+    std::atomic<int> holders{1};
     int device = 0;
     int num_sms = 0;
     size_t l2_bytes = 0;
@@ -46,8 +49,35 @@ struct mi_context {
     size_t spare_array_bytes = 0;
 };
 
+namespace mi {
+void context_release(mi_context* ctx);  // by one holder; the last one's takes it down
+// An object's hold on its context: what an object gives back goes to the context, so a context
+// that is destroyed first (a garbage collector finalises in any order) goes with its last
+// object.
+class Held {
+public:
+    Held() = default;
+    Held(const Held&) = delete;
+    Held& operator=(const Held&) = delete;
+    Held& operator=(mi_context* c) {
+        if (c) c->holders.fetch_add(1, std::memory_order_relaxed);
+        if (ctx_) context_release(ctx_);
+        ctx_ = c;
+        return *this;
+    }
+    ~Held() {
+        if (ctx_) context_release(ctx_);
+    }
+    operator mi_context*() const { return ctx_; }
+    mi_context* operator->() const { return ctx_; }
+
+private:
+    mi_context* ctx_ = nullptr;
+};
+}  // namespace mi
+
 struct mi_image {
-    mi_context* ctx = nullptr;
+    mi::Held ctx;
     mi_geometry geo{};
     float* data = nullptr;  // device, x-fastest
     int64_t n = 0;
@@ -189,7 +219,7 @@ struct MomentsWs {
 }  // namespace mi
 
 struct mi_metric {
-    mi_context* ctx = nullptr;
+    mi::Held ctx;
     int metric_kind = 0;          // MI_METRIC_MATTES, MI_METRIC_MEAN_SQUARES, MI_METRIC_CORRELATION
     mi_geometry fgeo{}, mgeo{};
     float* fixed = nullptr;       // device copy of the fixed volume (whole-grid mean squares and correlation)
