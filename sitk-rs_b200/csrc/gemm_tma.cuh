@@ -110,9 +110,13 @@ __device__ __forceinline__ uint64_t swizzled_desc_mn(uint32_t addr) {
            (2ull << 61);
 }
 
+// ReLU whose sign bit says whether z was positive: 0 for a z so small that BF16 rounds it to
+// zero, −0 for one that is not positive (or NaN). −0 counts as 0 wherever it is used.
+__device__ __forceinline__ float relu(float z) { return z > 0.f ? z : -0.f; }
+
 // What becomes of an element z of the product: stored in C, or where that is null as BF16 in
-// X; z + bias[column] with a bias (the layers' widths are multiples of four), negative
-// values cut off when relu is set. Splits store the plain partial products in C. With
+// X; z + bias[column] with a bias (the layers' widths are multiples of four), then relu()
+// when relu is set. Splits store the plain partial products in C. With
 // `tma` the blocks leave by TMA through the output's map: pitch and base multiples of 16
 // bytes. X always goes that way.
 struct Epilogue {
@@ -345,7 +349,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {
                             const float v = __uint_as_float(r[q + k]) + add[k];
-                            r[q + k] = __float_as_uint(E.relu ? fmaxf(v, 0.f) : v);
+                            r[q + k] = __float_as_uint(E.relu ? relu(v) : v);
                         }
                     }
                 }

@@ -265,12 +265,12 @@ __global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t
     GSTRIDE(i, mn) {
         float acc = 0.0f;
         for (int s = 0; s < splits; ++s) acc += part[(int64_t)s * mn + i];
-        x[i] = __float2bfloat16(fmaxf(acc + bias[i % cols], 0.0f));
+        x[i] = __float2bfloat16(tc::relu(acc + bias[i % cols]));
     }
 }
 
 // The gradient dZ of the layer below from that of a layer's input: dx through the ReLU (its
-// output a is positive where its input was), as BF16 for the next products, and the
+// output a has no sign where its input was positive: tc::relu), as BF16 for the next products, and the
 // CTA's column sums (the bias gradient) of the FP32 values into part[CTA]. dx comes
 // from the layer's product dcol: for a fully connected layer it is dcol itself (D = 0); for
 // a convolution over D³ inputs of C channels it is the transpose of im2col as a gather,
@@ -327,11 +327,10 @@ __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol
             for (int q = 0; q < 8; ++q) v = make_float4(v.x + t[q].x, v.y + t[q].y, v.z + t[q].z, v.w + t[q].w);
         }
         const uint2 act = __ldg(reinterpret_cast<const uint2*>(a + r * C + c));
-        // ReLU outputs: not negative, so positive means not zero
-        v.x = act.x & 0x7fffu ? v.x : 0.f;
-        v.y = act.x & 0x7fff0000u ? v.y : 0.f;
-        v.z = act.y & 0x7fffu ? v.z : 0.f;
-        v.w = act.y & 0x7fff0000u ? v.w : 0.f;
+        v.x = act.x & 0x8000u ? 0.f : v.x;
+        v.y = act.x & 0x80000000u ? 0.f : v.y;
+        v.z = act.y & 0x8000u ? 0.f : v.z;
+        v.w = act.y & 0x80000000u ? 0.f : v.w;
         *reinterpret_cast<uint2*>(dzb + r * C + c) = make_uint2(pack_bf16(v.x, v.y), pack_bf16(v.z, v.w));
         sum = make_float4(sum.x + v.x, sum.y + v.y, sum.z + v.z, sum.w + v.w);
     }
