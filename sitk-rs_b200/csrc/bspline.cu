@@ -542,12 +542,15 @@ __global__ void k_bs_unsort(const uint32_t* __restrict__ order, const uint16_t* 
 // j ≡ ⌊t/16⌋ (mod 16) of each staged group; the sixteen partial sums are then combined in
 // order. The support weights are continuous factors of the derivative, formed in FP32 from
 // the FP64 grid index; the sums are FP64. FP32 → FP64 conversions run at an eighth of the
-// FP64 pipe's rate, so the gradient is staged in FP64 and two of a thread's four weights
-// are widened by integer operations (weights are not negative; a zero becomes 2^-127).
-// Every sample through 112 conversions on one CTA a cell took 102 µs on an 8³ mesh.
-__device__ __forceinline__ double widen_weight(float w) {
+// FP64 pipe's rate, so the gradient is staged in FP64 and the weights are moved into FP64 by
+// shifts alone, 2^896 too small (weights are not negative; zeros and subnormal ones keep
+// their value); powers of two on the staged gradient and on the sums make up for it, so the
+// sums are those of the plain weights. Every sample through 112 conversions on one CTA a
+// cell took 102 µs on an 8³ mesh.
+constexpr double WEIGHT_UP = 0x1p800, SUM_UP = 0x1p96;  // together 2^896
+__device__ __forceinline__ double small_weight(float w) {
     const unsigned int b = __float_as_uint(w);
-    return __hiloint2double((int)((b >> 3) + 0x38000000u), (int)(b << 29));
+    return __hiloint2double((int)(b >> 3), (int)(b << 29));
 }
 
 __global__ void __launch_bounds__(BS_BLOCK)
@@ -609,8 +612,8 @@ k_bs_cell_deriv(const __grid_constant__ SamplerParams P, const __grid_constant__
                 }
             }
         }
-        *reinterpret_cast<double2*>(sg + 4 * t) = make_double2((double)G[0], (double)G[1]);
-        sg[4 * t + 2] = (double)G[2];
+        *reinterpret_cast<double2*>(sg + 4 * t) = make_double2((double)G[0] * WEIGHT_UP, (double)G[1] * WEIGHT_UP);
+        sg[4 * t + 2] = (double)G[2] * WEIGHT_UP;
 #pragma unroll
         for (int q = 0; q < 12; q += 4)
             *reinterpret_cast<float4*>(sw + 12 * t + q) = make_float4(W[q], W[q + 1], W[q + 2], W[q + 3]);
@@ -622,8 +625,8 @@ k_bs_cell_deriv(const __grid_constant__ SamplerParams P, const __grid_constant__
             const float4 wz = *reinterpret_cast<const float4*>(sw + 12 * jj + 8);
             const double2 g01 = *reinterpret_cast<const double2*>(sg + 4 * jj);
             const double g2 = sg[4 * jj + 2];
-            const double w[4] = {(double)(wxy * wz.x), widen_weight(wxy * wz.y), (double)(wxy * wz.z),
-                                 widen_weight(wxy * wz.w)};
+            const double w[4] = {small_weight(wxy * wz.x), small_weight(wxy * wz.y), small_weight(wxy * wz.z),
+                                 small_weight(wxy * wz.w)};
 #pragma unroll
             for (int kz = 0; kz < 4; ++kz) {
                 acc[kz][0] = fma(w[kz], g01.x, acc[kz][0]);
@@ -636,7 +639,7 @@ k_bs_cell_deriv(const __grid_constant__ SamplerParams P, const __grid_constant__
     // the 16 phases of each column, summed in phase order
     for (int kz = 0; kz < 4; ++kz) {
 #pragma unroll
-        for (int d = 0; d < 3; ++d) red[d][t] = acc[kz][d];
+        for (int d = 0; d < 3; ++d) red[d][t] = acc[kz][d] * SUM_UP;
         __syncthreads();
         if (t < 48) {
             const int d = t >> 4, q = t & 15, qx = q & 3, qy = q >> 2;
