@@ -211,6 +211,7 @@ struct MomentsWs {
     int grid = 0, grid_grad = 0;     // CTAs of the value's pass, and with the derivative
     double* partials = nullptr;      // [slots][grid]
     double* shift = nullptr;         // correlation's shift, then that of a repeated pass
+    double base[2] = {0.0, 0.0};     // the shift: of the fixed values, of the moving
     unsigned int* counter = nullptr; // arrivals
     double* host = nullptr;          // pinned, mapped mirror of the folded moments, then the tag
     double* host_dev = nullptr;      // the mirror's device address
