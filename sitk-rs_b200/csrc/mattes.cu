@@ -459,6 +459,14 @@ int hist_grid(mi_context* ctx, int64_t n, int occ, int B) {
     return std::max(1, clusters) * HIST_CLUSTER;
 }
 
+void drop_brick_layout(mi_metric* m) {
+    for (uint32_t** p : {&m->codes, &m->chunk_run, &m->run_brick, &m->run_chunk0, &m->run_start}) {
+        dev_free(m->ctx, *p);
+        *p = nullptr;
+    }
+    m->nchunks = m->nruns = 0;
+}
+
 void free_metric(mi_metric* m) {
     if (!m) return;
     if (m->mtex) cudaDestroyTextureObject(m->mtex);
@@ -471,11 +479,7 @@ void free_metric(mi_metric* m) {
     dev_free(ctx, m->mmask);
     dev_free(ctx, m->samples);
     dev_free(ctx, m->fbin);
-    dev_free(ctx, m->codes);
-    dev_free(ctx, m->chunk_run);
-    dev_free(ctx, m->run_brick);
-    dev_free(ctx, m->run_chunk0);
-    dev_free(ctx, m->run_start);
+    drop_brick_layout(m);
     dev_free(ctx, m->ws.hist);
     dev_free(ctx, m->ws.partials);
     dev_free(ctx, m->ws.vsum);
@@ -668,7 +672,7 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
 // The brick layout of the walk (build_samples with bricks; the whole grid sorted here)
 // and its fixed bins: runs of samples per brick (CUB run-length encoding), each padded to whole
 // chunks of 32, the codes scattered to their padded positions.
-mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
+mi_status fill_brick_layout(mi_context* ctx, mi_metric* m) {
     cudaStream_t st = ctx->stream;
     const int64_t n = m->n_samples;
     const int bl = m->brick_bl;
@@ -808,6 +812,13 @@ mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
     }
 #undef TRY_L
     return done(MI_OK);
+}
+
+// The same, whole or not at all: a metric whose layout could not be built has none.
+mi_status build_brick_layout(mi_context* ctx, mi_metric* m) {
+    const mi_status s = fill_brick_layout(ctx, m);
+    if (s != MI_OK) drop_brick_layout(m);
+    return s;
 }
 
 // The staged-tile pass's shape (tile.cuh): whether the linear moving volume meets the
