@@ -523,11 +523,12 @@ int64_t brick_count(const int64_t* size, int bl) {
     return n;
 }
 
-// The sort of a list by brick key (kept is replaced by the sorted list) and, with `first`, the
-// first sample of every brick. The launches are left on the stream.
+// The sort of a list by brick key (kept, `room` long, is replaced by the sorted list, no longer
+// than it has to be: a mask may leave few of a draw) and, with `first`, the first sample of
+// every brick. The launches are left on the stream.
 template <typename K>
 mi_status sort_samples(mi_context* ctx, const int64_t* size, int bl, int bits, int64_t nbricks, int64_t n, uint32_t** kept,
-                       uint32_t* first) {
+                       size_t room, uint32_t* first) {
     cudaStream_t st = ctx->stream;
     const int block = 256, grid = grid_for(n, block, ctx->num_sms * 8);
     const int64_t nx = size[0], ny = size[1];
@@ -544,6 +545,14 @@ mi_status sort_samples(mi_context* ctx, const int64_t* size, int bl, int bits, i
     if (e == cudaSuccess) e = cub::DeviceRadixSort::SortKeys(nullptr, bytes, keys, sorted, (int)n, 0, bits, st);
     if (e == cudaSuccess) e = dev_alloc(ctx, &tmp, bytes);
     if (e == cudaSuccess) e = cub::DeviceRadixSort::SortKeys(tmp, bytes, keys, sorted, (int)n, 0, bits, st);
+    if (e == cudaSuccess && pad4(n) < room) {
+        uint32_t* list = nullptr;
+        e = dev_alloc(ctx, &list, pad4(n) * 4);
+        if (e == cudaSuccess) {
+            dev_free(ctx, *kept);
+            *kept = list;
+        }
+    }
     if (e == cudaSuccess) {
         k_key_voxel<K><<<grid, block, 0, st>>>(sorted, n, nx, ny, bl, nbx, nby, *kept);
         if (first)
@@ -659,12 +668,12 @@ mi_status build_samples(mi_context* ctx, mi_metric* m, const mi_image* fixed_mas
         while (bits < 64 && ((uint64_t)1 << (bits - 3 * bl)) < (uint64_t)nbricks) ++bits;
         if (first) MI_CHECK_CUDA(ctx, dev_alloc(ctx, first, (size_t)(nbricks + 1) * 4));
         const mi_status s = bits <= 32
-                                ? sort_samples<uint32_t>(ctx, size, bl, bits, nbricks, nkept, &kept, first ? *first : nullptr)
-                                : sort_samples<unsigned long long>(ctx, size, bl, bits, nbricks, nkept, &kept,
-                                                                   first ? *first : nullptr);
+                                ? sort_samples<uint32_t>(ctx, size, bl, bits, nbricks, nkept, &m->samples, pad4(count),
+                                                         first ? *first : nullptr)
+                                : sort_samples<unsigned long long>(ctx, size, bl, bits, nbricks, nkept, &m->samples,
+                                                                   pad4(count), first ? *first : nullptr);
         if (s != MI_OK) return s;
     }
-    m->samples = kept;
     m->n_samples = nkept;
     return MI_OK;
 }

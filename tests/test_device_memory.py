@@ -1,0 +1,11 @@
+"""What the host side holds on the device, and what it leaves when an allocation is refused (no
+device needed)."""
+from host_program import compile_and_run
+
+
+def test_staged_tile_layout_is_whole_or_absent(tmp_path):
+    assert "refused in turn" in compile_and_run("brick_layout", tmp_path)
+
+
+def test_sample_list_is_as_long_as_its_samples(tmp_path):
+    assert "1 samples" in compile_and_run("sample_list", tmp_path)
