@@ -113,6 +113,10 @@ typedef struct mi_metric mi_metric;
  * memory goes with the last of them. */
 mi_status mi_context_create(int device, mi_context** out);
 mi_status mi_context_destroy(mi_context* ctx);
+/* Gives back to the device what the context keeps of freed objects for the next ones (at most
+ * 4 GB of blocks, 1 GB of arrays and 256 MB of its pool), for the allocators of others: the
+ * library's own allocations take it by themselves. No reference counterpart. */
+mi_status mi_context_trim(mi_context* ctx);
 mi_status mi_context_sync(mi_context* ctx);
 /* Detail text of the last failure on ctx (valid until the next call on ctx). */
 const char* mi_last_error(const mi_context* ctx);

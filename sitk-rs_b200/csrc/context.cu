@@ -7,6 +7,7 @@
 
 #include <cuda_runtime.h>
 #include <cudaTypedefs.h>
+#include <algorithm>
 #include <cstdio>
 #include <cstring>
 #include <map>
@@ -72,8 +73,10 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 //   pinned blocks  slabs of 64 small ones, kept until the context goes; of the larger ones up
 //                  to PINNED_SPARES of each size of at most PINNED_KEEP bytes
 //   arrays         at most SPARE_ARRAYS of SPARE_ARRAY_BYTES together, taken by exact shape
-// All of it goes back to the device when an allocation does not fit beside it, and with the
-// context. A block is reused in the order of the context's one stream, so nothing waits.
+// A block is reused in the order of the context's one stream, so nothing waits. What every
+// context of the device keeps (but for the slabs) goes back when a device allocation of any of
+// them does not fit beside it; a context's own, when it is trimmed (for the allocators of
+// others: mi_context_trim), and with the context.
 constexpr unsigned long long POOL_KEEP = 256ull << 20;  // what the pool keeps of freed pages
 constexpr size_t LARGE = (size_t)1 << 20, LARGE_BYTES = (size_t)4 << 30;
 constexpr size_t SPARE_ARRAYS = 64, SPARE_ARRAY_BYTES = (size_t)1 << 30;
@@ -113,14 +116,55 @@ void drop_blocks(mi_context* ctx, size_t bytes) {
     }
 }
 
-// Everything kept goes back to the device, for an allocation that did not fit beside it.
+// The contexts there are (never destroyed: a context may go at the process's end).
+std::mutex& g_contexts_mutex = *new std::mutex;
+std::vector<mi_context*>& g_contexts = *new std::vector<mi_context*>;
+
+// Waits for the work of every stream, as cudaFree of a cudaMalloc'd block does: here a word
+// kept for it. That is allowed while another thread captures a graph on another stream, when
+// cudaDeviceSynchronize fails and invalidates the capture (a batch in another thread lost
+// its registration so). False when there is no word to be had (spare_mutex held).
+bool wait_for_device(mi_context* ctx) {
+    if (!ctx->word && cudaMalloc(&ctx->word, 1) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->word = nullptr;
+        return false;
+    }
+    cudaFree(ctx->word);
+    if (cudaMalloc(&ctx->word, 1) != cudaSuccess) {
+        cudaGetLastError();
+        ctx->word = nullptr;
+    }
+    return true;
+}
+
+// Everything a context keeps goes back, once no work uses it (spare_mutex held).
+void drop_kept(mi_context* ctx) {
+    for (const SpareBlock& b : ctx->spare_blocks) {
+        ctx->large_blocks.erase(b.p);
+        cudaFree(b.p);
+    }
+    ctx->spare_blocks.clear();
+    ctx->spare_block_bytes = 0;
+    drop_arrays(ctx, 0, 0);
+    for (auto& c : ctx->pinned_large) {
+        for (unsigned char* p : c.second) cudaFreeHost(p);
+        c.second.clear();
+    }
+    cudaMemPoolTrimTo(ctx->pool, 0);
+}
+
+// The same of every context of the device, for an allocation of `ctx` that did not fit beside it.
 void give_back(mi_context* ctx) {
     cudaGetLastError();
-    std::lock_guard<std::mutex> g(ctx->spare_mutex);
-    drop_blocks(ctx, 0);
-    drop_arrays(ctx, 0, 0);
-    cudaStreamSynchronize(ctx->stream);
-    cudaMemPoolTrimTo(ctx->pool, 0);
+    std::lock_guard<std::mutex> g(g_contexts_mutex);
+    // (only here does a thread hold more than one of these)
+    std::vector<std::unique_lock<std::mutex>> held;
+    for (mi_context* c : g_contexts)
+        if (c->device == ctx->device) held.emplace_back(c->spare_mutex);
+    if (!wait_for_device(ctx)) return;
+    for (mi_context* c : g_contexts)
+        if (c->device == ctx->device) drop_kept(c);
 }
 
 cudaError_t pool_alloc(mi_context* ctx, void** p, size_t bytes) {
@@ -173,32 +217,29 @@ void dev_free(mi_context* ctx, void* p) {
     drop_blocks(ctx, LARGE_BYTES);
 }
 
-// Waits for the work of every stream as cudaFree of a cudaMalloc'd block does, which is allowed
-// while another thread captures a graph on another stream; cudaDeviceSynchronize then
-// fails and invalidates that capture (a batch in another thread lost its registration so).
-void wait_for_device(mi_context* ctx) {
-    void* word = nullptr;
-    cudaError_t e = cudaMalloc(&word, 1);
-    if (e == cudaErrorMemoryAllocation) {
+void wait_for_all_streams(mi_context* ctx) {
+    for (int turn = 0; turn < 2; ++turn) {
+        {
+            std::lock_guard<std::mutex> g(ctx->spare_mutex);
+            if (wait_for_device(ctx)) return;
+        }
         give_back(ctx);
-        e = cudaMalloc(&word, 1);
     }
-    if (e == cudaSuccess)
-        cudaFree(word);
-    else
-        cudaDeviceSynchronize();
+    cudaDeviceSynchronize();
 }
 
 void context_release(mi_context* ctx) {
     if (ctx->holders.fetch_sub(1, std::memory_order_acq_rel) != 1) return;
+    {
+        std::lock_guard<std::mutex> g(g_contexts_mutex);
+        g_contexts.erase(std::remove(g_contexts.begin(), g_contexts.end(), ctx), g_contexts.end());
+    }
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
     cudaStreamDestroy(ctx->stream);
-    for (const SpareArray& a : ctx->spare_arrays) cudaFreeArray(a.array);
-    for (const SpareBlock& b : ctx->spare_blocks) cudaFree(b.p);
+    drop_kept(ctx);
     for (unsigned char* slab : ctx->pinned_slabs) cudaFreeHost(slab);
-    for (auto& c : ctx->pinned_large)
-        for (unsigned char* p : c.second) cudaFreeHost(p);
+    cudaFree(ctx->word);
     cudaMemPoolDestroy(ctx->pool);
     delete ctx;
 }
@@ -357,13 +398,27 @@ mi_status mi_context_create(int device, mi_context** out) {
     c->l2_bytes = (size_t)l2;
     if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
     if (e == cudaSuccess) e = mi::create_pool(c);
+    if (e == cudaSuccess) e = cudaMalloc(&c->word, 1);
     if (e != cudaSuccess) {
         if (c->pool) cudaMemPoolDestroy(c->pool);
         if (c->stream) cudaStreamDestroy(c->stream);
         delete c;
         return e == cudaErrorNoDevice ? MI_ERR_NO_DEVICE : MI_ERR_CUDA;
     }
+    {
+        std::lock_guard<std::mutex> g(mi::g_contexts_mutex);
+        mi::g_contexts.push_back(c);
+    }
     *out = c;
+    return MI_OK;
+}
+
+mi_status mi_context_trim(mi_context* ctx) {
+    if (!ctx) return MI_ERR_INVALID_ARGUMENT;
+    MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
+    MI_CHECK_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    std::lock_guard<std::mutex> g(ctx->spare_mutex);
+    mi::drop_kept(ctx);
     return MI_OK;
 }
 
@@ -371,6 +426,10 @@ mi_status mi_context_destroy(mi_context* ctx) {
     if (!ctx) return MI_ERR_INVALID_ARGUMENT;
     cudaSetDevice(ctx->device);
     cudaStreamSynchronize(ctx->stream);
+    {
+        std::lock_guard<std::mutex> g(ctx->spare_mutex);
+        mi::drop_kept(ctx);
+    }
     mi::context_release(ctx);
     return MI_OK;
 }
@@ -500,7 +559,7 @@ mi_status mi_image_free(mi_image* img) {
     cudaSetDevice(img->ctx->device);
     // Voxels that were lent out (mi_image_device_ptr) may still be read by work of any stream;
     // the library's own calls are done with them, or come before the block's next use.
-    if (img->lent) mi::wait_for_device(img->ctx);
+    if (img->lent) mi::wait_for_all_streams(img->ctx);
     mi::dev_free(img->ctx, img->data);
     delete img;
     return MI_OK;

@@ -47,6 +47,7 @@ struct mi_context {
     std::unordered_map<void*, size_t> large_blocks;  // every large block, in use or spare
     std::list<mi::SpareArray> spare_arrays;  // oldest first
     size_t spare_array_bytes = 0;
+    void* word = nullptr;  // a cudaMalloc'd one, freed to wait for the device (context.cu)
 };
 
 namespace mi {
@@ -289,7 +290,7 @@ cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
     return e;
 }
 void dev_free(mi_context* ctx, void* p);
-void wait_for_device(mi_context* ctx);  // for the work of all of its streams
+void wait_for_all_streams(mi_context* ctx);  // of the device
 // Pinned host memory mapped into the device (`dev`, its device address, may be null), freed
 // with the size it was asked for.
 constexpr size_t PINNED_BLOCK = 512;

@@ -37,7 +37,7 @@ EXPORTED = [
     "mi_initnet_prepare", "mi_metric_create_ex", "mi_image_resample_nearest",
     "mi_metric_value_and_derivative_bspline", "mi_metric_bspline_records", "mi_image_read_meta",
     "mi_image_read_meta_host", "mi_image_read_nifti", "mi_image_read_nifti_host",
-    "mi_metric_set_tile_staging", "mi_metric_get_tile_staging",
+    "mi_metric_set_tile_staging", "mi_metric_get_tile_staging", "mi_context_trim",
 ]
 
 
@@ -98,6 +98,8 @@ def load(path: str | None = None):
     L.mi_context_create.argtypes = [ctypes.c_int, P(vp)]
     L.mi_context_destroy.argtypes = [vp]
     L.mi_context_sync.argtypes = [vp]
+    L.mi_context_trim.argtypes = [vp]
+    L.mi_context_trim.restype = ctypes.c_int
     L.mi_last_error.argtypes = [vp]
     L.mi_last_error.restype = ctypes.c_char_p
     L.mi_context_stream.argtypes = [vp]

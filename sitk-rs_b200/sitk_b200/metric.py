@@ -50,6 +50,10 @@ class Context:
     def sync(self):
         _lib.check(_lib.load().mi_context_sync(self.handle), self.handle)
 
+    def trim(self):
+        """Gives back to the device what the context keeps of freed objects (mi_context_trim)."""
+        _lib.check(_lib.load().mi_context_trim(self.handle), self.handle)
+
     def stream(self) -> int:
         return _lib.load().mi_context_stream(self.handle) or 0
 
