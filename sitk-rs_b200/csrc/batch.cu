@@ -128,7 +128,7 @@ struct Line {
     int lo, hi;                // the run
 };
 template <class Key>
-__device__ __forceinline__ Line lay_out(const Work* __restrict__ work, int npairs, Key key) {
+__device__ __forceinline__ Line lay_out(const Work* work, int npairs, Key key) {
     __shared__ unsigned long long sums[32];
     const int per = (npairs + (int)blockDim.x - 1) / (int)blockDim.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     Line l;
@@ -159,7 +159,7 @@ struct Place {
 };
 // at < l.total; the whole CTA
 template <class Key>
-__device__ __forceinline__ Place locate(const Work* __restrict__ work, const Line& l, unsigned long long at, Key key) {
+__device__ __forceinline__ Place locate(const Work* work, const Line& l, unsigned long long at, Key key) {
     __shared__ Place found;
     __syncthreads();  // the last one was read
     unsigned long long x = l.first;

@@ -176,7 +176,7 @@ __device__ __forceinline__ void request_tile(uint32_t dst, const CUtensorMap* ma
 template <int NT, bool A_KROWS, bool B_KROWS, int MT = 1>
 __global__ void __launch_bounds__(TMA_THREADS, 1)
 k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
-           const __grid_constant__ CUtensorMap mapOut, int M, int N, int K, const Epilogue E, int splits, unsigned int* __restrict__ err) {
+           const __grid_constant__ CUtensorMap mapOut, int M, int N, int K, const Epilogue E, int splits, unsigned int* err) {
     static_assert(!B_KROWS || NT % 64 == 0, "k-rows tiles come in boxes of 64");
     static_assert(MT == 1 || (!A_KROWS && 2 * NT <= 512), "two blocks of rows fill the tensor memory");
     using S = TmaShape<NT, MT>;
@@ -344,7 +344,7 @@ k_gemm_tma(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUt
 #pragma unroll
                     for (int q = 0; q < W; q += 4) {
                         if (col0 + q >= N) break;
-                        const float4 b = __ldg(reinterpret_cast<const float4*>(E.bias + col0 + q));
+                        const float4 b = __ldca(reinterpret_cast<const float4*>(E.bias + col0 + q));
                         const float add[4] = {b.x, b.y, b.z, b.w};
 #pragma unroll
                         for (int k = 0; k < 4; ++k) {

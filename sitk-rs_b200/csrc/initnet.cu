@@ -216,7 +216,7 @@ __device__ __forceinline__ uint32_t pack_bf16(float a, float b) {
 // same in every pair, blockIdx.y. The caller's input may start on any float: a voxel's two
 // channels are one load only where it starts on eight bytes.
 template <int D, int CIN, int KP, typename T>
-__global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, __nv_bfloat16* __restrict__ col) {
+__global__ void __launch_bounds__(256) k_im2col(const T* x, int B, __nv_bfloat16* col) {
     constexpr uint32_t Do = D / 2, PARTS = KP / 8, N = Do * Do * Do * PARTS;
     pdl::launch_dependents();
     const uint32_t i = blockIdx.x * 256 + threadIdx.x;  // of a sample's rows
@@ -244,13 +244,13 @@ __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, 
                 float2 f = make_float2(0.f, 0.f);
                 if (off[q] >= 0) {
                     const T* at = in + 2 * off[q];
-                    f = paired ? __ldg(reinterpret_cast<const float2*>(at)) : make_float2(__ldg(at), __ldg(at + 1));
+                    f = paired ? __ldca(reinterpret_cast<const float2*>(at)) : make_float2(__ldca(at), __ldca(at + 1));
                 }
                 w[q] = pack_bf16(f.x, f.y);
             }
             v = make_uint4(w[0], w[1], w[2], w[3]);
         } else {
-            if (off[0] >= 0) v = __ldg(reinterpret_cast<const uint4*>(in + (size_t)off[0] * CIN + part % (CIN / 8) * 8));
+            if (off[0] >= 0) v = __ldca(reinterpret_cast<const uint4*>(in + (size_t)off[0] * CIN + part % (CIN / 8) * 8));
         }
         reinterpret_cast<uint4*>(col)[(size_t)b * N + i] = v;
     }
@@ -258,14 +258,13 @@ __global__ void __launch_bounds__(256) k_im2col(const T* __restrict__ x, int B, 
 
 // The end of a layer's forward product that was split over K: the slices summed in order,
 // the bias, ReLU, BF16.
-__global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t mn, const float* __restrict__ bias,
-                             int cols, __nv_bfloat16* __restrict__ x) {
+__global__ void k_slices_act(const float* part, int splits, int64_t mn, const float* bias, int cols, __nv_bfloat16* x) {
     pdl::launch_dependents();
     pdl::wait_previous();
     GSTRIDE(i, mn) {
         float acc = 0.0f;
-        for (int s = 0; s < splits; ++s) acc += part[(int64_t)s * mn + i];
-        x[i] = __float2bfloat16(tc::relu(acc + bias[i % cols]));
+        for (int s = 0; s < splits; ++s) acc += __ldcg(part + (int64_t)s * mn + i);
+        x[i] = __float2bfloat16(tc::relu(acc + __ldca(bias + i % cols)));
     }
 }
 
@@ -280,8 +279,8 @@ __global__ void k_slices_act(const float* __restrict__ part, int splits, int64_t
 // caches, 43 µs tap by tap. (Gather, ReLU, conversion and sums were five launches; the
 // sums, 4,096 rows a thread in order, took 0.9–1.1 ms each.)
 template <int D, int C, int KP>
-__global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol, const __nv_bfloat16* __restrict__ a,
-                                                  int64_t rows, __nv_bfloat16* __restrict__ dzb, float* __restrict__ part) {
+__global__ void __launch_bounds__(256) k_back_act(const float* dcol, const __nv_bfloat16* a, int64_t rows,
+                                                  __nv_bfloat16* dzb, float* part) {
     constexpr int G = C / 4;  // threads a row
     static_assert(256 % G == 0, "a thread's channels stay the same");
     __shared__ float4 sums[256];
@@ -292,7 +291,7 @@ __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol
     for (int64_t r = ((int64_t)blockIdx.x * 256 + threadIdx.x) / G; r < rows; r += (int64_t)gridDim.x * (256 / G)) {
         float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
         if constexpr (D == 0) {
-            v = __ldg(reinterpret_cast<const float4*>(dcol + r * C + c));
+            v = __ldcg(reinterpret_cast<const float4*>(dcol + r * C + c));
         } else {
             constexpr int Do = D / 2;
             const uint32_t in = (uint32_t)(r % (D * D * D));
@@ -319,14 +318,14 @@ __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol
                 t[q] = make_float4(0.f, 0.f, 0.f, 0.f);
                 if (tap[0][z] >= 0 && tap[1][y] >= 0 && tap[2][xx] >= 0) {
                     const int64_t row = ((b * Do + o[0][z]) * Do + o[1][y]) * Do + o[2][xx];
-                    t[q] = __ldg(reinterpret_cast<const float4*>(dcol + row * KP +
-                                                                 ((tap[0][z] * 3 + tap[1][y]) * 3 + tap[2][xx]) * C + c));
+                    t[q] = __ldcg(reinterpret_cast<const float4*>(dcol + row * KP +
+                                                                  ((tap[0][z] * 3 + tap[1][y]) * 3 + tap[2][xx]) * C + c));
                 }
             }
 #pragma unroll
             for (int q = 0; q < 8; ++q) v = make_float4(v.x + t[q].x, v.y + t[q].y, v.z + t[q].z, v.w + t[q].w);
         }
-        const uint2 act = __ldg(reinterpret_cast<const uint2*>(a + r * C + c));
+        const uint2 act = __ldcg(reinterpret_cast<const uint2*>(a + r * C + c));
         v.x = act.x & 0x8000u ? 0.f : v.x;
         v.y = act.x & 0x80000000u ? 0.f : v.y;
         v.z = act.y & 0x8000u ? 0.f : v.z;
@@ -347,16 +346,15 @@ __global__ void __launch_bounds__(256) k_back_act(const float* __restrict__ dcol
 
 // loss = mean (out − t)², dout = 2(out − t)/n as BF16 rows of ld, its column sums into
 // colsum (one CTA, fixed order)
-__global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, const float* __restrict__ t, int rows, int cols,
-                                             __nv_bfloat16* __restrict__ dzb, int ld, float* __restrict__ colsum,
-                                             float* __restrict__ loss) {
+__global__ void __launch_bounds__(256) k_mse(const float* out, const float* t, int rows, int cols, __nv_bfloat16* dzb, int ld,
+                                             float* colsum, float* loss) {
     __shared__ float red[256];
     pdl::launch_dependents();
     pdl::wait_previous();
     const int n = rows * cols;
     float acc = 0.0f;
     for (int i = threadIdx.x; i < n; i += 256) {
-        const float d = out[i] - t[i];
+        const float d = __ldca(out + i) - __ldca(t + i);
         dzb[i / cols * ld + i % cols] = __float2bfloat16(2.0f * d / (float)n);
         acc += d * d;
     }
@@ -373,7 +371,7 @@ __global__ void __launch_bounds__(256) k_mse(const float* __restrict__ out, cons
         const int c = c0 + threadIdx.x / 16, q = threadIdx.x % 16;
         float s = 0.0f;
         if (c < cols)
-            for (int r = q; r < rows; r += 16) s += 2.0f * (out[r * cols + c] - t[r * cols + c]) / (float)n;
+            for (int r = q; r < rows; r += 16) s += 2.0f * (__ldca(out + r * cols + c) - __ldca(t + r * cols + c)) / (float)n;
         red[threadIdx.x] = s;
         __syncthreads();
         if (q == 0 && c < cols) {
@@ -418,7 +416,7 @@ __global__ void __launch_bounds__(256) k_update(const __grid_constant__ Tensors 
         i = blk * 32 + lane;
         if (i < t.n)
 #pragma unroll 8
-            for (int s = warp; s < t.parts; s += 8) g += __ldg(t.part + (int64_t)s * t.n + i);
+            for (int s = warp; s < t.parts; s += 8) g += __ldcg(t.part + (int64_t)s * t.n + i);
         red[warp][lane] = g;
         __syncthreads();
         if (warp > 0) return;
@@ -429,7 +427,7 @@ __global__ void __launch_bounds__(256) k_update(const __grid_constant__ Tensors 
         if (i >= t.n) return;
         if (t.part)
 #pragma unroll 4
-            for (int s = 0; s < t.parts; ++s) g += __ldg(t.part + (int64_t)s * t.n + i);
+            for (int s = 0; s < t.parts; ++s) g += __ldcg(t.part + (int64_t)s * t.n + i);
         else
             g = t.g[i];
     }

@@ -2,6 +2,11 @@
 // scheduled once every CTA of the one before has called launch_dependents() (or left), and
 // waits in wait_previous() for that kernel to complete, with its writes visible, before it
 // touches any of them. Without the attribute the wait returns at once.
+//
+// Such a kernel begins while the launches before it still write, so it reads memory by coherent
+// loads only: __ldca, __ldcg or plain ones through pointers that are not const __restrict__
+// (of which, as of __ldg, the compiler may make non-coherent loads, valid for what nobody
+// writes while the kernel lives, and free to move before the wait).
 #pragma once
 
 #include <cuda_runtime.h>
