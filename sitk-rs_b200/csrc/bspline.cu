@@ -230,11 +230,21 @@ __device__ __noinline__ int bs_sample(const SamplerParams& P, const BSplineDev& 
     return BS_VALID;
 }
 
-// The coefficients from the host's pinned copy: kept on the device (`coef`, for the exact
-// chain), and as control points in moving index space, M·coef, one 32-byte row each; the
-// derivative cleared.
+// Up to this many coefficients and derivatives cross in a pinned copy, and the host looks for
+// the largest coefficient; more are copied from and to the caller's memory, and the device
+// looks (one more wait): beyond it the host's copies and its search cost more. 335,000
+// samples, the value and with the derivative, µs: 59,049 coefficients 114 and 259 pinned,
+// 116 and 325 copied; 89,373: 141 and 375, 130 and 436; 128,625: 176 and 520, 154 and 564;
+// 902,289: 917 and 3,158, 502 and 2,852.
+constexpr int64_t PINNED_COEFS = 98304;
+
+// The coefficients `from` the host's pinned copy or the device's: kept on the device (`coef`
+// where it is not null, for the exact chain), and as control points in moving index space,
+// M·coef, one 32-byte row each; the derivative cleared; the largest |coefficient|'s bits (those
+// of NaN pass infinity's) into `top` where it is not null.
 __global__ void k_bs_points(const SamplerParams P, int64_t nper, const double* __restrict__ from, double* __restrict__ coef,
-                            double4* __restrict__ pts, double* __restrict__ deriv) {
+                            double4* __restrict__ pts, double* __restrict__ deriv, unsigned long long* __restrict__ top) {
+    unsigned long long most = 0ull;
     for (int64_t q = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; q < nper; q += (int64_t)gridDim.x * blockDim.x) {
         const double x = from[q], y = from[nper + q], z = from[2 * nper + q];
         double4 v;
@@ -243,12 +253,20 @@ __global__ void k_bs_points(const SamplerParams P, int64_t nper, const double* _
         v.z = P.mp2i[6] * x + P.mp2i[7] * y + P.mp2i[8] * z;
         v.w = 0.0;
         pts[q] = v;
-        coef[q] = x;
-        coef[nper + q] = y;
-        coef[2 * nper + q] = z;
+        if (coef) {
+            coef[q] = x;
+            coef[nper + q] = y;
+            coef[2 * nper + q] = z;
+        }
         if (deriv)
             for (int d = 0; d < 3; ++d) deriv[d * nper + q] = 0.0;
+        if (top)
+            for (double c : {x, y, z}) most = max(most, (unsigned long long)__double_as_longlong(c) & 0x7fffffffffffffffull);
     }
+    if (!top) return;
+#pragma unroll
+    for (int off = 16; off; off >>= 1) most = max(most, __shfl_xor_sync(0xffffffffu, most, off));
+    if ((threadIdx.x & 31) == 0 && most) atomicMax(top, most);
 }
 
 // The cubic B-spline's four weights at the fraction t ∈ [0, 1] of the support cell.
@@ -263,6 +281,7 @@ __device__ __forceinline__ void bs_weights(double t, double* w) {
 // The grouping of the samples by support cell (once per grid).
 struct CellPlan {
     const uint32_t* order;  // walk position of the j-th sample in cell order
+    const uint32_t* cell;   // its cell (ncells: outside)
     const uint32_t* flat;   // its voxel
     const uint8_t* fbin;    // its fixed bin
     const uint32_t* off;    // [cells + 1] first sample of every cell; the rest lie outside
@@ -310,27 +329,13 @@ k_bs_hist(const __grid_constant__ SamplerParams P, const __grid_constant__ BSpli
     const int B = P.bins, B2 = B * B, nb = B2 + B, words = bs_copy_words(B);
     for (int q = threadIdx.x; q < copies * words; q += blockDim.x) bh[q] = 0u;
     const uint32_t j0 = blockIdx.x * per_cta, j1 = min(a.n, j0 + per_cta);
-    // the cell of this thread's first sample: the last whose offset does not pass it
-    uint32_t cell = 0;
-    {
-        const uint32_t j = min(j0 + 2 * threadIdx.x, a.n ? a.n - 1 : 0u);
-        uint32_t lo = 0, hi = C.ncells + 1;  // off[lo] ≤ j < off[hi], off[ncells + 1] = n
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (__ldg(C.off + mid) <= j)
-                lo = mid;
-            else
-                hi = mid;
-        }
-        cell = lo;
-    }
     __syncthreads();
     unsigned int* mine = bh + (threadIdx.x & (copies - 1)) * words;
     const uint32_t ncx = (uint32_t)(S.gsize[0] - 3), ncy = (uint32_t)(S.gsize[1] - 3);
 
     // the affine part of a sample, and its cubic weights in its cell
     auto begin = [&](uint32_t j, BsSample& q, double (&w)[3][4]) {
-        while (cell < C.ncells && j >= __ldg(C.off + cell + 1)) ++cell;
+        const uint32_t cell = __ldg(C.cell + j);
         q.cell = cell;
         q.flat = __ldg(C.flat + j);
         uint32_t i, jj, k;
@@ -688,23 +693,59 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     }
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     cudaStream_t st = ctx->stream;
+    Workspace& ws = m->ws;
+    const bool pinned = ncoef <= PINNED_COEFS;
     if ((size_t)ncoef > m->bs_cap) {
         dev_free(ctx, m->bs_coef);
         dev_free(ctx, m->bs_deriv);
         dev_free(ctx, m->bs_points);
-        pinned_free(ctx, m->bs_host, m->bs_cap * sizeof(double));
-        m->bs_host = m->bs_host_dev = nullptr;
         m->bs_coef = m->bs_deriv = nullptr;
         m->bs_points = nullptr;
         m->bs_cap = 0;
         MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_coef, (size_t)ncoef * sizeof(double)));
         MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_deriv, (size_t)ncoef * sizeof(double)));
         MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_points, (size_t)S.nper * sizeof(double4)));
-        MI_CHECK_CUDA(ctx, pinned_alloc(ctx, (void**)&m->bs_host, (void**)&m->bs_host_dev, (size_t)ncoef * sizeof(double)));
         m->bs_cap = (size_t)ncoef;
     }
-    std::memcpy(m->bs_host, coef, (size_t)ncoef * sizeof(double));
-    Workspace& ws = m->ws;
+    if (pinned && (size_t)ncoef > m->bs_host_cap) {
+        pinned_free(ctx, m->bs_host, m->bs_host_cap * sizeof(double));
+        m->bs_host = m->bs_host_dev = nullptr;
+        m->bs_host_cap = 0;
+        MI_CHECK_CUDA(ctx, pinned_alloc(ctx, (void**)&m->bs_host, (void**)&m->bs_host_dev, (size_t)ncoef * sizeof(double)));
+        m->bs_host_cap = (size_t)ncoef;
+    }
+    // the largest |coefficient|, by its bits
+    unsigned long long top = 0ull;
+    const auto points = [&](const double* from, double* keep, unsigned long long* most) {
+        k_bs_points<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((S.nper + 127) / 128, (int64_t)ctx->num_sms * 8)), 128,
+                      0, st>>>(m->base, S.nper, from, keep, reinterpret_cast<double4*>(m->bs_points),
+                               derivative ? m->bs_deriv : nullptr, most);
+        return cudaGetLastError();
+    };
+    if (pinned) {
+        std::memcpy(m->bs_host, coef, (size_t)ncoef * sizeof(double));
+        // eight at a time
+        unsigned long long most[8] = {};
+        const auto bits_at = [&](int64_t q) {
+            unsigned long long v;
+            std::memcpy(&v, coef + q, 8);
+            return v & 0x7fffffffffffffffull;
+        };
+        int64_t q = 0;
+        for (; q + 8 <= ncoef; q += 8)
+            for (int e = 0; e < 8; ++e) most[e] = std::max(most[e], bits_at(q + e));
+        for (; q < ncoef; ++q) most[0] = std::max(most[0], bits_at(q));
+        for (unsigned long long v : most) top = std::max(top, v);
+        MI_CHECK_CUDA(ctx, points(m->bs_host_dev, m->bs_coef, nullptr));
+    } else {
+        unsigned long long* most = reinterpret_cast<unsigned long long*>(ws.result);  // (free until the pass)
+        MI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->bs_coef, coef, (size_t)ncoef * sizeof(double), cudaMemcpyHostToDevice, st));
+        MI_CHECK_CUDA(ctx, cudaMemsetAsync(most, 0, sizeof(*most), st));
+        MI_CHECK_CUDA(ctx, points(m->bs_coef, nullptr, most));
+        MI_CHECK_CUDA(ctx, cudaMemcpyAsync(ws.host_result, most, sizeof(*most), cudaMemcpyDeviceToHost, st));
+        MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
+        std::memcpy(&top, ws.host_result, sizeof(top));
+    }
     const int B = m->bins;
     const uint32_t n = (uint32_t)m->n_samples;
     // The point map without the displacement (the identity stage): c = cA·idx + cb.
@@ -719,19 +760,7 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     FastBounds F;
     {
         double cmax = 0.0, gmag = 0.0;
-        // the largest |coefficient|, by its bits (those of NaN pass infinity's), eight at a time
-        unsigned long long top[8] = {};
-        auto bits_at = [&](int64_t q) {
-            unsigned long long v;
-            std::memcpy(&v, coef + q, 8);
-            return v & 0x7fffffffffffffffull;
-        };
-        int64_t q8 = 0;
-        for (; q8 + 8 <= ncoef; q8 += 8)
-            for (int e = 0; e < 8; ++e) top[e] = std::max(top[e], bits_at(q8 + e));
-        for (; q8 < ncoef; ++q8) top[0] = std::max(top[0], bits_at(q8));
-        for (int e = 1; e < 8; ++e) top[0] = std::max(top[0], top[e]);
-        std::memcpy(&cmax, top, 8);
+        std::memcpy(&cmax, &top, 8);
         const bool finite = cmax <= DBL_MAX;
         S.zero = cmax == 0.0 ? 1 : 0;
         double to_index = 0.0;
@@ -787,7 +816,8 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
         dev_free(ctx, m->bs_off);
         dev_free(ctx, m->bs_flat);
         dev_free(ctx, m->bs_fbin);
-        m->bs_order = m->bs_off = m->bs_flat = nullptr;
+        dev_free(ctx, m->bs_cell);
+        m->bs_order = m->bs_off = m->bs_flat = m->bs_cell = nullptr;
         m->bs_fbin = nullptr;
         const bool any = S.gsize[0] > 3 && S.gsize[1] > 3 && S.gsize[2] > 3;
         const int64_t ncells = any ? (S.gsize[0] - 3) * (S.gsize[1] - 3) * (S.gsize[2] - 3) : 0;
@@ -795,7 +825,7 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
             return set_error(ctx, MI_ERR_INVALID_ARGUMENT, "B-spline grid too large (≥ 2^31 support cells)");
         m->bs_ncells = ncells;
         const size_t cap = std::max<uint32_t>(n, 1u);
-        uint32_t *cell = nullptr, *idx = nullptr, *sorted = nullptr;
+        uint32_t *cell = nullptr, *idx = nullptr;
         void* tmp = nullptr;
         size_t sort_bytes = 0;
         int bits = 1;
@@ -803,7 +833,7 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
         const int g = (int)std::max<int64_t>(1, std::min<int64_t>(want, (int64_t)ctx->num_sms * 8));
         cudaError_t e = dev_alloc(ctx, &cell, cap * 4);
         if (e == cudaSuccess) e = dev_alloc(ctx, &idx, cap * 4);
-        if (e == cudaSuccess) e = dev_alloc(ctx, &sorted, cap * 4);
+        if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_cell, cap * 4);
         if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_order, cap * 4);
         if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_flat, cap * 4);
         if (e == cudaSuccess) e = dev_alloc(ctx, &m->bs_fbin, cap);
@@ -812,26 +842,25 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
             k_bs_cell_of<<<g, BS_BLOCK, 0, st>>>(P, S, m->samples, n, (uint32_t)ncells, cell, idx);
             e = cudaGetLastError();
             if (e == cudaSuccess)
-                e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, cell, sorted, idx, m->bs_order, (int)n, 0, bits, st);
+                e = cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, cell, m->bs_cell, idx, m->bs_order, (int)n, 0, bits, st);
             if (e == cudaSuccess) e = dev_alloc(ctx, &tmp, sort_bytes);
             if (e == cudaSuccess)
-                e = cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, cell, sorted, idx, m->bs_order, (int)n, 0, bits, st);
+                e = cub::DeviceRadixSort::SortPairs(tmp, sort_bytes, cell, m->bs_cell, idx, m->bs_order, (int)n, 0, bits, st);
         }
         if (e == cudaSuccess) {
-            k_bs_plan<<<g, BS_BLOCK, 0, st>>>(sorted, m->bs_order, m->samples, m->fbin, n, (uint32_t)ncells, m->bs_off,
+            k_bs_plan<<<g, BS_BLOCK, 0, st>>>(m->bs_cell, m->bs_order, m->samples, m->fbin, n, (uint32_t)ncells, m->bs_off,
                                               m->bs_flat, m->bs_fbin);
             e = cudaGetLastError();
         }
         dev_free(ctx, tmp);
         dev_free(ctx, cell);
         dev_free(ctx, idx);
-        dev_free(ctx, sorted);
         if (e != cudaSuccess) return cuda_status(ctx, e, "B-spline support cells");
         std::memcpy(m->bs_key, fixed18, sizeof(m->bs_key));
         m->bs_have_key = true;
     }
     if (!m->bs_pr) MI_CHECK_CUDA(ctx, dev_alloc(ctx, &m->bs_pr, (size_t)B * B * sizeof(float)));
-    const CellPlan C{m->bs_order, m->bs_flat, m->bs_fbin, m->bs_off, (uint32_t)m->bs_ncells};
+    const CellPlan C{m->bs_order, m->bs_cell, m->bs_flat, m->bs_fbin, m->bs_off, (uint32_t)m->bs_ncells};
     const size_t hsm = bs_hist_smem(B);
     const size_t csm = (size_t)BS_BLOCK * (4 * sizeof(double) + 12 * sizeof(float)) + (size_t)B * B * sizeof(float);
     const bool rec = derivative || records;
@@ -839,9 +868,6 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     mi_status ls = raise_smem_limit(ctx, hist_fn, hsm);
     if (ls == MI_OK) ls = raise_smem_limit(ctx, (const void*)k_bs_cell_deriv, csm);
     if (ls != MI_OK) return ls;
-    k_bs_points<<<(unsigned)std::max<int64_t>(1, std::min<int64_t>((S.nper + 127) / 128, (int64_t)ctx->num_sms * 8)), 128, 0,
-                  st>>>(P, S.nper, m->bs_host_dev, m->bs_coef, reinterpret_cast<double4*>(m->bs_points),
-                         derivative ? m->bs_deriv : nullptr);
     // one round of CTAs, each a stretch of whole blocks of sample pairs (more where a counter
     // could otherwise see more than 65,536 samples)
     const int64_t blocks = std::max<int64_t>(1, ((int64_t)n + 2 * BS_HIST_BLOCK - 1) / (2 * BS_HIST_BLOCK));
@@ -874,14 +900,14 @@ mi_status evaluate_bspline(mi_metric* m, const double* fixed18, const double* co
     MI_CHECK_CUDA(ctx, cudaGetLastError());
     // (the coefficients have been read before the derivative comes back)
     if (derivative)
-        MI_CHECK_CUDA(ctx, cudaMemcpyAsync(m->bs_host, m->bs_deriv, (size_t)ncoef * sizeof(double), cudaMemcpyDeviceToHost,
-                                           st));
+        MI_CHECK_CUDA(ctx, cudaMemcpyAsync(pinned ? m->bs_host : derivative, m->bs_deriv, (size_t)ncoef * sizeof(double),
+                                           cudaMemcpyDeviceToHost, st));
     if (walk_bins) {
         MI_CHECK_CUDA(ctx, cudaMemcpyAsync(records, walk_bins, (size_t)n * sizeof(uint16_t), cudaMemcpyDeviceToHost, st));
         dev_free(ctx, walk_bins);
     }
     MI_CHECK_CUDA(ctx, cudaStreamSynchronize(st));
-    if (derivative) std::memcpy(derivative, m->bs_host, (size_t)ncoef * sizeof(double));
+    if (derivative && pinned) std::memcpy(derivative, m->bs_host, (size_t)ncoef * sizeof(double));
     if (value) *value = ws.host_result[0];
     if (valid) *valid = (int64_t)ws.host_result[1];
     return MI_OK;

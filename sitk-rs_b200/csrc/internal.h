@@ -262,10 +262,12 @@ struct mi_metric {
     bool bs_have_key = false;
     uint32_t* bs_order = nullptr;  // sample indices sorted by cell (valid-region samples first)
     uint32_t* bs_off = nullptr;    // [cells + 1] offsets into bs_order
-    uint32_t* bs_flat = nullptr;   // the samples' voxels and fixed bins in that order
+    uint32_t* bs_cell = nullptr;   // the samples' cells, voxels and fixed bins in that order
+    uint32_t* bs_flat = nullptr;
     uint8_t* bs_fbin = nullptr;
     double* bs_host = nullptr;     // pinned copy of the coefficients in, the derivative out
     double* bs_host_dev = nullptr; // and its device address
+    size_t bs_host_cap = 0;        // its capacity, in doubles
     void* bs_points = nullptr;     // control points in moving index space (double4 each)
     int64_t bs_ncells = 0;
     float* bs_pr = nullptr;        // the pRatio·nFactor table of the last evaluation

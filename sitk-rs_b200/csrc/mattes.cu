@@ -497,10 +497,11 @@ void free_metric(mi_metric* m) {
     dev_free(ctx, m->bs_deriv);
     dev_free(ctx, m->bs_order);
     dev_free(ctx, m->bs_off);
+    dev_free(ctx, m->bs_cell);
     dev_free(ctx, m->bs_flat);
     dev_free(ctx, m->bs_fbin);
     dev_free(ctx, m->bs_points);
-    pinned_free(ctx, m->bs_host, m->bs_cap * sizeof(double));
+    pinned_free(ctx, m->bs_host, m->bs_host_cap * sizeof(double));
     dev_free(ctx, m->bs_pr);
     delete m;
 }
