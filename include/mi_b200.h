@@ -134,9 +134,7 @@ mi_status mi_image_from_device(mi_context* ctx, const float* device_ptr,
 mi_status mi_image_to_host(const mi_image* img, float* dst, size_t n_elements);
 mi_status mi_image_geometry(const mi_image* img, mi_geometry* out);
 /* Device address of the image's f32 voxels (borrowed; valid until mi_image_free, which then
- * waits for the work of every stream of the device). The first call moves the voxels into an
- * allocation of their own, which may be shared with other devices and processes (not while
- * the context's stream is captured, nor where there is no room for it). */
+ * waits for the work of every stream of the device). */
 const float* mi_image_device_ptr(const mi_image* img);
 mi_status mi_image_free(mi_image* img);
 

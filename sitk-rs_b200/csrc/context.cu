@@ -217,45 +217,6 @@ void dev_free(mi_context* ctx, void* p) {
     drop_blocks(ctx, LARGE_BYTES);
 }
 
-// The voxels of an image whose address is about to be given out, moved to a cudaMalloc'd block:
-// the pool's blocks cannot be shared with other processes or mapped by other devices, and
-// what may use a lent address has to be waited for at the end (mi_image_free). Where there is
-// no room, or the context's stream is being captured, they stay. An open capture of another
-// stream is not disturbed.
-void lend(mi_image* img) {
-    mi_context* ctx = img->ctx;
-    img->lent = true;
-    int device = 0;
-    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaGetDevice(&device) != cudaSuccess || cudaSetDevice(ctx->device) != cudaSuccess ||
-        cudaThreadExchangeStreamCaptureMode(&mode) != cudaSuccess) {
-        cudaGetLastError();
-        return;
-    }
-    void* p = nullptr;
-    if (cudaStreamIsCapturing(ctx->stream, &capture) == cudaSuccess && capture == cudaStreamCaptureStatusNone) {
-        const size_t bytes = (size_t)img->n * sizeof(float);
-        cudaError_t e = cudaMalloc(&p, bytes);
-        if (e == cudaErrorMemoryAllocation) {
-            give_back(ctx);
-            e = cudaMalloc(&p, bytes);
-        }
-        if (e == cudaSuccess) e = cudaMemcpyAsync(p, img->data, bytes, cudaMemcpyDeviceToDevice, ctx->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
-        if (e == cudaSuccess) {
-            dev_free(ctx, img->data);
-            img->data = static_cast<float*>(p);
-            img->own_block = true;
-        } else if (p) {
-            cudaFree(p);
-        }
-    }
-    cudaGetLastError();
-    cudaThreadExchangeStreamCaptureMode(&mode);
-    cudaSetDevice(device);
-}
-
 void wait_for_all_streams(mi_context* ctx) {
     for (int turn = 0; turn < 2; ++turn) {
         {
@@ -589,22 +550,17 @@ mi_status mi_image_geometry(const mi_image* img, mi_geometry* out) {
 
 const float* mi_image_device_ptr(const mi_image* img) {
     if (!img) return nullptr;
-    if (!img->lent) mi::lend(const_cast<mi_image*>(img));
+    img->lent = true;
     return img->data;
 }
 
 mi_status mi_image_free(mi_image* img) {
     if (!img) return MI_ERR_INVALID_ARGUMENT;
     cudaSetDevice(img->ctx->device);
-    // Voxels that were lent out (mi_image_device_ptr) may still be read by work of any stream,
-    // which cudaFree waits for; the library's own calls are done with them, or come before
-    // the block's next use.
-    if (img->own_block) {
-        cudaFree(img->data);
-    } else {
-        if (img->lent) mi::wait_for_all_streams(img->ctx);
-        mi::dev_free(img->ctx, img->data);
-    }
+    // Voxels that were lent out (mi_image_device_ptr) may still be read by work of any stream;
+    // the library's own calls are done with them, or come before the block's next use.
+    if (img->lent) mi::wait_for_all_streams(img->ctx);
+    mi::dev_free(img->ctx, img->data);
     delete img;
     return MI_OK;
 }

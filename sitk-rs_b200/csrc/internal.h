@@ -82,8 +82,7 @@ struct mi_image {
     mi_geometry geo{};
     float* data = nullptr;  // device, x-fastest
     int64_t n = 0;
-    bool lent = false;       // its device address was given out
-    bool own_block = false;  // data is a cudaMalloc'd block (context.cu)
+    mutable bool lent = false;  // its device address was given out
 };
 
 namespace mi {
@@ -294,7 +293,6 @@ cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
 }
 void dev_free(mi_context* ctx, void* p);
 void wait_for_all_streams(mi_context* ctx);  // of the device
-void lend(mi_image* img);
 // Pinned host memory mapped into the device (`dev`, its device address, may be null), freed
 // with the size it was asked for.
 constexpr size_t PINNED_BLOCK = 512;
