@@ -66,10 +66,14 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // pair takes 0.65–0.75 ms at any size up to 128 MB, a 128-byte cudaHostAlloc / cudaFreeHost
 // pair 2.2 ms and a layered array 0.45 ms; the pool hands a block out and back in 4 µs.
 // A metric holds about twenty blocks, so its set-up was mostly these calls.
-//   device memory  a stream-ordered pool of the context for blocks below LARGE, and spare
-//                  blocks of at most LARGE_BYTES together above it, taken by the nearest
-//                  size (the pool maps freed pages anew where a block of another size takes
-//                  their place: 0.2–5 ms for 64–128 MB)
+//   device memory  a stream-ordered pool of the context for blocks below LARGE; above it spare
+//                  blocks of the pool, at most SPARE_BLOCKS of LARGE_BYTES together, taken by
+//                  the nearest size (the pool maps freed pages anew where a block of another
+//                  size takes their place: 0.2–5 ms for 64–128 MB). Images of any size have
+//                  cudaMalloc'd blocks, kept in the same way: their address may be given out,
+//                  and memory of a pool is neither shared with other processes nor mapped by
+//                  other devices (for all large blocks they made a process's first batch of
+//                  24 pairs 42–48 ms; 30 with this, 24 with the pool alone)
 //   pinned blocks  slabs of 64 small ones, kept until the context goes; of the larger ones up
 //                  to PINNED_SPARES of each size of at most PINNED_KEEP bytes
 //   arrays         at most SPARE_ARRAYS of SPARE_ARRAY_BYTES together, taken by exact shape
@@ -78,7 +82,8 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // them does not fit beside it; a context's own, when it is trimmed (for the allocators of
 // others: mi_context_trim), and with the context.
 constexpr unsigned long long POOL_KEEP = 256ull << 20;  // what the pool keeps of freed pages
-constexpr size_t LARGE = (size_t)1 << 20, LARGE_BYTES = (size_t)4 << 30;
+constexpr size_t LARGE = (size_t)1 << 20, LARGE_BYTES = (size_t)4 << 30, SPARE_BLOCKS = 256;
+constexpr size_t IMAGE_GRAIN = (size_t)1 << 16;  // of images below LARGE
 constexpr size_t SPARE_ARRAYS = 64, SPARE_ARRAY_BYTES = (size_t)1 << 30;
 constexpr size_t SLAB_BLOCKS = 64, PINNED_SPARES = 4, PINNED_KEEP = (size_t)16 << 20;
 
@@ -104,14 +109,16 @@ void drop_arrays(mi_context* ctx, size_t count, size_t bytes) {
     }
 }
 
-// The spare large blocks beyond `bytes` together go to the pool, oldest first (spare_mutex
-// held).
-void drop_blocks(mi_context* ctx, size_t bytes) {
-    while (!ctx->spare_blocks.empty() && ctx->spare_block_bytes > bytes) {
+// The spare blocks beyond `count` of `bytes` together go, oldest first (spare_mutex held).
+void drop_blocks(mi_context* ctx, size_t count, size_t bytes) {
+    while (!ctx->spare_blocks.empty() && (ctx->spare_blocks.size() > count || ctx->spare_block_bytes > bytes)) {
         const auto oldest = ctx->spare_blocks.begin();
         ctx->spare_block_bytes -= oldest->bytes;
         ctx->large_blocks.erase(oldest->p);
-        cudaFreeAsync(oldest->p, ctx->stream);
+        if (oldest->image)
+            cudaFree(oldest->p);
+        else
+            cudaFreeAsync(oldest->p, ctx->stream);
         ctx->spare_blocks.erase(oldest);
     }
 }
@@ -177,16 +184,13 @@ cudaError_t pool_alloc(mi_context* ctx, void** p, size_t bytes) {
     return e;
 }
 
-}  // namespace
-
-cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
-    if (bytes < LARGE) return pool_alloc(ctx, p, bytes ? bytes : 1);
-    bytes = (bytes + LARGE - 1) & ~(LARGE - 1);
+// A block that is kept, or a spare one of up to a quarter more.
+cudaError_t block_alloc(mi_context* ctx, void** p, size_t bytes, bool image) {
     {
         std::lock_guard<std::mutex> g(ctx->spare_mutex);
         auto best = ctx->spare_blocks.end();
         for (auto it = ctx->spare_blocks.begin(); it != ctx->spare_blocks.end(); ++it)
-            if (it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
+            if (it->image == image && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
                 (best == ctx->spare_blocks.end() || it->bytes < best->bytes))
                 best = it;
         if (best != ctx->spare_blocks.end()) {
@@ -196,11 +200,37 @@ cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
             return cudaSuccess;
         }
     }
-    const cudaError_t e = pool_alloc(ctx, p, bytes);
-    if (e == cudaSuccess) {
-        std::lock_guard<std::mutex> g(ctx->spare_mutex);
-        ctx->large_blocks[*p] = bytes;
+    cudaError_t e;
+    if (image) {
+        e = cudaMalloc(p, bytes);
+        if (e == cudaErrorMemoryAllocation) {
+            give_back(ctx);
+            e = cudaMalloc(p, bytes);
+        }
+    } else {
+        e = pool_alloc(ctx, p, bytes);
     }
+    if (e != cudaSuccess) {
+        *p = nullptr;
+        return e;
+    }
+    std::lock_guard<std::mutex> g(ctx->spare_mutex);
+    ctx->large_blocks[*p] = SpareBlock{*p, bytes, image};
+    return e;
+}
+
+}  // namespace
+
+cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes) {
+    if (bytes < LARGE) return pool_alloc(ctx, p, bytes ? bytes : 1);
+    return block_alloc(ctx, p, (bytes + LARGE - 1) & ~(LARGE - 1), false);
+}
+
+cudaError_t image_alloc(mi_context* ctx, float** p, int64_t voxels) {
+    const size_t bytes = (size_t)voxels * sizeof(float), grain = bytes < LARGE ? IMAGE_GRAIN : LARGE;
+    void* v = nullptr;
+    const cudaError_t e = block_alloc(ctx, &v, (bytes + grain - 1) & ~(grain - 1), true);
+    *p = static_cast<float*>(v);
     return e;
 }
 
@@ -212,9 +242,9 @@ void dev_free(mi_context* ctx, void* p) {
         cudaFreeAsync(p, ctx->stream);
         return;
     }
-    ctx->spare_blocks.push_back(SpareBlock{p, large->second});
-    ctx->spare_block_bytes += large->second;
-    drop_blocks(ctx, LARGE_BYTES);
+    ctx->spare_blocks.push_back(large->second);
+    ctx->spare_block_bytes += large->second.bytes;
+    drop_blocks(ctx, SPARE_BLOCKS, LARGE_BYTES);
 }
 
 void wait_for_all_streams(mi_context* ctx) {
@@ -459,7 +489,7 @@ mi_status mi_image_upload(mi_context* ctx, const void* host, mi_dtype dtype,
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     int64_t n = geometry->size[0] * geometry->size[1] * geometry->size[2];
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)n * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::image_alloc(ctx, &d, n));
     cudaError_t e = cudaSuccess;
     if (dtype == MI_F32) {
         e = cudaMemcpyAsync(d, host, (size_t)n * 4, cudaMemcpyHostToDevice, ctx->stream);
@@ -511,7 +541,7 @@ mi_status mi_image_from_device(mi_context* ctx, const float* device_ptr, const m
     MI_CHECK_CUDA(ctx, cudaSetDevice(ctx->device));
     int64_t n = geometry->size[0] * geometry->size[1] * geometry->size[2];
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)n * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::image_alloc(ctx, &d, n));
     cudaError_t e = cudaMemcpyAsync(d, device_ptr, (size_t)n * 4, cudaMemcpyDeviceToDevice, ctx->stream);
     if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
     if (e != cudaSuccess) {

@@ -22,10 +22,11 @@ struct SpareArray {
     bool layered;
     size_t bytes() const { return extent[0] * extent[1] * extent[2] * element; }
 };
-// A large block of device memory waiting for its next use.
+// A block of device memory that waits for its next use between two; an image's is cudaMalloc'd.
 struct SpareBlock {
     void* p;
     size_t bytes;
+    bool image;
 };
 }  // namespace mi
 
@@ -44,7 +45,7 @@ struct mi_context {
     std::map<size_t, std::vector<unsigned char*>> pinned_large;  // spare ones by size
     std::list<mi::SpareBlock> spare_blocks;  // oldest first
     size_t spare_block_bytes = 0;
-    std::unordered_map<void*, size_t> large_blocks;  // every large block, in use or spare
+    std::unordered_map<void*, mi::SpareBlock> large_blocks;  // every such block, in use or spare
     std::list<mi::SpareArray> spare_arrays;  // oldest first
     size_t spare_array_bytes = 0;
     void* word = nullptr;  // a cudaMalloc'd one, freed to wait for the device (context.cu)
@@ -280,7 +281,7 @@ mi_status cuda_status(mi_context* ctx, cudaError_t e, const char* where);
 // The driver's cuTensorMapEncodeTiled, or null.
 PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder();
 
-// Device memory from the context's pool, ordered on the context's stream: a block may be
+// Device memory from what the context keeps, ordered on the context's stream: a block may be
 // freed while work on that stream still uses it, and what reuses it comes after that
 // work. Memory that another stream touches is freed only once that stream is done.
 cudaError_t dev_alloc_bytes(mi_context* ctx, void** p, size_t bytes);
@@ -291,6 +292,7 @@ cudaError_t dev_alloc(mi_context* ctx, T** p, size_t bytes) {
     *p = static_cast<T*>(v);
     return e;
 }
+cudaError_t image_alloc(mi_context* ctx, float** p, int64_t voxels);  // an image's voxels
 void dev_free(mi_context* ctx, void* p);
 void wait_for_all_streams(mi_context* ctx);  // of the device
 // Pinned host memory mapped into the device (`dev`, its device address, may be null), freed

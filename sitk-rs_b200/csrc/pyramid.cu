@@ -650,7 +650,7 @@ mi_status gauss_axis(mi_context* ctx, const TI* in, double* mid, TO* out, const 
 mi_status new_image(mi_context* ctx, const mi_geometry& geo, mi_image** out) {
     const int64_t n = geo.size[0] * geo.size[1] * geo.size[2];
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)n * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::image_alloc(ctx, &d, n));
     mi_image* img = new (std::nothrow) mi_image();
     if (!img) {
         mi::dev_free(ctx, d);

@@ -113,7 +113,7 @@ mi_status new_cube(mi_context* ctx, int n, mi_image** out) {
     g.direction[0] = g.direction[4] = g.direction[8] = 1.0;
     const int64_t nv = (int64_t)n * n * n;
     float* d = nullptr;
-    MI_CHECK_CUDA(ctx, mi::dev_alloc(ctx, &d, (size_t)nv * sizeof(float)));
+    MI_CHECK_CUDA(ctx, mi::image_alloc(ctx, &d, nv));
     mi_image* img = new (std::nothrow) mi_image();
     if (!img) {
         mi::dev_free(ctx, d);
