@@ -1104,8 +1104,11 @@ __device__ TailCtx deriv_phase(const SamplerParams& P, const EvalArgs& a, double
 // (value_term, slice_sum) into a.vsum, and the last CTA folds them (fold_slices), so
 // the value has the bits of every other form. No CTA waits for another before its
 // record stream, and the histogram pass ends at its flush.
+// The shared memory: moment scratch, the table, then (on whole 8 bytes: the table's B² floats
+// are odd with B) the column sums and fixed counts.
+__host__ __device__ inline size_t stream_table_floats(int B) { return ((size_t)B * B + 1) & ~(size_t)1; }
 __host__ __device__ inline size_t stream_smem(int B) {
-    return 32 * (size_t)NMOM * sizeof(double) + (size_t)B * B * sizeof(float) + (size_t)2 * B * 8;
+    return 32 * (size_t)NMOM * sizeof(double) + stream_table_floats(B) * sizeof(float) + (size_t)2 * B * 8;
 }
 
 // Its first part: the table, margins and counts in dsh, the tail state returned, and the
@@ -1119,7 +1122,7 @@ __device__ __forceinline__ TableCtx stream_table(const SamplerParams& P, const E
                                                  typename Src::Group& cur) {
     const int B = P.bins, B2 = B * B;
     float* pr = reinterpret_cast<float*>(dsh + 32 * NMOM);
-    unsigned long long* col = reinterpret_cast<unsigned long long*>(pr + B2);
+    unsigned long long* col = reinterpret_cast<unsigned long long*>(pr + stream_table_floats(B));
     unsigned long long* cnt = col + B;
     const int lane = threadIdx.x & 31;
     const int bd = (int)blockDim.x;
@@ -1191,7 +1194,7 @@ __device__ __forceinline__ void stream_rows(const SamplerParams& P, const EvalAr
     const int B = P.bins, B2 = B * B;
     double* red = dsh;
     const float* pr = reinterpret_cast<const float*>(dsh + 32 * NMOM);
-    const unsigned long long* col = reinterpret_cast<const unsigned long long*>(pr + B2);
+    const unsigned long long* col = reinterpret_cast<const unsigned long long*>(pr + stream_table_floats(B));
     const unsigned long long* cnt = col + B;
     const int lane = threadIdx.x & 31;
     const int bd = (int)blockDim.x;
