@@ -16,8 +16,8 @@
 // sample's validity and both Parzen bins are the reference's exactly.
 //
 //   k_bs_hist   pass 1: the joint histogram (FP64 Parzen taps quantised at the metric's
-//               fine unit 2^-kf, u64 shared-memory copies flushed with u64 atomics) and
-//               a record per sample (bins, Parzen fraction, moving gradient) in cell order.
+//               fine unit 2^-kf, added as 16-bit halves to u32 shared-memory copies, which
+//               are flushed with u64 atomics) and a record per sample (bins, Parzen fraction, moving gradient) in cell order.
 //               Its last CTA forms the tail from the integer histogram (value, and the
 //               pRatio·nFactor table into global memory).
 //   k_bs_cell_deriv  one or more CTAs per support cell: each valid sample of the cell adds
@@ -30,7 +30,7 @@
 //
 // Bound: FP64 operations (about 360 a sample in pass 1, 192 in the derivative, two cycles a
 // warp each), the L1's share of the control points and few warps beside the registers that
-// takes: pass 1 136 µs (FP64 pipe 33 % busy, L1 60 %) and the derivative 74 µs for 1.68 M
+// takes: pass 1 136 µs (FP64 pipe 33 % busy, L1 60 %) and the derivative 77 µs for 1.68 M
 // samples on an 8³ mesh. With the exact chain for every sample (about 1,000 operations,
 // twelve of them divisions) and 64-bit shared-memory atomics pass 1 took 341 µs.
 #include <cub/device/device_radix_sort.cuh>

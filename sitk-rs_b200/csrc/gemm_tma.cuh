@@ -18,8 +18,8 @@
 // for more than it gives (12 TB/s seen) before the tensor pipe is full; with MT = 2 a CTA
 // takes two blocks of 128 rows on one B tile, 64 KB for twice the operations, and one
 // accumulator (of 512 columns) instead of two. Narrow products (NT ≤ 64) are bound by the
-// bytes of A. 4096³: 109 µs a call with two blocks (1,263 TFLOP/s, 0.79 of 1.59 PFLOP/s), 118
-// with one; the one-stage kernel of gemm_tc.cuh took 1,489 µs. Products of few k are
+// bytes of A. 4096³ with warm caches: 109 µs a call with two blocks (1,263 TFLOP/s, 0.77 of the
+// measured 1,646), 118 with one (126 and 134 with cold inputs); the one-stage kernel of gemm_tc.cuh took 1,489 µs. Products of few k are
 // bound by their output: 32,768 × 432 × 32 writes 57 MB in 18 µs by TMA stores, 32 µs when
 // the four warps turned the blocks in shared memory and stored rows themselves (290
 // instructions a block).

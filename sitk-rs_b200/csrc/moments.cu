@@ -41,8 +41,8 @@
 // and the FP64 pipe is 28 % busy. So a cell's value and gradient are lerps sharing
 // their differences (22 FP64 operations; products of corner weights took about 130), floors
 // and integer conversions are adds of 2^52-sized constants, the decisions that are not
-// near a threshold compare integers. Evaluations: 240×239×155 mean squares 156 → 126 µs, 256³ at 10 %
-// correlation 86 → 55 µs and mean squares 51 → 42 µs.
+// near a threshold compare integers. Evaluations: 240×239×155 mean squares 156 → 122 µs, 256³ at 10 %
+// correlation 86 → 56 µs and mean squares 51 → 42 µs.
 #include <cfloat>
 #include <cmath>
 #include <cstring>
