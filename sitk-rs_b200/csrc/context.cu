@@ -83,7 +83,7 @@ PFN_cuTensorMapEncodeTiled_v12000 tensor_map_encoder() {
 // others: mi_context_trim), and with the context.
 constexpr unsigned long long POOL_KEEP = 256ull << 20;  // what the pool keeps of freed pages
 constexpr size_t LARGE = (size_t)1 << 20, LARGE_BYTES = (size_t)4 << 30, SPARE_BLOCKS = 256;
-constexpr size_t IMAGE_GRAIN = (size_t)1 << 16;  // of images below LARGE
+constexpr size_t IMAGE_GRAIN = (size_t)1 << 16, SMALL_IMAGE = (size_t)16 << 20;  // the grain below LARGE
 constexpr size_t SPARE_ARRAYS = 64, SPARE_ARRAY_BYTES = (size_t)1 << 30;
 constexpr size_t SLAB_BLOCKS = 64, PINNED_SPARES = 4, PINNED_KEEP = (size_t)16 << 20;
 
@@ -184,13 +184,15 @@ cudaError_t pool_alloc(mi_context* ctx, void** p, size_t bytes) {
     return e;
 }
 
-// A block that is kept, or a spare one of up to a quarter more.
+// A block that is kept, or a spare one of up to a quarter more, twice as much for an image
+// below SMALL_IMAGE (whose cudaMalloc takes longer than all the rest of making it).
 cudaError_t block_alloc(mi_context* ctx, void** p, size_t bytes, bool image) {
+    const size_t most = image && bytes < SMALL_IMAGE ? 2 * bytes : bytes + bytes / 4;
     {
         std::lock_guard<std::mutex> g(ctx->spare_mutex);
         auto best = ctx->spare_blocks.end();
         for (auto it = ctx->spare_blocks.begin(); it != ctx->spare_blocks.end(); ++it)
-            if (it->image == image && it->bytes >= bytes && it->bytes <= bytes + bytes / 4 &&
+            if (it->image == image && it->bytes >= bytes && it->bytes <= most &&
                 (best == ctx->spare_blocks.end() || it->bytes < best->bytes))
                 best = it;
         if (best != ctx->spare_blocks.end()) {
